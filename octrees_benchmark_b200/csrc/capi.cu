@@ -125,7 +125,8 @@ bool valid_algo(int a) { return a >= OCT_NEIGHBORS && a <= OCT_NEIGHBORS_STRUCT;
 
 // Count or fill pass of a radius search on the configured path.  With the
 // packet path the query order (sorted along the curve) is computed once per
-// call by the first pass and reused by the second.
+// call by the first pass and reused by the second; packets of one query need
+// no order (its five launches cost ~45 us, a walk of 2k such packets 116 us).
 cudaError_t radius_pass(Cloud& c, int kernel, int algo, bool fill, const double* dq, uint64_t nq, const double* dr,
                         double radius, unsigned long long* counts, unsigned long long* counts2,
                         const unsigned long long* offs, uint32_t* out, uint64_t cap, const uint32_t** order) {
@@ -137,7 +138,7 @@ cudaError_t radius_pass(Cloud& c, int kernel, int algo, bool fill, const double*
         c.rel_built = true;
     }
     if ((e = c.stats.reserve(64)) != cudaSuccess) return e;
-    if (!*order && (e = launch_query_order(c, dq, nq, order)) != cudaSuccess) return e;
+    if (!*order && packet_width(nq, c.device) > 1 && (e = launch_query_order(c, dq, nq, order)) != cudaSuccess) return e;
     return launch_radius_packet(c, kernel, algo, fill ? 1 : 0, fp32_on_radius(c.fp32_filter), dq, nq, dr, radius,
                                 *order, counts, counts2, offs, out, cap);
 }
@@ -154,7 +155,7 @@ int radius_chunks(Cloud& c, int kernel, int algo, const double* dq, uint64_t nq,
     CK(c.ck_first.reserve(4 * nq));
     CK(c.ck_ctr.reserve(256));
     const uint32_t* order = nullptr;
-    CK(launch_query_order(c, dq, nq, &order));
+    if (packet_width(nq, c.device) > 1) CK(launch_query_order(c, dq, nq, &order));
     if (fp32_on_radius(c.fp32_filter) && !c.rel_built) {  // the FP32 filter reads leaf-relative coordinates
         CK(launch_leaf_rel(c));
         c.rel_built = true;

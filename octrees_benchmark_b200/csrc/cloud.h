@@ -106,7 +106,7 @@ struct SearchReq {
     const double* radii;        // per-query radii (radius requests) or null
     double radius;              // radius when radii is null
     uint64_t q_begin, q_end;    // global query positions of this request
-    uint64_t packet_begin;      // first packet (32 queries) of the request in the launch
+    uint64_t packet_begin;      // first packet of the request in the launch
     uint64_t out_begin;         // kNN: first output slot (previous requests' nq * k)
     uint32_t k;                 // kNN k
     uint32_t cloud_id;          // distinct per cloud within the table (radii reload key)
@@ -121,7 +121,8 @@ struct DynGroup {
     const SearchReq* reqs;      // the group's requests (device), positions ascending
     uint32_t nreq;
     uint32_t kmax;              // kNN: largest k of the group
-    uint64_t packets;           // radius: 32-query packets of the group
+    uint64_t packets;           // packets of the group
+    uint64_t width;             // radius: queries per packet (packet_width)
     uint64_t q_begin;           // first query position of the group
     uint64_t nq;                // queries of the group
 };
@@ -292,14 +293,16 @@ struct ChunkArgs {
 };
 constexpr uint32_t kResultChunk = 64;
 
+// Queries per packet (1 to 32) of a packet radius launch over nq queries.
+uint32_t packet_width(uint64_t nq, int device);
 // Packet radius search.  Either one request (`single`, host copy, `packets`
-// packets) or the group of a batch (`d_grp`, sizes read on the device); with
+// packets of `width` queries) or the group of a batch (`d_grp`, sizes read on the device); with
 // both, every request of the group is on the cloud `single->cv` (kernel
 // parameters instead of per-request views).
 // mode: 0 count, 1 fill at d_offsets, 2 one pass into `chunks` (counts and
 // first chunks written; neighbors / neighborsPrune, FP64 only).
 cudaError_t launch_radius_table(int device, cudaStream_t s, int kernel, int algo, int mode, bool fp32,
-                                const DynGroup* d_grp, const SearchReq* single, uint64_t packets,
+                                const DynGroup* d_grp, const SearchReq* single, uint64_t packets, uint32_t width,
                                 const uint32_t* d_order, unsigned long long* d_counts, unsigned long long* d_counts2,
                                 const unsigned long long* d_offsets, uint32_t* d_out, uint64_t out_capacity,
                                 uint32_t* d_packet_ctr, unsigned long long* d_stats, uint32_t* d_err,

@@ -462,7 +462,7 @@ cudaError_t enqueue_work(oct_engine e) {
         for (int v = 0; v < kRadiusVariants; ++v) {
             if (!((e->sig >> v) & 1ull)) continue;
             const int kernel = v >> 2, algo = (v & 2) ? OCT_NEIGHBORS_PRUNE : OCT_NEIGHBORS;
-            if ((r = launch_radius_table(e->device, s, kernel, algo, 2, (v & 1) != 0, &dyn->groups[v], one, 0, order,
+            if ((r = launch_radius_table(e->device, s, kernel, algo, 2, (v & 1) != 0, &dyn->groups[v], one, 0, 0, order,
                                          counts, nullptr, nullptr, nullptr, 0, ctr + 2 * v, stats, err,
                                          e->radius_bps, &ck)) != cudaSuccess)
                 return r;
@@ -648,8 +648,10 @@ int submit(oct_engine e, const oct_request* rq, uint32_t n) {
     }
     // sizes, then capacities (growing drops graphs), then the packed table
     uint64_t n_total = 0, n_radius = 0, knn_slots = 0;
+    uint64_t var_nq[kRadiusVariants + kKnnVariants] = {};
     for (uint32_t i : rows) {
         n_total += rq[i].nq;
+        var_nq[var[i]] += rq[i].nq;
         if (rq[i].type == OCT_REQ_RADIUS) n_radius += rq[i].nq;
         else knn_slots += rq[i].nq * rq[i].k;
     }
@@ -722,9 +724,10 @@ int submit(oct_engine e, const oct_request* rq, uint32_t n) {
         gr.reqs = d_table + t;
         gr.q_begin = pos;
         gr.kmax = 0;
-        // packets: 32 queries (radius), kKnnGroupQueries (group kNN); the per-query kNN kernel ignores them
+        // packets: packet_width queries (radius), kKnnGroupQueries (group kNN); the per-query kNN kernel ignores them
         const bool group_knn = e->knn_group && v >= kRadiusVariants && v < kRadiusVariants + 2;
-        const uint64_t per = group_knn ? kKnnGroupQueries : 32;
+        gr.width = packet_width(var_nq[v], e->device);
+        const uint64_t per = group_knn ? kKnnGroupQueries : gr.width;
         uint32_t t0 = t;
         for (; t < m && var[rows[t]] == v; ++t) {
             const uint32_t i = rows[t];

@@ -1,12 +1,12 @@
 // Batched ("packet") radius search: neighbors / neighborsPrune / neighborsStruct
-// for 32 spatially ordered queries per warp.
+// for up to 32 spatially ordered queries per warp (packet_width).
 //
 // Reference path replaced: the same as radius_search.cu - singleTraversal
 // (inc/structures/linear_octree.hpp:653-686) with the criteria and leaf actions of
 // neighborsStruct (695-736), neighborsPrune (746-784) and neighbors (796-816).
 //
 // B200 design.  The query centres are first ordered along the cloud's curve
-// (launch_query_order), so the 32 queries of a warp are neighbours in space and
+// (launch_query_order), so the queries of a warp are neighbours in space and
 // need almost the same octants.  The warp walks the tree once for all of them:
 // at every internal node each lane judges the 8 children for its own query (the
 // reference's predicates, bit for bit), and a child is pushed with two lane
@@ -58,6 +58,7 @@ struct PacketArgs {
                                 // one_cloud, single.cv is the cloud of every request of grp
     const DynGroup* grp;        // sizes and request table of a batch group (device)
     uint64_t packets;           // packets of a single-request launch
+    uint32_t width;             // queries per packet of a single-request launch (1 to 32)
     bool one_cloud;             // host dispatch: grp's requests all search single.cv
     const uint32_t* order;      // query visiting order (global positions), or null
     unsigned long long* counts;
@@ -310,10 +311,12 @@ __global__ void __launch_bounds__(kPkThreads) k_radius_packet(PacketArgs a) {
     const SearchReq* reqs = nullptr;
     uint32_t nreq = 1;
     uint64_t packets = a.packets;
+    uint32_t width = a.width;
     if (MULTI) {
         reqs = a.grp->reqs;
         nreq = a.grp->nreq;
         packets = a.grp->packets;
+        width = a.grp->width;
     }
     const uint32_t lbit = 1u << lane;
     uint32_t* sn = st_node[warp];
@@ -348,8 +351,8 @@ __global__ void __launch_bounds__(kPkThreads) k_radius_packet(PacketArgs a) {
             __syncwarp();
         }
         const uint64_t q_begin = RQ(q_begin);
-        const uint64_t i = q_begin + 32ull * (packet - RQ(packet_begin)) + lane;
-        const bool valid = i < RQ(q_end);
+        const uint64_t i = q_begin + (uint64_t)width * (packet - RQ(packet_begin)) + lane;
+        const bool valid = (uint32_t)lane < width && i < RQ(q_end);
         const uint64_t qg = valid ? (a.order ? (uint64_t)a.order[i] : i) : q_begin;  // global query position
         const uint64_t ql = qg - q_begin;                                              // within the request
         const uint32_t qi = (uint32_t)qg;
@@ -1014,8 +1017,22 @@ CloudView cloud_view(const Cloud& c) {
     return v;
 }
 
+// Queries per packet: the widest of 1, 2, ... 16 that still leaves every resident warp (8 blocks per SM)
+// two packets.  A wide packet reads each node once for all its queries, but it is one warp's serial walk:
+// kernel time of sphere r = 2.5 searches of the 10M-point tile at widths 1 / 2 / 4 / 8 / 16 / 32, in us:
+//   100 centres 82 / 117 / 155 / 252 / 483 / 946     30k 398 / 360 / 375 / 418 / 618 / 1012
+//   2k   116 / 139 / 182 / 309 / 516 / 976           100k 1127 / 825 / 700 / 704 / 836 / 935
+//   8k   190 / 222 / 296 / 442 / 737 / 1237          500k 5234 / 3202 / 2380 / 2113 / 2017 / 2122
+// (with circles of 560 points on a dense tile 100k: 3446 / 2478 / 2006 / 1899 / 2123 / 2985).
+uint32_t packet_width(uint64_t nq, int device) {
+    const uint64_t packets = (uint64_t)sm_count_p(device) * kPkWarps * 8 * 2;
+    uint32_t w = 16;
+    while (w > 1 && (nq + w - 1) / w < packets) w >>= 1;
+    return w;
+}
+
 cudaError_t launch_radius_table(int device, cudaStream_t s, int kernel, int algo, int mode, bool fp32,
-                                const DynGroup* d_grp, const SearchReq* single, uint64_t packets,
+                                const DynGroup* d_grp, const SearchReq* single, uint64_t packets, uint32_t width,
                                 const uint32_t* d_order, unsigned long long* d_counts, unsigned long long* d_counts2,
                                 const unsigned long long* d_offsets, uint32_t* d_out, uint64_t out_capacity,
                                 uint32_t* d_packet_ctr, unsigned long long* d_stats, uint32_t* d_err,
@@ -1028,6 +1045,7 @@ cudaError_t launch_radius_table(int device, cudaStream_t s, int kernel, int algo
     a.grp = d_grp;
     a.one_cloud = d_grp != nullptr && single != nullptr;  // a batch on one cloud: its view in `single`
     a.packets = packets;
+    a.width = width;
     a.order = d_order;
     a.counts = d_counts;
     a.counts2 = d_counts2;
@@ -1100,7 +1118,8 @@ cudaError_t launch_radius_packet(Cloud& c, int kernel, int algo, int mode, bool 
     r.approx_cut = c.approx_cut;
     r.approx_upper = (uint32_t)c.approx_upper;
     KernelClock clk(c, 0);
-    e = launch_radius_table(c.device, c.stream, kernel, algo, mode, fp32, nullptr, &r, (nq + 31) / 32, d_order,
+    const uint32_t w = packet_width(nq, c.device);
+    e = launch_radius_table(c.device, c.stream, kernel, algo, mode, fp32, nullptr, &r, (nq + w - 1) / w, w, d_order,
                             d_counts, d_counts2, d_offsets, d_out, out_capacity, c.packet_ctr.as<uint32_t>(),
                             c.stats.as<unsigned long long>(), c.d_err.as<uint32_t>(), 0, chunks);
     clk.stop();

@@ -311,6 +311,30 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_top(unsigned long long* p
     if (threadIdx.x == 0) partials[m] = carry;
 }
 
+// The whole scan of up to kScanTile values in one block: one launch of ~3 us where the three
+// kernels of the long scan take ~9 (what a call of a few hundred centres waits for).
+__global__ void __launch_bounds__(kScanThreads) k_scan_one(const unsigned long long* in, uint32_t n,
+                                                           unsigned long long* out) {
+    __shared__ unsigned long long red[33];
+    unsigned long long v[kScanItems];
+    unsigned long long s = 0;
+#pragma unroll
+    for (int j = 0; j < kScanItems; ++j) {
+        const uint32_t i = threadIdx.x * kScanItems + j;
+        v[j] = (i < n) ? in[i] : 0ull;
+        s += v[j];
+    }
+    unsigned long long tot;
+    unsigned long long e = block_excl_scan(s, red, &tot);
+#pragma unroll
+    for (int j = 0; j < kScanItems; ++j) {
+        const uint32_t i = threadIdx.x * kScanItems + j;
+        if (i < n) out[i] = e;
+        e += v[j];
+    }
+    if (threadIdx.x == 0) out[n] = tot;
+}
+
 __global__ void __launch_bounds__(kScanThreads) k_scan_apply(const unsigned long long* in, uint64_t n,
                                                              const unsigned long long* partials,
                                                              unsigned long long* out) {
@@ -413,6 +437,10 @@ cudaError_t launch_scan_u64(Cloud& c, const unsigned long long* d_in, unsigned l
     if ((e = c.q_scan_tmp.reserve(8 * (blocks + 2))) != cudaSuccess) return e;
     unsigned long long* part = c.q_scan_tmp.as<unsigned long long>();
     if (n == 0) return cudaMemsetAsync(d_out, 0, 8, c.stream);
+    if (blocks == 1) {
+        k_scan_one<<<1, kScanThreads, 0, c.stream>>>(d_in, (uint32_t)n, d_out);
+        return cudaGetLastError();
+    }
     k_scan_partials<<<(unsigned)blocks, kScanThreads, 0, c.stream>>>(d_in, n, part);
     k_scan_top<<<1, kScanThreads, 0, c.stream>>>(part, blocks);
     k_scan_apply<<<(unsigned)blocks, kScanThreads, 0, c.stream>>>(d_in, n, part, d_out);
