@@ -147,9 +147,11 @@ cudaError_t radius_pass(Cloud& c, int kernel, int algo, bool fill, const double*
 // to its chain of result chunks, the counts are scanned, and the chains are
 // compacted into the CSR output.  A pool that turned out too small leaves the
 // counts exact: it is sized from the total and the traversal runs once more.
+// d_points (neighborsStruct ranges): every query's points; else NULL, and neighborsStruct searches its index set.
 int radius_chunks(Cloud& c, int kernel, int algo, const double* dq, uint64_t nq, const double* dr, double radius,
-                  unsigned long long* doffs, uint64_t* total) {
-    const int pass_algo = (algo == OCT_NEIGHBORS_STRUCT) ? OCT_NEIGHBORS_PRUNE : algo;  // same index set
+                  unsigned long long* doffs, uint64_t* total, unsigned long long* d_points = nullptr) {
+    const uint64_t per = d_points ? 2 : 1;  // chunk entries of a result
+    const int pass_algo = (algo == OCT_NEIGHBORS_STRUCT && !d_points) ? OCT_NEIGHBORS_PRUNE : algo;  // same index set
     unsigned long long* dc = c.q_counts.as<unsigned long long>();
     CK(c.stats.reserve(64));
     CK(c.ck_first.reserve(4 * nq));
@@ -164,7 +166,7 @@ int radius_chunks(Cloud& c, int kernel, int algo, const double* dq, uint64_t nq,
     for (int attempt = 0; attempt < 2; ++attempt) {
         // pool: every query's partial last chunk plus the results (a guess of 128 per query at first)
         const uint64_t want = attempt == 0 ? std::max<uint64_t>(c.ck_cap, 3 * nq + 1024)
-                                           : tot / kResultChunk + nq + 1024;
+                                           : per * tot / kResultChunk + nq + 1024;
         if (want > 0xfffffff0ull) return set_error(c, OCT_ERR_INVALID_ARG, "too many results for one call");
         if (want > c.ck_cap) {
             CK(c.ck_pool.reserve(4ull * kResultChunk * want));
@@ -175,7 +177,7 @@ int radius_chunks(Cloud& c, int kernel, int algo, const double* dq, uint64_t nq,
                      c.ck_ctr.as<uint32_t>(), c.ck_cap};
         CK(cudaMemsetAsync(ck.ctr, 0, 4, c.stream));
         CK(launch_radius_packet(c, kernel, pass_algo, 2, fp32_on_radius(c.fp32_filter), dq, nq, dr, radius, order,
-                                dc, nullptr, nullptr, nullptr, 0, &ck));
+                                dc, d_points, nullptr, nullptr, 0, &ck));
         CK(launch_scan_u64(c, dc, doffs, nq));
         CK(cudaMemcpyAsync(c.pinned, doffs + nq, 8, cudaMemcpyDeviceToHost, c.stream));
         const int st = sync_and_check(c, kErrChunkCapacity);
@@ -1119,13 +1121,19 @@ static int ranges_search(oct_cloud h, int kernel, const double* centers, uint64_
         doffs = c.q_offsets.as<unsigned long long>();
     }
     const uint32_t* order = nullptr;
-    CK(radius_pass(c, kernel, OCT_NEIGHBORS_STRUCT, false, dq, nq, dr, radius, dranges, dpoints, nullptr, nullptr, 0,
-                   &order));
-    CK(launch_scan_u64(c, dranges, doffs, nq));
-    CK(cudaMemcpyAsync(c.pinned, doffs + nq, 8, cudaMemcpyDeviceToHost, c.stream));
-    if ((st = sync_and_check(c)) != OCT_OK) return st;
     uint64_t tot;
-    memcpy(&tot, c.pinned, 8);
+    const bool one_pass = c.packet && !c.two_pass && nq;
+    if (one_pass) {
+        if ((st = radius_chunks(c, kernel, OCT_NEIGHBORS_STRUCT, dq, nq, dr, radius, doffs, &tot, dpoints)) != OCT_OK)
+            return st;
+    } else {
+        CK(radius_pass(c, kernel, OCT_NEIGHBORS_STRUCT, false, dq, nq, dr, radius, dranges, dpoints, nullptr, nullptr,
+                       0, &order));
+        CK(launch_scan_u64(c, dranges, doffs, nq));
+        CK(cudaMemcpyAsync(c.pinned, doffs + nq, 8, cudaMemcpyDeviceToHost, c.stream));
+        if ((st = sync_and_check(c)) != OCT_OK) return st;
+        memcpy(&tot, c.pinned, 8);
+    }
     if (total_ranges) *total_ranges = tot;
     if (!dev && range_offsets) CK(cudaMemcpyAsync(range_offsets, doffs, 8 * (nq + 1), cudaMemcpyDeviceToHost, c.stream));
     if (!dev && point_counts && nq) CK(cudaMemcpyAsync(point_counts, dpoints, 8 * nq, cudaMemcpyDeviceToHost, c.stream));
@@ -1138,8 +1146,15 @@ static int ranges_search(oct_cloud h, int kernel, const double* centers, uint64_
         CK(c.q_out.reserve(8 * (tot ? tot : 1)));
         dout = c.q_out.as<uint32_t>();
     }
-    CK(radius_pass(c, kernel, OCT_NEIGHBORS_STRUCT, true, dq, nq, dr, radius, nullptr, nullptr, doffs, dout, tot,
-                   &order));
+    if (one_pass) {
+        const ChunkArgs ck{c.ck_pool.as<uint32_t>(), c.ck_next.as<uint32_t>(), c.ck_first.as<uint32_t>(),
+                           c.ck_ctr.as<uint32_t>(), c.ck_cap};
+        CK(launch_chunk_compact(c.device, c.stream, dranges, doffs, ck, dout, 2 * tot, nq, nullptr,
+                                c.d_err.as<uint32_t>(), 2));
+    } else {
+        CK(radius_pass(c, kernel, OCT_NEIGHBORS_STRUCT, true, dq, nq, dr, radius, nullptr, nullptr, doffs, dout, tot,
+                       &order));
+    }
     if (!dev && tot) CK(cudaMemcpyAsync(pairs, dout, 8 * tot, cudaMemcpyDeviceToHost, c.stream));
     if (!dev) return sync_and_check(c);
     return OCT_OK;

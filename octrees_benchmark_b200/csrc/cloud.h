@@ -300,20 +300,22 @@ uint32_t packet_width(uint64_t nq, int device);
 // both, every request of the group is on the cloud `single->cv` (kernel
 // parameters instead of per-request views).
 // mode: 0 count, 1 fill at d_offsets, 2 one pass into `chunks` (counts and
-// first chunks written; neighbors / neighborsPrune, FP64 only).
+// first chunks written; neighborsStruct also writes d_counts2).
 cudaError_t launch_radius_table(int device, cudaStream_t s, int kernel, int algo, int mode, bool fp32,
                                 const DynGroup* d_grp, const SearchReq* single, uint64_t packets, uint32_t width,
                                 const uint32_t* d_order, unsigned long long* d_counts, unsigned long long* d_counts2,
                                 const unsigned long long* d_offsets, uint32_t* d_out, uint64_t out_capacity,
                                 uint32_t* d_packet_ctr, unsigned long long* d_stats, uint32_t* d_err,
                                 int blocks_per_sm = 0, const ChunkArgs* chunks = nullptr);
-// Chains of result chunks into CSR (after the counts are scanned into d_offsets).
+// Chains of result chunks into CSR (after the counts are scanned into d_offsets);
+// per = 2 for ranges (two entries a result; d_out and out_capacity count entries).
 // Per query, the sum of splitmix64's output function over its result chain.
 cudaError_t launch_chunk_hash(int device, cudaStream_t s, const unsigned long long* d_counts, const ChunkArgs& chunks,
                               unsigned long long* d_hashes, uint64_t n, uint32_t* d_err);
 cudaError_t launch_chunk_compact(int device, cudaStream_t s, const unsigned long long* d_counts,
                                  const unsigned long long* d_offsets, const ChunkArgs& chunks, uint32_t* d_out,
-                                 uint64_t out_capacity, uint64_t n, const uint64_t* d_n, uint32_t* d_err);
+                                 uint64_t out_capacity, uint64_t n, const uint64_t* d_n, uint32_t* d_err,
+                                 uint32_t per = 1);
 // kNN, one warp per query.  Either one request (`single`, nq queries, k <= 64,
 // register lists) or the group of a batch (`d_grp`, kmax = the group's largest
 // k: register lists up to 64, shared-memory lists up to 1024).

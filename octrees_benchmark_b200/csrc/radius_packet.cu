@@ -8,18 +8,27 @@
 // B200 design.  The query centres are first ordered along the cloud's curve
 // (launch_query_order), so the queries of a warp are neighbours in space and
 // need almost the same octants.  The warp walks the tree once for all of them:
-// at every internal node each lane judges the 8 children for its own query (the
-// reference's predicates, bit for bit), and a child is pushed with two lane
-// masks - the lanes for which it is fully inside (they emit its whole range
-// when it is popped) and the lanes that must descend into it.  Pushing the
-// children lowest octant last keeps every lane's output in ascending order.
-// Leaves, FP64 neighbors / neighborsPrune (the transposed test): the lanes load
-// 32 consecutive points and test them against one query of the descend mask at
-// a time, so all lanes work and the ballot is that query's hit mask, stored in
-// one coalesced write.  neighborsStruct and the FP32 form stage a leaf's points
-// in shared memory and every lane of the mask tests its own query against all
-// of them.  Fully-inside ranges are written by the whole warp.  Packets are
-// handed out by an atomic counter so that long and short packets balance.
+// at every internal node the lanes judge the 8 children for four queries at a
+// time (the reference's predicates, bit for bit), and a child is pushed with two
+// masks - the queries for which it is fully inside (they get its whole range
+// when it is popped) and those that must descend into it.  Pushing the
+// children lowest octant last keeps every query's output in ascending order.
+// Leaves (the transposed test): the lanes load 32 consecutive points of up to
+// kLeafGroup neighbouring leaves and test them against one query of the leaves'
+// masks at a time; the ballot is that query's hit mask, stored in one coalesced
+// write, or cut into the runs that neighborsStruct returns.  Fully-inside ranges
+// are written by the whole warp.  Packets are handed out by an atomic counter so
+// that long and short packets balance.
+//
+// Bound: instruction issue (2.45k warp instructions per query at r = 2.5 on the
+// 10M-point tile, DRAM below 5 % of peak): the pair loop takes about 1k of them,
+// the child tests 0.6k.  500k queries there: 2122 us with one leaf at a time and
+// one pass per four active queries, 1904 us with the leaf groups, 1638 us with
+// the aligned fours (no bit search per query), 24-byte stack records and the
+// one-chunk fast path of the hit store; 100k circles of 593 points over leaves
+// of 32 on a 2M-point tile 1899 -> 1416 -> 1159 us; 50k neighborsStruct squares
+// (count + fill, one lane per query over a leaf's points, then one pass of this
+// form) 4.9 -> 1.2 ms.
 //
 // Output: count pass + scan + fill at the scanned offsets, or one pass in which
 // every query appends its results to its own chain of 64-entry chunks (see
@@ -52,6 +61,8 @@ constexpr int kPkThreads = 32 * kPkWarps;
 constexpr int kPkStack = 8 * (kMaxDepth + 1);
 constexpr uint32_t kChunk = kResultChunk;  // entries per result chunk (one-pass mode)
 constexpr uint32_t kNoChunk = 0xffffffffu;
+constexpr uint32_t kNotOpen = 0xffffffffu;
+constexpr int kLeafGroup = 8;  // leaves tested as one run of points
 
 struct PacketArgs {
     SearchReq single;           // the request of a single-cloud search (grp == null); with
@@ -255,6 +266,9 @@ __device__ __forceinline__ LeafCtx get_ctx(const float* row) {
     return c;
 }
 
+// Bits 0, 8, 16 and 24 of x as a 4-bit number (the products land on distinct bits: no carries).
+__device__ __forceinline__ uint32_t four_bits(uint32_t x) { return (((x & 0x01010101u) * 0x01020408u) >> 24) & 15u; }
+
 // is_inside of lane j's query for point p: the same expressions, operand for operand.
 template <int KT>
 __device__ __forceinline__ bool inside_of(const double (*q)[kQpRow], int j, double px, double py, double pz) {
@@ -274,35 +288,36 @@ __device__ __forceinline__ bool inside_of(const double (*q)[kQpRow], int j, doub
     }
 }
 
-// CHUNK (with FILL, transposed form only): one pass instead of count + fill.
-// Each query appends its results to its own chain of kChunk-entry chunks taken
-// from a pool (contiguous chunks for one long range, so positions stay
-// linear); per query the count and the first chunk are written, and
-// k_chunk_compact moves every chain into the CSR array after the scan.
-template <int KT, int ALGO, bool FILL, bool F32, int MULTI, bool CHUNK = false>
+// MODE 0 counts, 1 fills at scanned offsets, 2 (one pass) appends each query's
+// results to its own chain of kChunk-entry chunks taken from a pool (contiguous
+// chunks for one long range, so positions stay linear); per query the count and
+// the first chunk are written, and k_chunk_compact moves every chain into the CSR
+// array after the scan.  A neighborsStruct range takes two entries.
+//
+// Leaves are tested in groups: up to kLeafGroup leaves that are next on the stack
+// (ascending, possibly with gaps) form one run of points, 32 of them on the lanes
+// at a time, each lane with its own leaf's query masks.  Leaves hold 10 to 30
+// points (empty octants are dropped), so a leaf at a time leaves half the lanes
+// idle and pays a stack pop per leaf.
+template <int KT, int ALGO, int MODE, bool F32, int MULTI>
 __global__ void __launch_bounds__(kPkThreads) k_radius_packet(PacketArgs a) {
-    // Transposed leaf test (neighbors / neighborsPrune, FP64 or FP32 filter): the
-    // lanes hold consecutive points and test them against one query of the mask
-    // at a time, so every lane does useful work and the ballot is that query's
-    // hit mask.  The FP32 form reads the points' leaf-relative coordinates and
-    // each query's context for the leaf (made once per leaf by the query's own
-    // lane); a point inside the error band is re-tested in FP64.
-    constexpr bool kT = (ALGO != kStruct);
-    static_assert(!CHUNK || (FILL && kT), "one-pass mode needs the transposed form");
-    constexpr int kStage = (kT || F32) ? 1 : kPkWarps;  // FP64 point staging, per-lane FP64 form only
+    // The leaf test is transposed: the lanes hold consecutive points and test them
+    // against one query of the masks at a time, so every lane does useful work and
+    // the ballot is that query's hit mask.  The FP32 form reads the points'
+    // leaf-relative coordinates and each query's context for the leaf (made once
+    // per leaf by the query's own lane, so its groups are single leaves); a point
+    // inside the error band is re-tested in FP64.
+    constexpr bool kRanges = (ALGO == kStruct);
+    constexpr bool kChain = (MODE == 2);
+    constexpr int kGroup = F32 ? 1 : kLeafGroup;
     constexpr int kCtxF = (KT == kSphere || KT == kCircle) ? 8 : 12;  // floats of a query's FP32 leaf context row
-    __shared__ __align__(16) float s_ctx[(F32 && kT) ? kPkWarps : 1][32][kCtxF];
+    __shared__ __align__(16) float s_ctx[F32 ? kPkWarps : 1][32][kCtxF];
     __shared__ CloudView s_view[MULTI == 1 ? kPkWarps : 1];
-    __shared__ uint32_t st_node[kPkWarps][kPkStack];
-    __shared__ uint32_t st_fc[kPkWarps][kPkStack];     // first child, 0 for a leaf
-    __shared__ uint2 st_rg[kPkWarps][kPkStack];        // point range
-    __shared__ uint32_t st_over[kPkWarps][kPkStack];
-    __shared__ uint32_t st_in[kPkWarps][kPkStack];
-    __shared__ uint8_t st_depth[kPkWarps][kPkStack];
+    __shared__ uint32_t st_node[F32 ? kPkWarps : 1][kPkStack];
+    __shared__ uint4 st_nd[kPkWarps][kPkStack];  // first child (0 for a leaf), point range, depth
+    __shared__ uint2 st_qm[kPkWarps][kPkStack];  // query masks: overlapping, fully inside
     __shared__ double s_rad[kPkWarps][kMaxDepth + 1][3];
     __shared__ __align__(16) double s_qp[kPkWarps][32][kQpRow];
-    __shared__ double sx[kStage][32], sy[kStage][32], sz[kStage][32];
-    __shared__ float4 sp[(F32 && !kT) ? kPkWarps : 1][32];
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     double (*s_radii)[3] = s_rad[warp];
@@ -319,12 +334,9 @@ __global__ void __launch_bounds__(kPkThreads) k_radius_packet(PacketArgs a) {
         width = a.grp->width;
     }
     const uint32_t lbit = 1u << lane;
-    uint32_t* sn = st_node[warp];
-    uint32_t* sf = st_fc[warp];
-    uint2* sr = st_rg[warp];
-    uint32_t* so = st_over[warp];
-    uint32_t* si = st_in[warp];
-    uint8_t* sd = st_depth[warp];
+    uint32_t* sn = st_node[F32 ? warp : 0];
+    uint4* sf = st_nd[warp];
+    uint2* sm = st_qm[warp];
     unsigned long long n_tests = 0, n_retests = 0;
 
     for (;;) {
@@ -358,17 +370,19 @@ __global__ void __launch_bounds__(kPkThreads) k_radius_packet(PacketArgs a) {
         const uint32_t qi = (uint32_t)qg;
         const double* qc = RQ(centers);
         const double* qrad = RQ(radii);
-        const uint32_t approx_cut = (ALGO == kStruct) ? RQ(approx_cut) : 0u;
-        const bool approx_upper = (ALGO == kStruct) && RQ(approx_upper) != 0;
+        const uint32_t approx_cut = kRanges ? RQ(approx_cut) : 0u;
+        const bool approx_upper = kRanges && RQ(approx_upper) != 0;
         SearchKernel k;
         k.init(qc[3 * ql], qc[3 * ql + 1], qc[3 * ql + 2], qrad ? qrad[ql] : RQ(radius));
         __syncwarp();  // the previous packet's reads of s_qp are done
         put_query<KT>(s_qp[warp], lane, k);  // read by the other lanes after a __syncwarp
-        unsigned long long cnt = 0, cnt2 = 0, base = 0;
-        if (FILL && !CHUNK && valid) base = a.offs[qi];
+        // per lane (its own query): results (ranges for neighborsStruct), points of the ranges,
+        // where the fill starts
+        uint32_t cnt = 0, cnt2 = 0;
+        unsigned long long base = 0;
+        if (MODE == 1 && valid) base = a.offs[qi];
         bool overflow = false;
-        bool open = false;  // neighborsStruct: a run of inside points is open
-        uint32_t rs = 0;
+        uint32_t open_at = kNotOpen;  // neighborsStruct: first point of the run that crosses into the next 32 points
         // one-pass mode: this lane's chain (current chunk, entries used in it, first chunk)
         uint32_t ck_cur = kNoChunk, ck_fill = kChunk, ck_first = kNoChunk;
         bool ck_over = false;
@@ -376,6 +390,8 @@ __global__ void __launch_bounds__(kPkThreads) k_radius_packet(PacketArgs a) {
         // Reserve n > 0 entries at the end of lane j's chain (warp-uniform call):
         // returns where they go - the first `room` continue chunk `cur`, the rest
         // are linear from chunk `nc` on (new chunks taken as one contiguous run).
+        // A pool that is too small leaves the chain full: nothing more is stored,
+        // the counts stay exact and the host runs again.
         struct ChunkPos {
             uint32_t cur, fill, room, nc;
         };
@@ -390,211 +406,252 @@ __global__ void __launch_bounds__(kPkThreads) k_radius_packet(PacketArgs a) {
                 uint32_t nc = 0;
                 if (lane == 0) nc = atomicAdd(a.chunk_ctr, m);
                 nc = __shfl_sync(0xffffffffu, nc, 0);
-                p.nc = nc;
                 const bool fits = (uint64_t)nc + m <= a.chunk_cap;
-                if (!fits) ck_over = true;  // the pool is too small: counts stay exact, the host re-runs
                 if (fits) {
+                    p.nc = nc;
                     if (lane == 0 && p.cur != kNoChunk) a.chunk_next[p.cur] = nc;
                     for (uint32_t t = lane; t + 1 < m; t += 32) a.chunk_next[nc + t] = nc + t + 1;
+                } else {
+                    ck_over = true;
                 }
                 if (lane == j) {
-                    if (ck_cur == kNoChunk) ck_first = nc;
-                    ck_cur = nc + m - 1;
-                    ck_fill = n - p.room - (m - 1) * kChunk;
+                    if (fits) {
+                        if (ck_cur == kNoChunk) ck_first = nc;
+                        ck_cur = nc + m - 1;
+                        ck_fill = n - p.room - (m - 1) * kChunk;
+                    } else {
+                        ck_fill = kChunk;
+                    }
                 }
             } else if (lane == j) {
                 ck_fill += n;
             }
-            if (lane == j) cnt += n;
             return p;
         };
         auto chunk_store = [&](const ChunkPos& p, uint32_t r, uint32_t v) {
-            const uint64_t pos = (r < p.room) ? (uint64_t)p.cur * kChunk + p.fill + r
-                                              : (uint64_t)p.nc * kChunk + (r - p.room);
-            if (pos < (uint64_t)a.chunk_cap * kChunk) a.chunk_pool[pos] = v;
+            if (r < p.room) a.chunk_pool[(uint64_t)p.cur * kChunk + p.fill + r] = v;
+            else if (p.nc != kNoChunk) a.chunk_pool[(uint64_t)p.nc * kChunk + (r - p.room)] = v;
+        };
+        // neighborsStruct, a range to the lane's own query (lanes diverge): chunks hold whole pairs
+        auto lane_range = [&](uint32_t f, uint32_t l) {
+            if (MODE == 1) {
+                const unsigned long long o = base + cnt;
+                if (o < a.out_cap) {
+                    a.out[2 * o] = f;
+                    a.out[2 * o + 1] = l;
+                } else {
+                    overflow = true;
+                }
+            }
+            if (kChain) {
+                bool room = ck_fill < kChunk;
+                if (!room) {
+                    const uint32_t nc = atomicAdd(a.chunk_ctr, 1u);
+                    if (nc < a.chunk_cap) {
+                        if (ck_cur != kNoChunk) a.chunk_next[ck_cur] = nc;
+                        else ck_first = nc;
+                        ck_cur = nc;
+                        ck_fill = 0;
+                        room = true;
+                    } else {
+                        ck_over = true;
+                    }
+                }
+                if (room) {
+                    uint32_t* d = a.chunk_pool + (uint64_t)ck_cur * kChunk + ck_fill;
+                    d[0] = f;
+                    d[1] = l;
+                    ck_fill += 2;
+                }
+            }
+            cnt += 1;
+            cnt2 += l - f;
         };
 
-        auto emit_range = [&](uint32_t f, uint32_t l) {  // per lane
-            if constexpr (ALGO == kStruct) {
-                if (FILL) {
-                    const unsigned long long o = base + cnt;
-                    if (o < a.out_cap) {
-                        a.out[2 * o] = f;
-                        a.out[2 * o + 1] = l;
+        // Query j's hits among the lanes' points (lane's point `idx`): appended in ascending order.
+        // neighborsStruct: starts bit v = lane v is the first point of its leaf, cont = lane 31's leaf
+        // goes on in the next 32 points; the maximal runs inside one leaf become ranges.
+        auto take = [&](int j, bool in, uint32_t idx, uint32_t starts, bool cont) {
+            const uint32_t hb = __ballot_sync(0xffffffffu, in);
+            if constexpr (!kRanges) {
+                (void)starts;
+                (void)cont;
+                if (!hb) return;
+                const uint32_t n = __popc(hb), rank = __popc(hb & lanemask_lt());
+                if constexpr (kChain) {
+                    const uint32_t fill = __shfl_sync(0xffffffffu, ck_fill, j);
+                    if (fill + n <= kChunk) {
+                        const uint32_t cur = __shfl_sync(0xffffffffu, ck_cur, j);
+                        if (in) a.chunk_pool[(uint64_t)cur * kChunk + (fill + rank)] = idx;
+                        if (lane == j) ck_fill = fill + n;
                     } else {
-                        overflow = true;
+                        const ChunkPos p = chunk_reserve(j, n);
+                        if (in) chunk_store(p, rank, idx);
                     }
-                }
-                cnt += 1;
-                cnt2 += (unsigned long long)(l - f);
-            } else {
-                if (FILL) {
-                    for (uint32_t t = f; t < l; ++t) {
-                        const unsigned long long o = base + cnt + (t - f);
-                        if (o < a.out_cap) a.out[o] = t;
-                        else overflow = true;
-                    }
-                }
-                cnt += (unsigned long long)(l - f);
-            }
-        };
-        auto hit = [&](uint32_t idx, bool in) {  // per lane, points in order
-            if constexpr (ALGO == kStruct) {
-                if (in && !open) {
-                    open = true;
-                    rs = idx;
-                } else if (!in && open) {
-                    open = false;
-                    emit_range(rs, idx);
-                }
-            } else {
-                if (in) {
-                    if (FILL) {
-                        const unsigned long long o = base + cnt;
+                } else if constexpr (MODE == 1) {
+                    const unsigned long long o = __shfl_sync(0xffffffffu, base + cnt, j) + rank;
+                    if (in) {
                         if (o < a.out_cap) a.out[o] = idx;
                         else overflow = true;
                     }
-                    ++cnt;
+                }
+                if (lane == j) cnt += n;
+            } else {
+                const uint32_t oa = __shfl_sync(0xffffffffu, open_at, j);
+                const bool opened = oa != kNotOpen;
+                if (!hb && !opened) return;
+                const uint32_t rs = hb & (~(hb << 1) | starts) & ~(opened ? 1u : 0u);  // first points of runs
+                uint32_t re = hb & (~(hb >> 1) | (starts >> 1));                       // last points of runs
+                const bool stays = cont && (hb >> 31);
+                if (stays) re &= 0x7fffffffu;
+                const uint32_t closed = (opened && !(hb & 1u)) ? 1u : 0u;  // the open run ended with the last 32 points
+                const uint32_t m = __popc(re) + closed;
+                if (MODE != 0 && m) {
+                    const uint32_t below = rs & (lanemask_lt() | lbit);
+                    const uint32_t f = below ? idx - (uint32_t)(lane - (31 - __clz(below))) : oa;
+                    const uint32_t r = closed + __popc(re & lanemask_lt());
+                    const bool ends = (re >> lane) & 1u;
+                    if constexpr (kChain) {
+                        const ChunkPos p = chunk_reserve(j, 2 * m);
+                        if (closed && lane == 0) {
+                            chunk_store(p, 0, oa);
+                            chunk_store(p, 1, idx);
+                        }
+                        if (ends) {
+                            chunk_store(p, 2 * r, f);
+                            chunk_store(p, 2 * r + 1, idx + 1);
+                        }
+                    } else {
+                        const unsigned long long o = __shfl_sync(0xffffffffu, base + cnt, j);
+                        if (o + m <= a.out_cap) {
+                            if (closed && lane == 0) {
+                                a.out[2 * o] = oa;
+                                a.out[2 * o + 1] = idx;
+                            }
+                            if (ends) {
+                                a.out[2 * (o + r)] = f;
+                                a.out[2 * (o + r) + 1] = idx + 1;
+                            }
+                        } else {
+                            overflow = true;
+                        }
+                    }
+                }
+                uint32_t next_open = kNotOpen;
+                if (stays) {
+                    const uint32_t last = __shfl_sync(0xffffffffu, idx, 31);
+                    next_open = rs ? last - (uint32_t)__clz(rs) : oa;
+                }
+                if (lane == j) {
+                    cnt += m;
+                    cnt2 += __popc(hb);
+                    open_at = next_open;
                 }
             }
         };
-        auto scan_leaf = [&](uint32_t node, uint2 rg, uint32_t mask) {
-            if constexpr (kT) {
-                if constexpr (F32) {  // each query of the mask: its context for this leaf, from its own lane
-                    __syncwarp();
-                    if ((mask >> lane) & 1u) {
-                        LeafCtx ctx;
-                        leaf_ctx<KT>(kernel_of<KT>(s_qp[warp], lane), RQV(centers) + 3ull * node, ctx);
-                        put_ctx<KT>(s_ctx[warp][lane], ctx);
-                    }
-                    __syncwarp();
-                } else {
-                    (void)node;
+
+        // The `g` leaves from stack slot `top` down: their points against the queries that overlap them
+        // (lanes < g hold the leaves' ranges and masks).
+        auto scan_leaves = [&](int top, int g) {
+            uint2 rg = make_uint2(0u, 0u);
+            uint32_t lo = 0, li = 0;
+            if (lane < g) {
+                const uint4 nd = sf[top - lane];
+                const uint2 qm = sm[top - lane];
+                rg = make_uint2(nd.y, nd.z);
+                lo = qm.x;
+                li = qm.y;
+                n_tests += (unsigned long long)__popc(lo) * (rg.y - rg.x);
+            }
+            if constexpr (F32) {  // each query of the leaf's mask: its context, from its own lane
+                const uint32_t mask = __shfl_sync(0xffffffffu, lo, 0);
+                const uint32_t node = sn[top];
+                __syncwarp();
+                if ((mask >> lane) & 1u) {
+                    LeafCtx ctx;
+                    leaf_ctx<KT>(kernel_of<KT>(s_qp[warp], lane), RQV(centers) + 3ull * node, ctx);
+                    put_ctx<KT>(s_ctx[warp][lane], ctx);
                 }
-                for (uint32_t b = rg.x; b < rg.y; b += 32) {
-                    const uint32_t idx = b + lane;
-                    const bool in_range = idx < rg.y;
-                    double px = 0.0, py = 0.0, pz = 0.0;
-                    float4 pf = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                    if (in_range) {
-                        if constexpr (F32) {
-                            pf = RQV(rel)[idx];
-                        } else {
-                            px = RQV(xs)[idx];
-                            py = RQV(ys)[idx];
-                            pz = RQV(zs)[idx];
-                        }
+                __syncwarp();
+            }
+            // first: the leaves' points as one run; leaf l holds [first, first + length) of it
+            const uint32_t len = rg.y - rg.x;
+            uint32_t end = len;
+#pragma unroll
+            for (int off = 1; off < kGroup; off <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, end, off);
+                if (lane >= off) end += y;
+            }
+            const uint32_t first = end - len;
+            const uint32_t total = __shfl_sync(0xffffffffu, end, kGroup - 1);  // lanes g .. kGroup - 1 add 0
+            for (uint32_t b = 0; b < total; b += 32) {
+                const uint32_t v = b + lane;
+                const bool in_range = v < total;
+                uint32_t idx, mo, mi, uni, starts = 0;
+                bool cont = false;
+                if constexpr (kGroup == 1) {
+                    idx = __shfl_sync(0xffffffffu, rg.x, 0) + v;
+                    mo = __shfl_sync(0xffffffffu, lo, 0);
+                    mi = __shfl_sync(0xffffffffu, li, 0);
+                    uni = mo | mi;
+                    if (kRanges) {
+                        starts = b == 0 ? 1u : 0u;
+                        cont = total > b + 32;
                     }
-                    // query j's hits among the lanes' points: appended to its chunks, or stored ascending
-                    // in one coalesced store (FILL), and counted
-                    auto take = [&](int j, bool in) {
-                        const uint32_t hb = __ballot_sync(0xffffffffu, in);
-                        if constexpr (CHUNK) {
-                            if (hb) {
-                                const ChunkPos p = chunk_reserve(j, __popc(hb));
-                                if (in) chunk_store(p, __popc(hb & lanemask_lt()), idx);
-                            }
-                            return;
-                        }
-                        if (FILL && hb) {
-                            const unsigned long long o0 = __shfl_sync(0xffffffffu, base + cnt, j);
-                            if (in) {
-                                const unsigned long long o = o0 + __popc(hb & lanemask_lt());
-                                if (o < a.out_cap) a.out[o] = idx;
-                                else overflow = true;
-                            }
-                        }
-                        if (lane == j) cnt += __popc(hb);
-                    };
-                    uint32_t rem = mask;
-                    while (rem) {
-                        const int j = __ffs(rem) - 1;
-                        rem &= rem - 1;
-                        if constexpr (F32) {
-                            bool in;
-                            const int r = in_range ? f32_test<KT>(get_ctx<KT>(s_ctx[warp][j]), pf) : 0;
+                } else {
+                    // the lane's leaf: leaves begun before b, plus those that begin at or below the lane
+                    const bool is = lane < g;
+                    const uint32_t before = __popc(__ballot_sync(0xffffffffu, is && first < b));
+                    const bool here = is && first >= b && first < b + 32;
+                    starts = __reduce_or_sync(0xffffffffu, here ? 1u << (first - b) : 0u);
+                    const int e = (int)(before + __popc(starts & (lanemask_lt() | lbit))) - 1;
+                    idx = __shfl_sync(0xffffffffu, rg.x - first, e) + v;
+                    mo = __shfl_sync(0xffffffffu, lo, e);
+                    mi = __shfl_sync(0xffffffffu, li, e);
+                    uni = __reduce_or_sync(0xffffffffu, (is && first < b + 32 && end > b) ? (lo | li) : 0u);
+                    if (kRanges) cont = __any_sync(0xffffffffu, is && first < b + 32 && end > b + 32);
+                }
+                double px = 0.0, py = 0.0, pz = 0.0;
+                float4 pf = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                if (in_range) {
+                    if constexpr (F32) {
+                        pf = RQV(rel)[idx];
+                    } else {
+                        px = RQV(xs)[idx];
+                        py = RQV(ys)[idx];
+                        pz = RQV(zs)[idx];
+                    }
+                } else {
+                    mo = mi = 0;
+                }
+                for (uint32_t rem = uni; rem;) {
+                    const int j = 31 - __clz(rem);
+                    const uint32_t jb = 1u << j;
+                    rem ^= jb;
+                    if constexpr (F32) {
+                        bool in = (mi & jb) != 0;
+                        if (mo & jb) {
+                            const int r = f32_test<KT>(get_ctx<KT>(s_ctx[warp][j]), pf);
                             if (r < 0) {  // inside the error band: the reference's FP64 expression decides
                                 in = inside_of<KT>(s_qp[warp], j, RQV(xs)[idx], RQV(ys)[idx], RQV(zs)[idx]);
                                 ++n_retests;
                             } else {
                                 in = r > 0;
                             }
-                            take(j, in);
-                        } else {
-                            // two queries at a time: their FP64 tests are independent, so their latencies
-                            // overlap instead of adding up
-                            const bool two = rem != 0;
-                            const int j2 = two ? __ffs(rem) - 1 : j;
-                            if (two) rem &= rem - 1;
-                            const bool in = in_range && inside_of<KT>(s_qp[warp], j, px, py, pz);
-                            const bool in2 = two && in_range && inside_of<KT>(s_qp[warp], j2, px, py, pz);
-                            take(j, in);
-                            if (two) take(j2, in2);
                         }
-                    }
-                    if (lane == 0) n_tests += (unsigned long long)__popc(mask) * ((rg.y - b < 32u) ? (rg.y - b) : 32u);
-                }
-            } else {
-            const bool mine = (mask & lbit) != 0;
-            LeafCtx ctx;
-            if (F32 && mine) leaf_ctx<KT>(k, RQV(centers) + 3ull * node, ctx);
-            for (uint32_t b = rg.x; b < rg.y; b += 32) {
-                const uint32_t idx = b + lane;
-                if (idx < rg.y) {
-                    if constexpr (F32) {
-                        sp[warp][lane] = RQV(rel)[idx];
+                        take(j, in, idx, starts, cont);
                     } else {
-                        sx[warp][lane] = RQV(xs)[idx];
-                        sy[warp][lane] = RQV(ys)[idx];
-                        sz[warp][lane] = RQV(zs)[idx];
+                        // two queries at a time: their FP64 tests are independent, so their latencies
+                        // overlap instead of adding up
+                        const int j2 = rem ? 31 - __clz(rem) : j;
+                        const uint32_t jb2 = rem ? 1u << j2 : 0u;
+                        rem ^= jb2;
+                        const bool t1 = inside_of<KT>(s_qp[warp], j, px, py, pz);
+                        const bool t2 = inside_of<KT>(s_qp[warp], j2, px, py, pz);
+                        take(j, ((t1 ? mo : mi) | mi) & jb, idx, starts, cont);
+                        if (jb2) take(j2, ((t2 ? mo : mi) | mi) & jb2, idx, starts, cont);
                     }
                 }
-                __syncwarp();
-                const uint32_t m = (rg.y - b < 32u) ? (rg.y - b) : 32u;
-                // bit t: staged point t is inside this lane's query
-                uint32_t hits = 0;
-                if (mine) {
-                    for (uint32_t t = 0; t < m; ++t) {
-                        bool in;
-                        if constexpr (F32) {
-                            const int r = f32_test<KT>(ctx, sp[warp][t]);
-                            if (r < 0) {
-                                in = is_inside<KT>(k, RQV(xs)[b + t], RQV(ys)[b + t], RQV(zs)[b + t]);
-                                ++n_retests;
-                            } else {
-                                in = r > 0;
-                            }
-                        } else {
-                            in = is_inside<KT>(k, sx[warp][t], sy[warp][t], sz[warp][t]);
-                        }
-                        if constexpr (ALGO == kStruct) hit(b + t, in);
-                        else hits |= (uint32_t)in << t;
-                    }
-                    n_tests += m;
-                }
-                if constexpr (ALGO != kStruct) {
-                    if (FILL) {  // every lane's hits in one coalesced store, lane after lane
-                        uint32_t rem = __ballot_sync(0xffffffffu, hits != 0);
-                        while (rem) {
-                            const int j = __ffs(rem) - 1;
-                            rem &= rem - 1;
-                            const uint32_t hj = __shfl_sync(0xffffffffu, hits, j);
-                            const unsigned long long o0 = __shfl_sync(0xffffffffu, base + cnt, j);
-                            if ((hj >> lane) & 1u) {
-                                const unsigned long long o = o0 + __popc(hj & lanemask_lt());
-                                if (o < a.out_cap) a.out[o] = b + lane;
-                                else overflow = true;
-                            }
-                        }
-                    }
-                    cnt += __popc(hits);
-                }
-                __syncwarp();
-            }
-            if (ALGO == kStruct && mine && open) {
-                open = false;
-                emit_range(rs, rg.y);
-            }
             }
         };
 
@@ -617,12 +674,9 @@ __global__ void __launch_bounds__(kPkThreads) k_radius_packet(PacketArgs a) {
                 const uint32_t fc0 = RQV(offsets)[0];
                 const uint2 rg0 = RQV(ranges)[0];
                 if (lane == 0) {
-                    sn[0] = 0;
-                    sf[0] = fc0;
-                    sr[0] = rg0;
-                    so[0] = mo;
-                    si[0] = mi;
-                    sd[0] = 0;
+                    if (F32) sn[0] = 0;
+                    sf[0] = make_uint4(fc0, rg0.x, rg0.y, 0u);
+                    sm[0] = make_uint2(mo, mi);
                 }
                 sp_top = 1;
             }
@@ -630,35 +684,41 @@ __global__ void __launch_bounds__(kPkThreads) k_radius_packet(PacketArgs a) {
         __syncwarp();
         while (sp_top > 0) {
             --sp_top;
-            const uint32_t node = sn[sp_top];
-            const uint32_t fc = sf[sp_top];
-            const uint2 nrg = sr[sp_top];
-            const uint32_t mo = so[sp_top];
-            const uint32_t mi = si[sp_top];
-            const uint32_t depth = sd[sp_top];
+            const uint4 nd = sf[sp_top];
+            const uint32_t fc = nd.x;
+            const uint2 nrg = make_uint2(nd.y, nd.z);
+            if (fc == 0 && nrg.x != nrg.y) {
+                // a leaf: with it the leaves that follow on the stack
+                int g = 1;
+                if (kGroup > 1) {
+                    const int s = sp_top - lane;
+                    bool leaf = lane < kGroup && s >= 0 && sf[s].x == 0;
+                    if (kRanges && leaf) leaf = sf[s].y != sf[s].z;  // an empty inside leaf adds its own empty range
+                    g = __ffs(~__ballot_sync(0xffffffffu, leaf)) - 1;
+                }
+                scan_leaves(sp_top, g);
+                sp_top -= g - 1;
+                __syncwarp();
+                continue;
+            }
+            const uint2 qm = sm[sp_top];
+            const uint32_t mo = qm.x, mi = qm.y, depth = nd.w;
             __syncwarp();
-            if constexpr (ALGO == kStruct) {
-                if (mi & lbit) emit_range(nrg.x, nrg.y);
+            if constexpr (kRanges) {
+                if (mi & lbit) lane_range(nrg.x, nrg.y);
             } else if (mi) {
                 // a fully-inside node: every lane of mi adds the node's whole range; the
                 // warp writes it for one lane at a time, 32 consecutive indices per store
                 const uint32_t len = nrg.y - nrg.x;
-                if constexpr (CHUNK) {
-                    if (len) {
-                        uint32_t rem = mi;
-                        while (rem) {
-                            const int j = __ffs(rem) - 1;
-                            rem &= rem - 1;
+                if (MODE != 0 && len) {
+                    uint32_t rem = mi;
+                    while (rem) {
+                        const int j = __ffs(rem) - 1;
+                        rem &= rem - 1;
+                        if constexpr (kChain) {
                             const ChunkPos p = chunk_reserve(j, len);
                             for (uint32_t t = lane; t < len; t += 32) chunk_store(p, t, nrg.x + t);
-                        }
-                    }
-                } else {
-                    if (FILL) {
-                        uint32_t rem = mi;
-                        while (rem) {
-                            const int j = __ffs(rem) - 1;
-                            rem &= rem - 1;
+                        } else {
                             const unsigned long long o0 = __shfl_sync(0xffffffffu, base + cnt, j);
                             for (uint32_t t = lane; t < len; t += 32) {
                                 const unsigned long long o = o0 + t;
@@ -667,14 +727,10 @@ __global__ void __launch_bounds__(kPkThreads) k_radius_packet(PacketArgs a) {
                             }
                         }
                     }
-                    if (mi & lbit) cnt += len;
                 }
+                if (mi & lbit) cnt += len;
             }
-            if (mo == 0) continue;
-            if (fc == 0) {
-                scan_leaf(node, nrg, mo);
-                continue;
-            }
+            if (mo == 0 || fc == 0) continue;
             const uint32_t cd = depth + 1;
             // lane j (< 8) keeps child j's first-child link, range and lane masks
             uint32_t my_fc = 0, my_mo = 0, my_mi = 0;
@@ -685,53 +741,43 @@ __global__ void __launch_bounds__(kPkThreads) k_radius_packet(PacketArgs a) {
             }
             // neighborsApprox (linear_octree.hpp:979-985): below its precision level a
             // child is cut before any box test, its whole range added in upper-bound mode
-            const bool cut = ALGO == kStruct && approx_cut != 0 && cd >= approx_cut;
+            const bool cut = kRanges && approx_cut != 0 && cd >= approx_cut;
             {
-                // child tests transposed: lane = (query slot lane / 8, child lane % 8), the
-                // node's active queries four at a time, so a node that few queries of the
-                // packet reach costs few passes; each lane tests with the query's own
-                // SearchKernel and the child's centre, as the per-query walk does
-                const int slot = lane >> 3;
+                // child tests transposed: lane = (query slot lane / 8, child lane % 8), four
+                // consecutive queries of the packet at a time (those next to each other on the
+                // curve mostly reach the same nodes), skipping fours the node does not concern;
+                // each lane tests with the query's own SearchKernel and the child's centre, as
+                // the per-query walk does
                 const double* ocp = RQV(centers) + 3ull * (fc + (lane & 7));
                 const double oc[3] = {ocp[0], ocp[1], ocp[2]};
-                uint32_t rem = mo;
-                while (rem) {
-                    int ql[4];
-#pragma unroll
-                    for (int s = 0; s < 4; ++s) {
-                        ql[s] = rem ? __ffs(rem) - 1 : -1;
-                        rem &= rem - 1;
-                    }
-                    const int myq = slot == 0 ? ql[0] : slot == 1 ? ql[1] : slot == 2 ? ql[2] : ql[3];
+                int q0 = 0;
+                for (uint32_t rem = mo; rem; rem >>= 4, q0 += 4) {
+                    if (!(rem & 15u)) continue;
                     bool o = false, n = false;
-                    if (myq >= 0) {
-                        const SearchKernel kq = kernel_of<KT>(s_qp[warp], myq);
-                        if constexpr (ALGO == kNeighbors) {
-                            o = box_overlap<KT>(kq, oc, s_radii[cd]);
-                        } else if (cut) {
-                            n = approx_upper;
-                        } else {
-                            const int jj = box_intersect<KT>(kq, oc, s_radii[cd]);
-                            n = (jj == kInside);
-                            o = (jj == kOverlap);
-                        }
+                    const SearchKernel kq = kernel_of<KT>(s_qp[warp], q0 + (lane >> 3));
+                    if constexpr (ALGO == kNeighbors) {
+                        o = box_overlap<KT>(kq, oc, s_radii[cd]);
+                    } else if (cut) {
+                        n = approx_upper;
+                    } else {
+                        const int jj = box_intersect<KT>(kq, oc, s_radii[cd]);
+                        n = (jj == kInside);
+                        o = (jj == kOverlap);
                     }
+                    // bit 8 s + c of a ballot: query q0 + s against child c; lane c gathers its four bits
                     const uint32_t bo = __ballot_sync(0xffffffffu, o);
-                    const uint32_t bi = __ballot_sync(0xffffffffu, n);
-                    if (lane < 8) {  // bit 8 s + j of a ballot: query ql[s] against child j
-#pragma unroll
-                        for (int s = 0; s < 4; ++s) {
-                            if (ql[s] >= 0) {
-                                my_mo |= ((bo >> (8 * s + lane)) & 1u) << ql[s];
-                                my_mi |= ((bi >> (8 * s + lane)) & 1u) << ql[s];
-                            }
-                        }
+                    my_mo |= four_bits(bo >> (lane & 7)) << q0;
+                    if constexpr (ALGO != kNeighbors) {
+                        const uint32_t bi = __ballot_sync(0xffffffffu, n);
+                        my_mi |= four_bits(bi >> (lane & 7)) << q0;
                     }
                 }
+                my_mo &= mo;
+                my_mi &= mo;
             }
             if (lane < 8 && my_fc == 0 && my_rg.x == my_rg.y) {  // empty leaf: nothing to scan or add
                 my_mo = 0;
-                if (ALGO != kStruct) my_mi = 0;  // neighborsStruct still adds its empty range
+                if (!kRanges) my_mi = 0;  // neighborsStruct still adds its empty range
             }
             const uint32_t pushm = __ballot_sync(0xffffffffu, lane < 8 && (my_mo | my_mi) != 0);
             const int np = __popc(pushm);
@@ -742,22 +788,19 @@ __global__ void __launch_bounds__(kPkThreads) k_radius_packet(PacketArgs a) {
             if ((pushm >> lane) & 1u) {
                 // lowest octant on top of the stack
                 const int slot = sp_top + __popc(pushm >> (lane + 1));
-                sn[slot] = fc + lane;
-                sf[slot] = my_fc;
-                sr[slot] = my_rg;
-                so[slot] = my_mo;
-                si[slot] = my_mi;
-                sd[slot] = (uint8_t)cd;
+                if (F32) sn[slot] = fc + lane;
+                sf[slot] = make_uint4(my_fc, my_rg.x, my_rg.y, cd);
+                sm[slot] = make_uint2(my_mo, my_mi);
             }
             __syncwarp();
             sp_top += np;
         }
-        if (overflow) set_err(a.err, (FILL && !CHUNK) ? kErrOutputCapacity : kErrStackOverflow);
-        if (CHUNK && ck_over) set_err(a.err, kErrChunkCapacity);
-        if ((!FILL || CHUNK) && valid) {
+        if (overflow) set_err(a.err, MODE == 1 ? kErrOutputCapacity : kErrStackOverflow);
+        if (kChain && ck_over) set_err(a.err, kErrChunkCapacity);
+        if (MODE != 1 && valid) {
             a.counts[qi] = cnt;
-            if (CHUNK) a.chunk_first[qi] = ck_first;
-            if (ALGO == kStruct) a.counts2[qi] = cnt2;
+            if (kChain) a.chunk_first[qi] = ck_first;
+            if (kRanges) a.counts2[qi] = cnt2;
         }
         __syncwarp();
     }
@@ -810,16 +853,14 @@ cudaError_t launch_pk_m(const PacketArgs& a, int mode, bool fp32, int grid, cuda
         return cudaErrorInvalidValue;
     }
     if (mode == 2) {
-        if constexpr (ALGO != kStruct) {
-            if (fp32) k_radius_packet<KT, ALGO, true, true, MULTI, true><<<grid, kPkThreads, 0, s>>>(a);
-            else k_radius_packet<KT, ALGO, true, false, MULTI, true><<<grid, kPkThreads, 0, s>>>(a);
-        }
+        if (fp32) k_radius_packet<KT, ALGO, 2, true, MULTI><<<grid, kPkThreads, 0, s>>>(a);
+        else k_radius_packet<KT, ALGO, 2, false, MULTI><<<grid, kPkThreads, 0, s>>>(a);
     } else if (mode == 1) {
-        if (fp32) k_radius_packet<KT, ALGO, true, true, MULTI><<<grid, kPkThreads, 0, s>>>(a);
-        else k_radius_packet<KT, ALGO, true, false, MULTI><<<grid, kPkThreads, 0, s>>>(a);
+        if (fp32) k_radius_packet<KT, ALGO, 1, true, MULTI><<<grid, kPkThreads, 0, s>>>(a);
+        else k_radius_packet<KT, ALGO, 1, false, MULTI><<<grid, kPkThreads, 0, s>>>(a);
     } else {
-        if (fp32) k_radius_packet<KT, ALGO, false, true, MULTI><<<grid, kPkThreads, 0, s>>>(a);
-        else k_radius_packet<KT, ALGO, false, false, MULTI><<<grid, kPkThreads, 0, s>>>(a);
+        if (fp32) k_radius_packet<KT, ALGO, 0, true, MULTI><<<grid, kPkThreads, 0, s>>>(a);
+        else k_radius_packet<KT, ALGO, 0, false, MULTI><<<grid, kPkThreads, 0, s>>>(a);
     }
     return cudaGetLastError();
 }
@@ -857,7 +898,8 @@ __global__ void __launch_bounds__(256) k_chunk_compact(const unsigned long long*
                                                        const uint32_t* __restrict__ next,
                                                        const uint32_t* __restrict__ pool, uint64_t chunk_cap,
                                                        uint32_t* __restrict__ out, uint64_t out_cap, uint64_t n,
-                                                       const uint64_t* d_n, uint32_t* err) {
+                                                       const uint64_t* d_n, uint32_t per, uint32_t* err) {
+    // per: entries of a result (1 index, or 2 for a range); counts and offsets count results
     if (d_n) n = *d_n;
     const int lane = threadIdx.x & 31;
     const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
@@ -869,9 +911,9 @@ __global__ void __launch_bounds__(256) k_chunk_compact(const unsigned long long*
         unsigned long long cnt = 0, o = 0;
         uint32_t c0 = kNoChunk;
         if ((uint32_t)lane < S && q < n) {
-            cnt = counts[q];
+            cnt = counts[q] * per;
             if (cnt) {
-                o = offs[q];
+                o = offs[q] * per;
                 c0 = first[q];
             }
         }
@@ -1020,10 +1062,10 @@ CloudView cloud_view(const Cloud& c) {
 // Queries per packet: the widest of 1, 2, ... 16 that still leaves every resident warp (8 blocks per SM)
 // two packets.  A wide packet reads each node once for all its queries, but it is one warp's serial walk:
 // kernel time of sphere r = 2.5 searches of the 10M-point tile at widths 1 / 2 / 4 / 8 / 16 / 32, in us:
-//   100 centres 82 / 117 / 155 / 252 / 483 / 946     30k 398 / 360 / 375 / 418 / 618 / 1012
-//   2k   116 / 139 / 182 / 309 / 516 / 976           100k 1127 / 825 / 700 / 704 / 836 / 935
-//   8k   190 / 222 / 296 / 442 / 737 / 1237          500k 5234 / 3202 / 2380 / 2113 / 2017 / 2122
-// (with circles of 560 points on a dense tile 100k: 3446 / 2478 / 2006 / 1899 / 2123 / 2985).
+//   100 centres 71 / 100 / 137 / 225 / 420 / 843     30k 342 / 315 / 311 / 367 / 536 / 849
+//   2k   105 / 125 / 159 / 262 / 435 / 849           100k 968 / 688 / 588 / 588 / 664 / 772
+//   8k   176 / 198 / 265 / 385 / 626 / 1063          500k 4476 / 2618 / 1959 / 1735 / 1638 / 1720
+// (with circles of 560 points on a dense tile 100k: 2256 / 1560 / 1238 / 1159 / 1333 / 1937).
 uint32_t packet_width(uint64_t nq, int device) {
     const uint64_t packets = (uint64_t)sm_count_p(device) * kPkWarps * 8 * 2;
     uint32_t w = 16;
@@ -1060,7 +1102,7 @@ cudaError_t launch_radius_table(int device, cudaStream_t s, int kernel, int algo
     a.chunk_first = chunks ? chunks->first : nullptr;
     a.chunk_ctr = chunks ? chunks->ctr : nullptr;
     a.chunk_cap = chunks ? chunks->cap : 0;
-    if (mode == 2 && (!chunks || algo == kStruct)) return cudaErrorInvalidValue;
+    if (mode == 2 && (!chunks || (algo == kStruct && !d_counts2))) return cudaErrorInvalidValue;
     // persistent grid: warps take packets from the counter until none is left
     const uint64_t cap = (uint64_t)sm_count_p(device) * (blocks_per_sm > 0 ? blocks_per_sm : 12);
     const uint64_t want = d_grp ? cap : (packets + kPkWarps - 1) / kPkWarps;
@@ -1086,13 +1128,14 @@ cudaError_t launch_chunk_hash(int device, cudaStream_t s, const unsigned long lo
 
 cudaError_t launch_chunk_compact(int device, cudaStream_t s, const unsigned long long* d_counts,
                                  const unsigned long long* d_offsets, const ChunkArgs& chunks, uint32_t* d_out,
-                                 uint64_t out_capacity, uint64_t n, const uint64_t* d_n, uint32_t* d_err) {
+                                 uint64_t out_capacity, uint64_t n, const uint64_t* d_n, uint32_t* d_err,
+                                 uint32_t per) {
     if (!d_n && n == 0) return cudaSuccess;
     const uint64_t cap = (uint64_t)sm_count_p(device) * 8;
     const uint64_t want = d_n ? cap : (n + 31) / 32;  // 8 warps of at least 4 queries per block
     const int grid = (int)(want < cap ? (want ? want : 1) : cap);
     k_chunk_compact<<<grid, 256, 0, s>>>(d_counts, d_offsets, chunks.first, chunks.next, chunks.pool, chunks.cap,
-                                         d_out, out_capacity, n, d_n, d_err);
+                                         d_out, out_capacity, n, d_n, per, d_err);
     return cudaGetLastError();
 }
 
