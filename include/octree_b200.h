@@ -134,24 +134,28 @@ int oct_set_radius_group(oct_cloud cloud, int lanes);
  *               OCT_FP32_KNN (3): the kNN filter only; 0 (default): every test
  *               in FP64.  Results are the same.
  *  radius_lanes lanes per query when packet is 0: 8 (default), 16 or 32.
- *  knn_packet   1 (default): kNN with k <= 64 on the packet path walks the
- *               tree once per group of 4 curve-ordered queries per warp
- *               (queries whose provisional threshold turns out too small
- *               finish on the per-query kernel); 0: one warp per query,
- *               visited in curve order when packet is 1.
- *  knn_bucket   kNN with k <= 64 on the packet path scans any subtree of at
- *               most this many points as one contiguous range instead of
- *               descending into it (default 256; 0 descends to the leaves).
- *               Extra points cannot change the k best pairs.
+ *  knn_packet   1 (default): kNN on the packet path collects the points within
+ *               a provisional distance, one curve-ordered query per warp, and
+ *               ranks them at the end; 0: kNN with k <= 64 keeps a sorted
+ *               list and walks nearest first, one warp per query in curve
+ *               order.
+ *  knn_bucket   kNN on the packet path scans any subtree of at most this many
+ *               points (the collecting search: a quarter of it) as one
+ *               contiguous range instead of descending into it (default 256;
+ *               0 descends to the leaves).  Extra points cannot change the
+ *               k best pairs.
  *  reserved[0]  1: packet radius searches count, then fill at the scanned
  *               offsets; 0 (default): one pass into per-query result chunks.
- *  reserved[1]  kNN (k <= 64, packet path) provisional threshold, in percent of
- *               the radius holding k points at the density of the query's first
- *               cell: 0 = the default (120), < 0 = off.  Results are the same.
- *  reserved[2]  knn_packet: consecutive query groups a warp takes at a time
- *               (1-64; 0 = the default); every group after the first of a
- *               run starts from the previous group's k-th distances.  Results
- *               are the same. */
+ *  reserved[1]  kNN (packet path) provisional threshold: < 0 = off (the
+ *               collecting search then starts every query from the points
+ *               next to it); otherwise, for knn_packet 0 and k <= 64, in
+ *               percent of the radius holding k points at the density of the
+ *               query's first cell (0 = the default, 120).  Results are the
+ *               same.
+ *  reserved[2]  knn_packet: consecutive queries a warp takes at a time, in
+ *               pairs (1-64; 0 = the default, 4); every query after the
+ *               first of a run starts from the k-th distances before it.
+ *               Results are the same. */
 #define OCT_FP32_ALL 1    /* oct_search_config.fp32_filter: radius and kNN FP32 filters */
 #define OCT_FP32_RADIUS 2 /* the radius filter only */
 #define OCT_FP32_KNN 3    /* the kNN filter only */
@@ -371,8 +375,8 @@ int oct_engine_set_stream(oct_engine engine, void* cuda_stream);
 int oct_engine_last_error(oct_engine engine, char* buf, size_t len);
 /* Search configuration of the engine (oct_search_config: fp32_filter (0-3, as for
  * a cloud), knn_bucket;
- * knn_packet = 1 (the engine's default): kNN with k <= 64 in groups of 4
- * curve-ordered queries per warp, 0: one warp per query;
+ * knn_packet = 1 (the engine's default): the collecting kNN for every k, 0: k <= 64
+ * on the sorted-list kernel;
  * reserved[0] = radius blocks per SM, reserved[1] = kNN blocks per SM, 0 = default;
  * reserved[2] = 1 to run kNN after the radius search instead of beside it). */
 int oct_engine_set_config(oct_engine engine, const oct_search_config* config);

@@ -130,17 +130,13 @@ struct DynGroup {
 // Register kNN: provisional k-th distance = this factor x the radius that holds k
 // points at the density of the query's first cell (exact either way).
 constexpr double kKnnEstimate = 1.2;
-// Group kNN: consecutive query groups a warp takes at a time (the later ones start
-// from the previous group's k-th distances).
+// Curve-ordered kNN: consecutive queries a warp takes at a time, in pairs (the later
+// ones start from the k-th distances of those before them).  10M-point tile, 500k
+// queries of k = 50: runs of 8 take 2.74 ms, of 16 2.87, of 32 3.23 (L2 and L1 hits).
 constexpr uint32_t kKnnGroupChunk = 4;
-// group kNN heads: every kKnnHeadStride-th group is searched first, from the
-// density estimate; the others start from a neighbouring group's k-th distance
+// its heads: every kKnnHeadStride-th query is searched first, from its own node;
+// the others start from a neighbouring query's k-th distance
 constexpr uint32_t kKnnHeadStride = 16;
-// Queries per warp of the group kNN (4 or 8).  4: half the shared memory per
-// warp, so 28 warps per SM instead of 16, for ~1.6x the node visits per query;
-// ~20 % faster on the 10M-point tile (k = 50).
-constexpr uint32_t kKnnGroupQueries = 4;
-
 struct Cloud {
     oct_params params{};
     int device = 0;
@@ -188,7 +184,7 @@ struct Cloud {
     DevBuf qs_keys, qs_keys_alt, qs_ord, qs_ord_alt, qs_status, qs_ctl;
     uint32_t qs_epoch = 0;
     DevBuf packet_ctr;  // dynamic packet counters
-    DevBuf knn_fb;      // group kNN: fallback count (u64) at 0, fallback query list (u32) from byte 16
+    DevBuf knn_fb;      // collecting kNN: fallback count (u64) at 0, fallback query list (u32) from byte 16
     DevBuf knn_heads;   // group kNN: the heads' largest k-th distances (f64 per head)
     DevBuf stats;       // device counters: points tested, FP64 band re-tests, ...
     // FP32 leaf-relative coordinates (x, y, z, 0) per sorted point, built on demand
@@ -322,11 +318,10 @@ cudaError_t launch_chunk_compact(int device, cudaStream_t s, const unsigned long
 cudaError_t launch_knn_table(int device, cudaStream_t s, const DynGroup* d_grp, const SearchReq* single, uint64_t nq,
                              uint32_t kmax, const uint32_t* d_order, uint32_t bucket, uint32_t* d_idx, double* d_d2,
                              uint32_t* d_counts, uint32_t* d_err, int blocks_per_sm = 0, double est = 0.0);
-// Group kNN of a batch group (kmax <= 64: kKnnGroupQueries curve-ordered queries per warp),
-// then the per-query kernel over the queries it hands back.  d_fb: the
+// Curve-ordered kNN of a batch group, then the sorted-list kernels over the queries it hands back.  d_fb: the
 // fallback group (requests, kmax and q_begin of d_grp, nq = 0 before the
 // launch); d_fb_list: one entry per query position of the batch; d_packet_ctr:
-// two counters; blocks_per_sm > 0 caps the resident blocks of both launches.
+// three counters; blocks_per_sm > 0 caps the resident blocks of both launches.
 cudaError_t launch_knn_group_table(int device, cudaStream_t s, const DynGroup* d_grp, DynGroup* d_fb,
                                    const SearchReq* single, uint32_t kmax, const uint32_t* d_order, uint32_t bucket,
                                    uint32_t* d_idx, double* d_d2, uint32_t* d_counts, uint32_t* d_err,

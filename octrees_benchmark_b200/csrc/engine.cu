@@ -48,7 +48,7 @@ constexpr uint32_t kEpochLimit = (1u << 22) - 1;
 
 struct EngineDyn {
     DynGroup groups[kGroups];
-    DynGroup fb[2];     // group kNN (k <= 32, 64): the queries handed back to the per-query kernel
+    DynGroup fb[kKnnVariants];  // group kNN: the queries handed back to the sorted-list kernels
     uint64_t n_total;   // query positions of the batch (the sort size)
     uint64_t n_radius;  // radius positions [0, n_radius); kNN positions follow
     uint32_t nreq;      // requests in the table (non-empty ones)
@@ -271,7 +271,7 @@ struct oct_engine_s {
     uint32_t bucket = 128;
     int radius_bps = 0, knn_bps = 0;
     int serial = 0;  // 1: kNN after the radius search on one stream; 0: kNN forked beside it
-    int knn_group = 1;  // kNN with k <= 64: groups of kKnnGroupQueries queries per warp (0: one per warp)
+    int knn_group = 1;  // group kNN (0: k <= 64 on the per-query kernel)
     // device arrays
     DevBuf desc;  // EngineDyn, then the SearchReq table
     DevBuf keys[2], ord[2];
@@ -427,13 +427,13 @@ cudaError_t enqueue_work(oct_engine e) {
         cudaError_t r2 = cudaSuccess;
         for (int v = 0; v < kKnnVariants && r2 == cudaSuccess; ++v) {
             if (!((e->sig >> (kRadiusVariants + v)) & 1ull)) continue;
-            if (v < 2 && e->knn_group)
+            if (v >= 2 || e->knn_group)
                 r2 = launch_knn_group_table(e->device, ks, &dyn->groups[kRadiusVariants + v], &dyn->fb[v], one,
                                             32u << v, order, e->bucket, e->knn_idx.as<uint32_t>(),
                                             e->knn_d2.as<double>(), e->knn_counts.as<uint32_t>(), err,
                                             ctr + 2 * kRadiusVariants + 4 * v, e->knn_fb.as<uint32_t>(),
                                             kKnnEstimate, kKnnGroupChunk, e->knn_bps, e->knn_heads.as<double>(),
-                                            e->knn_heads.bytes, fp32_on_knn(e->fp32), stats + 2);
+                                            e->knn_heads.bytes, fp32_on_knn(e->fp32) && v < 2, stats + 2);
             else
                 r2 = launch_knn_table(e->device, ks, &dyn->groups[kRadiusVariants + v], one, 0, 32u << v,
                                       order, e->bucket, e->knn_idx.as<uint32_t>(), e->knn_d2.as<double>(),
@@ -678,10 +678,10 @@ int submit(oct_engine e, const oct_request* rq, uint32_t n) {
     if ((st = grow(e, e->knn_idx, 4 * std::max<uint64_t>(knn_slots, 1))) != OCT_OK) return st;
     if ((st = grow(e, e->knn_d2, 8 * std::max<uint64_t>(knn_slots, 1))) != OCT_OK) return st;
     if ((st = grow(e, e->knn_counts, 4 * std::max<uint64_t>(n_total, 1))) != OCT_OK) return st;
-    if (knn_slots && e->knn_group) {
+    if (knn_slots) {
         if ((st = grow(e, e->knn_fb, 4 * n_total)) != OCT_OK) return st;
-        // heads: one per kKnnHeadStride groups of every request (each request's groups round up)
-        const uint64_t groups = n_total / kKnnGroupQueries + m;
+        // heads: one per kKnnHeadStride groups of every request (at least one query a group)
+        const uint64_t groups = n_total + m;
         if ((st = grow(e, e->knn_heads, 8 * (groups / kKnnHeadStride + 2))) != OCT_OK) return st;
     }
     if ((st = grow(e, e->totals, sizeof(ReqTotal) * std::max<uint32_t>(m, 1))) != OCT_OK) return st;
@@ -724,10 +724,10 @@ int submit(oct_engine e, const oct_request* rq, uint32_t n) {
         gr.reqs = d_table + t;
         gr.q_begin = pos;
         gr.kmax = 0;
-        // packets: packet_width queries (radius), kKnnGroupQueries (group kNN); the per-query kNN kernel ignores them
-        const bool group_knn = e->knn_group && v >= kRadiusVariants && v < kRadiusVariants + 2;
+        // packets: packet_width queries (radius), single queries (kNN)
+        const bool group_knn = v >= kRadiusVariants && (e->knn_group || v >= kRadiusVariants + 2);
         gr.width = packet_width(var_nq[v], e->device);
-        const uint64_t per = group_knn ? kKnnGroupQueries : gr.width;
+        const uint64_t per = group_knn ? 1 : gr.width;
         uint32_t t0 = t;
         for (; t < m && var[rows[t]] == v; ++t) {
             const uint32_t i = rows[t];
@@ -838,7 +838,7 @@ int oct_engine_create(const oct_engine_params* p, oct_engine* out) {
     if (r == cudaSuccess && preload_kernels(e->device) != OCT_OK) r = cudaErrorInitializationError;
     if (r == cudaSuccess) r = e->sort_ctl.reserve(sizeof(SortCtl));
     if (r == cudaSuccess) r = e->epoch.reserve(256);
-    if (r == cudaSuccess) r = e->ctrs.reserve(4 * (2 * kRadiusVariants + 4 * 2));  // + group kNN (3 of 4 per variant)
+    if (r == cudaSuccess) r = e->ctrs.reserve(4 * (2 * kRadiusVariants + 4 * kKnnVariants));  // + group kNN (3 of 4 per variant)
     if (r == cudaSuccess) r = e->stats.reserve(64);
     if (r == cudaSuccess) r = e->summary.reserve(256);
     if (r == cudaSuccess) r = e->part.reserve(8 * (kScanBlocks + 1));
@@ -869,7 +869,7 @@ int oct_engine_create(const oct_engine_params* p, oct_engine* out) {
         const uint64_t tiles = (q + sort_tile_keys() - 1) / sort_tile_keys();
         const size_t want[][2] = {{0, 4 * q * 256}, {1, 8 * q * 256}, {2, sizeof(ReqTotal) * 1024},
                                   {3, table_offset() + 1024 * sizeof(SearchReq)}, {4, 256 * 8 * tiles},
-                                  {5, 8 * (q / kKnnGroupQueries / kKnnHeadStride + 1026)}, {6, 256}};
+                                  {5, 8 * (q / kKnnHeadStride + 1026)}, {6, 256}};
         DevBuf* bufs[] = {&e->knn_idx, &e->knn_d2, &e->totals, &e->desc, &e->sort_status, &e->knn_heads, &e->ck_ctr};
         for (const auto& w : want)
             if (r == cudaSuccess && grow(e, *bufs[w[0]], w[1]) != OCT_OK) r = cudaErrorMemoryAllocation;

@@ -16,7 +16,6 @@
 // (distance, index) resolves ties at the k-th distance by the lowest index.
 #include <algorithm>
 #include <cfloat>
-#include <cuda_fp16.h>
 
 #include "cloud.h"
 #include "search_kernels.cuh"
@@ -47,6 +46,7 @@ struct KnnArgs {
     const uint32_t* order;  // query visiting order (curve order), or nullptr
     uint32_t bucket;        // subtrees with at most this many points are scanned as one range
     const DynGroup* grp;    // table launch (k_knn<LCAP, true>): sizes and requests on the device
+    const unsigned long long* nq_dev;  // the query count in device memory (else nq)
 };
 
 __device__ __forceinline__ bool pair_less(double da, uint32_t ia, double db, uint32_t ib) {
@@ -135,6 +135,8 @@ __global__ void __launch_bounds__(kKnnThreads) k_knn(KnnArgs a) {
         nreq = a.grp->nreq;
         q0 = a.grp->q_begin;
         nq = a.grp->nq;
+    } else if (a.nq_dev) {
+        nq = *a.nq_dev;
     }
     const uint64_t nwarps = (uint64_t)gridDim.x * kKnnWarps;
     for (uint64_t w = (uint64_t)blockIdx.x * kKnnWarps + warp; w < nq; w += nwarps) {
@@ -143,11 +145,11 @@ __global__ void __launch_bounds__(kKnnThreads) k_knn(KnnArgs a) {
         uint32_t K = a.k;
         uint64_t o = q * (uint64_t)K;  // first output slot of this query
         const double* qc = a.q + 3 * q;
-        if (MULTI) {  // the request whose positions contain qpos (q_begin ascending)
+        if (MULTI) {  // the request whose positions contain q (q_begin ascending)
             uint32_t lo = 0, hi = nreq;
             while (hi - lo > 1) {
                 const uint32_t mid = (lo + hi) >> 1;
-                if (reqs[mid].q_begin <= qpos) lo = mid;
+                if (reqs[mid].q_begin <= q) lo = mid;
                 else hi = mid;
             }
             const SearchReq& rq = reqs[lo];
@@ -705,72 +707,87 @@ __global__ void __launch_bounds__(kKnnThreads, 8) k_knn_reg(KnnTableArgs a) {
 }
 
 // ---------------------------------------------------------------------------
-// Group kNN (k <= 64): kGrpQ (4) curve-ordered queries per warp share one walk.
+// Curve-ordered kNN: one query per warp, a walk that collects every point within
+// a provisional distance and ranks the collected points at the end.
 //
-// Consecutive queries along the curve are a few metres apart, so the octants
-// their searches need overlap almost entirely: 4 of them visit ~4.7 internal
-// nodes per query (8: ~2.9) where one query alone visits ~14 (10M-point tile,
-// k = 50).  Groups of 4 rather than 8 halve the shared memory per warp, so 28
-// warps fit on an SM instead of 16, which this latency-bound walk needs more.
-// The warp walks the tree once for its group, nearest first by the smallest
-// lower bound of the group; a child is pushed with the mask of queries that
-// accept it and, per query, its lower bound rounded down to FP16 (a popped
-// entry is skipped for a query whose threshold has since dropped below it; the
-// rounding only keeps entries).  At an internal node 32 / kGrpQ lanes per
-// query judge the 8 children.  A range (leaf, or subtree of at most `bucket`
-// points) is tested transposed: the lanes hold 32 consecutive points and test
-// them against one accepting query at a time, and the query's candidates
-// (pairs that beat its k-th pair) go to its own 32-entry buffer in shared
-// memory; a full buffer is merged into the query's sorted list (in shared
-// memory, R x 32 pairs) by the warp with the same register bitonic merge as
-// k_knn_reg.  Provisional thresholds: a warp takes `chunk` consecutive groups
-// at a time, and every group after the first of a run starts each query at
-// kGrpSeed x the largest k-th distance of the group before it (the k-th
-// distance varies slowly along the curve: this holds ~1.4 k points where the
-// density estimate of k_knn_reg holds several times more, so half the
-// candidates and merges go; longer runs widen the stretch of the curve that
-// the warps work on at once, which costs L2 hits).  Every kKnnHeadStride-th
-// group is a head: heads are handed out first and take k_knn_reg's density
-// estimate from the first range each query reaches; the first group of a run
-// (and each group handed out alone at the end) starts from the nearest head
-// of its request that has finished, or from the density estimate when none
-// has (no group waits for a head).  F32: range points are first tested in FP32
-// (centre-relative copies) against a per-query FP32 bound of the threshold
-// (knn_f32_threshold); only points not rejected take the FP64 distance.  A query that ends with fewer than k pairs
-// inside its provisional threshold, and every query of a group whose stack
-// overflowed, is appended to a fallback list that k_knn_reg completes exactly.
+// With a good provisional threshold the walk needs no order, no sorted list and
+// no merges: it is a radius search whose hits (squared distance, index) go to a
+// buffer of `cap` pairs in shared memory; if at least k pairs came in, the k
+// best are among them.  As the order is free, a step takes up to four nodes off
+// the stack, the 32 lanes judging their 32 children at once, and the point
+// ranges it finds are gathered and tested as one run of points, 32 lanes full
+// whatever the ranges' lengths.
+//
+// The final ranking is a counting sort: squared distances in the plane are
+// close to uniform, so `bins` equal bins of [0, threshold] hold one or two pairs
+// each; a pair's rank is its bin's start plus the pairs of the bin that precede
+// it by (distance, index), and the pair is written to that output slot.  (When a
+// bin holds more than kBinMany pairs the bins are taken again over the logarithm
+// of the distances, so far outliers do not press the others into one bin.)  A
+// buffer that runs full keeps the bins that hold its k smallest pairs and the
+// threshold drops to the largest pair kept.
+//
+// Thresholds: a warp takes `chunk` consecutive queries at a time, and every one
+// after the first of a run starts at kGrpSeed x the largest k-th distance of those
+// before it, each faded by kSeedFade a query (the k-th distance varies slowly along the curve;
+// longer runs widen the stretch of the curve that the warps work on at once,
+// which costs L2 hits).  Every kKnnHeadStride-th query is a head: heads are handed
+// out first; the first query of a run (and each query handed out alone at the
+// end) starts from the nearest head of its request that has finished.  A query
+// without a seed, and a query that found fewer than k pairs within its seeded
+// threshold, takes the k-th distance among the first 2 k points (3/2 k of k > 256) that a
+// best-first walk comes to (knn_near_ranges): an upper bound of its k-th
+// distance, so the walk that follows always suffices.  What is left (a stack or a buffer that cannot hold a
+// degenerate input) is appended to a fallback list that the sorted-list kernels
+// complete exactly.
+//
+// F32 (k <= 64): points are first tested in FP32 (centre-relative copies)
+// against an FP32 bound of the threshold (knn_f32_threshold); only points not
+// rejected take the FP64 distance.
+//
+// Bound: latency and issue (500k queries of k = 50 on the 10M-point tile: 3.7k
+// warp instructions a query where the sorted lists of four queries a warp took
+// 5.6k; 0.6 of a warp instruction a cycle and scheduler, dependent loads the
+// largest stall).  Two things cost more than they look: code that no longer fits
+// the instruction cache (the loops below are not unrolled: 3.42 -> 2.87 ms) and
+// shared memory, which is taken from the L1 that serves neighbouring queries
+// (2 KB more a block: 2.87 -> 2.97 ms).  Whole calls before (groups of four with
+// sorted lists for k <= 64, bitonic merges in shared memory above) and now:
+//   10M-point tile: 500k, k = 50 3700 -> 2787 us; 50k, k = 50 1069 -> 430; 5k, k = 50
+//   497 -> 195; 200, k = 50 345 -> 105; 5M: 30k, k = 250 2300 -> 710; 3k, k = 900
+//   2400 -> 610.  Only k = 1 in batches of 200k and more at cloud points is not
+//   faster (10M tile 500k 848 -> 863, 1M points at 20 a m^2 716 -> 789).
 // ---------------------------------------------------------------------------
 
-constexpr int kGrpQ = (int)kKnnGroupQueries;  // queries per warp: 4 or 8 (query masks are 8 bits)
-// blocks as shared memory allows: ~12.5 KB per warp of 8 queries, ~6.5 KB per warp of 4
-// (8 blocks of 4 warps: 32 warps per SM at up to 64 registers)
-constexpr int kGrpWarps = kGrpQ == 8 ? 2 : 4;
-constexpr int kGrpMinBlocks = 8;
+constexpr int kGrpWarps = 4;
 constexpr int kGrpThreads = 32 * kGrpWarps;
-constexpr int kGrpStack = 88;
-// provisional threshold / previous group's largest k-th distance (10M-point
-// tile, k = 50: 1.15 -> 4.28 ms, 1.2 -> 4.04, 1.3 -> 3.83, 1.4 -> 3.78, 1.5 -> 3.79;
-// results are the same for every factor: a threshold too small hands the query back)
-constexpr double kGrpSeed = 1.4;
+constexpr int kGrpStack = 200;        // nodes: 60 while four are taken at a time, then 7 more a level at most
+constexpr uint32_t kGrpRanges = 64;   // ranges gathered before they are tested
+constexpr int kScanBlocks = 2;        // 32-point blocks in flight (k = 50, 500k: 1 3.02 ms, 2 2.85, 4 3.22)
+constexpr double kGrpSeed = 1.5;      // provisional threshold / largest recent k-th distance of the run
+constexpr double kSeedFade = 0.95;    // what an earlier k-th distance counts for a query later (0.7: +8 % at k = 10)
+constexpr uint32_t kBinMany = 48;
 static_assert(kKnnHeadStride >= 2, "the groups between heads are numbered modulo kKnnHeadStride - 1");
 
 struct KnnGroupArgs {
     SearchReq single;                 // one request (grp == null)
     const DynGroup* grp;              // a batch group: sizes and requests on the device
-    uint64_t packets;                 // single: groups of kGrpQ queries
-    const uint32_t* order;            // visiting order (global query positions)
+    uint64_t packets;                 // single: queries
+    const uint32_t* order;            // visiting order (global query positions), or null
     uint32_t bucket;
+    uint32_t cap;                     // pairs of a query's buffer (a multiple of 32, at least k + 32 kScanBlocks)
+    uint32_t bins;                    // bins of the ranking (a multiple of 128)
     uint32_t* idx;
     double* d2;
     uint32_t* counts;
     uint32_t* err;
-    double est;                       // provisional-threshold factor (0: off, also no seeding)
+    double est;                       // > 0: groups are seeded; 0: every query starts from its own node
     uint32_t* packet_ctr;             // [0] runs of `chunk` groups, [1] single groups at the end, [2] heads
     uint32_t chunk;                   // consecutive groups per fetch (>= 1)
-    uint32_t head_stride;             // S > 1: every S-th group is a head, taken first (0: no heads)
+    uint32_t heads;                   // 1: every kKnnHeadStride-th query is a head, taken first
     double* head_kth;                 // per head: the largest k-th distance it found (NaN: not yet, < 0: none)
     unsigned long long* stats;        // FP32 filter: point tests, FP64 tests, band hits (may be null)
-    uint32_t* fb_list;                // queries left to k_knn_reg (global positions; a batch group's
+    uint32_t* fb_list;                // queries left to the sorted-list kernels (global positions; a batch group's
                                       // entries start at its q_begin)
     unsigned long long* fb_count;
 };
@@ -795,30 +812,299 @@ __device__ __forceinline__ float knn_f32_threshold(double thr, double ab) {
     return __double2float_ru(thr + 2.0 * err);
 }
 
-template <int R, int MULTI, bool F32>
-__global__ void __launch_bounds__(kGrpThreads, kGrpMinBlocks) k_knn_group(KnnGroupArgs a) {
-    constexpr int G = kGrpQ;
-    constexpr int LC = 32 * R;
-    __shared__ double s_ld[kGrpWarps][G][LC];
-    __shared__ uint32_t s_li[kGrpWarps][G][LC];
-    __shared__ double s_bd[kGrpWarps][G][32];
-    __shared__ uint32_t s_bi[kGrpWarps][G][32];
-    __shared__ double s_q[kGrpWarps][G][3];
-    __shared__ double s_thr[kGrpWarps][G];
-    __shared__ uint32_t s_thri[kGrpWarps][G];
-    __shared__ uint32_t s_nl[kGrpWarps][G];
-    __shared__ uint32_t s_nb[kGrpWarps][G];
-    __shared__ uint32_t s_qg[kGrpWarps][G];
-    // FP32 filter: query - box centre in FP32 with the query's FP32 threshold in w,
-    // and the query's A + B (box radius + |query - centre|_inf) for new thresholds
-    __shared__ float4 s_qf[F32 ? kGrpWarps : 1][G];
-    __shared__ double s_qab[F32 ? kGrpWarps : 1][G];
-    unsigned long long f_tests = 0, f_64 = 0, f_band = 0;
-    __shared__ uint32_t st_a[kGrpWarps][kGrpStack];
-    __shared__ uint32_t st_b[kGrpWarps][kGrpStack];
-    __shared__ __half st_lb[kGrpWarps][kGrpStack][G];  // per-query bounds, rounded down to FP16
-    __shared__ uint8_t st_d[kGrpWarps][kGrpStack];
-    __shared__ uint8_t st_m[kGrpWarps][kGrpStack];
+// Squared distances (>= 0, or +inf) to bins, non-decreasing: linear in the
+// distance (shift < 0), or in the bits of its FP32 value (its logarithm).
+struct BinMap {
+    float scale;
+    uint32_t lo;
+    int shift;
+    __device__ __forceinline__ uint32_t bin(double d, uint32_t bins) const {
+        if (shift < 0) {
+            const int b = (int)((float)d * scale);  // NaN (inf * 0) converts to 0
+            return (uint32_t)b < bins ? (uint32_t)b : bins - 1;
+        }
+        const uint32_t v = __float_as_uint((float)d);
+        const uint32_t b = v < lo ? 0u : (v - lo) >> shift;
+        return b < bins ? b : bins - 1;
+    }
+};
+
+// Bins of the n pairs at d, none above `top` (one warp): hist[b] becomes the number of pairs below bin b.
+__device__ __forceinline__ BinMap knn_bin_pairs(const double* d, uint32_t n, double top, uint32_t* hist,
+                                                uint32_t bins) {
+    const int lane = threadIdx.x & 31;
+    BinMap m;
+    m.scale = top > 0.0 && top < (double)INFINITY ? (float)bins / (float)top : 0.0f;
+    m.lo = 0;
+    m.shift = -1;
+    uint4* h4 = reinterpret_cast<uint4*>(hist);  // 128 bins a step, four on a lane
+#pragma unroll 1
+    for (int tries = 0;; ++tries) {
+        __syncwarp();
+#pragma unroll 1
+        for (uint32_t b = 0; b < bins; b += 128) h4[b / 4 + lane] = make_uint4(0u, 0u, 0u, 0u);
+        __syncwarp();
+#pragma unroll 1
+        for (uint32_t e = lane; e < n; e += 32) atomicAdd(&hist[m.bin(d[e], bins)], 1u);
+        __syncwarp();
+        uint32_t below = 0, most = 0;
+#pragma unroll 1
+        for (uint32_t b = 0; b < bins; b += 128) {
+            uint4 c = h4[b / 4 + lane];
+            const uint32_t sum = c.x + c.y + c.z + c.w;
+            most = max(most, max(max(c.x, c.y), max(c.z, c.w)));
+            uint32_t ex = sum;
+#pragma unroll
+            for (int off = 1; off < 32; off <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, ex, off);
+                if (lane >= off) ex += y;
+            }
+            const uint32_t all = __shfl_sync(0xffffffffu, ex, 31);
+            ex += below - sum;
+            below += all;
+            c.w = ex + c.x + c.y + c.z;
+            c.z = ex + c.x + c.y;
+            c.y = ex + c.x;
+            c.x = ex;
+            h4[b / 4 + lane] = c;
+        }
+        if (tries == 0 && __any_sync(0xffffffffu, most > kBinMany)) {
+            // over the logarithm of the distances instead
+            uint32_t lo = 0xffffffffu, hi = 0;
+#pragma unroll 1
+            for (uint32_t e = lane; e < n; e += 32) {
+                const uint32_t v = __float_as_uint((float)d[e]);  // zero (the query itself) goes to the first bin
+                if (v) lo = v < lo ? v : lo;
+                hi = v > hi ? v : hi;
+            }
+            m.lo = __reduce_min_sync(0xffffffffu, lo);
+            hi = __reduce_max_sync(0xffffffffu, hi);
+            m.shift = hi > m.lo ? 32 - __clz((hi - m.lo) / bins) : 0;  // (hi - lo) >> shift < bins
+            continue;
+        }
+        __syncwarp();
+        return m;
+    }
+}
+
+// The K-th smallest of the n squared distances at d as FP32 bits: radix selection, seven bits a pass.
+__device__ __noinline__ uint32_t knn_kth_bits(const double* d, uint32_t n, uint32_t K, uint32_t* hist) {
+    const int lane = threadIdx.x & 31;
+    uint4* h4 = reinterpret_cast<uint4*>(hist);
+    uint32_t prefix = 0, left = K;  // the bits so far; the K-th is the left-th smallest of those that begin so
+#pragma unroll 1
+    for (int shift = 25; shift >= -3; shift -= 7) {
+        const int sh = shift < 0 ? 0 : shift, bits = shift < 0 ? 4 : 7;
+        __syncwarp();
+        h4[lane] = make_uint4(0u, 0u, 0u, 0u);
+        __syncwarp();
+#pragma unroll 1
+        for (uint32_t e = lane; e < n; e += 32) {
+            const unsigned long long v = __float_as_uint((float)d[e]);
+            if ((v >> (sh + bits)) == prefix) atomicAdd(&hist[(uint32_t)(v >> sh) & ((1u << bits) - 1u)], 1u);
+        }
+        __syncwarp();
+        const uint4 c = h4[lane];
+        const uint32_t sum = c.x + c.y + c.z + c.w;
+        uint32_t in = sum;
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, in, off);
+            if (lane >= off) in += y;
+        }
+        const int at = __ffs(__ballot_sync(0xffffffffu, in >= left)) - 1;  // (n >= K: some lane)
+        uint32_t r = left - (in - sum), digit = 4 * lane;
+        if (r > c.x) {
+            r -= c.x;
+            ++digit;
+            if (r > c.y) {
+                r -= c.y;
+                ++digit;
+                if (r > c.z) {
+                    r -= c.z;
+                    ++digit;
+                }
+            }
+        }
+        left = __shfl_sync(0xffffffffu, r, at);
+        prefix = (prefix << bits) | __shfl_sync(0xffffffffu, digit, at);
+    }
+    __syncwarp();
+    return prefix;
+}
+
+// A full buffer of n >= K pairs: its K smallest are kept, at the front, with the others of the K-th's bin;
+// returns how many pairs those are and the largest of them.  More than `most` of them: the bins are given up
+// for the K-th distance itself (to FP32).  Out of line: the walks that call it stay short enough for the
+// instruction cache.
+struct KnnCut {
+    double top;
+    uint32_t n;
+};
+__device__ __noinline__ KnnCut knn_cut(double* d, uint32_t* ix, uint32_t n, double top, uint32_t K, uint32_t most,
+                                       uint32_t* hist, uint32_t bins) {
+    const int lane = threadIdx.x & 31;
+    __syncwarp();
+    if (!(top < (double)INFINITY)) {
+        top = 0.0;
+#pragma unroll 1
+        for (uint32_t e = lane; e < n; e += 32) top = fmax(top, d[e]);
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) top = fmax(top, __shfl_xor_sync(0xffffffffu, top, off));
+    }
+    const BinMap bm = knn_bin_pairs(d, n, top, hist, bins);
+    // pairs below the first bin that starts at or past K (hist ascends)
+    uint32_t kept = n;
+#pragma unroll 1
+    for (uint32_t b = lane; b < bins; b += 32) kept = hist[b] >= K ? min(kept, hist[b]) : kept;
+    kept = __reduce_min_sync(0xffffffffu, kept);
+    const bool exact = kept > most;
+    const uint32_t kth = exact ? knn_kth_bits(d, n, K, hist) : 0u;
+    KnnCut c;
+    c.n = 0;
+    c.top = 0.0;
+#pragma unroll 1
+    for (uint32_t t = 0; t < n; t += 32) {
+        const uint32_t e = t + lane;
+        double dd = 0.0;
+        uint32_t ii = 0;
+        bool keep = false;
+        if (e < n) {
+            dd = d[e];
+            ii = ix[e];
+            keep = exact ? __float_as_uint((float)dd) <= kth : hist[bm.bin(dd, bins)] < K;
+        }
+        const uint32_t kb = __ballot_sync(0xffffffffu, keep);
+        if (keep) {  // at or below the lanes' own positions
+            const uint32_t o = c.n + __popc(kb & lanemask_lt());
+            d[o] = dd;
+            ix[o] = ii;
+            c.top = fmax(c.top, dd);
+        }
+        c.n += __popc(kb);
+        __syncwarp();
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) c.top = fmax(c.top, __shfl_xor_sync(0xffffffffu, c.top, off));
+    return c;
+}
+
+// Bytes of dynamic shared memory of one warp.
+__host__ __device__ constexpr size_t knn_group_bytes(uint32_t cap, uint32_t bins) {
+    return (size_t)cap * 12 + (size_t)bins * 4 + (size_t)cap * 2;
+}
+
+// A cold query's first points: nodes and ranges taken best first (the smallest bound of all that are open, as
+// octants are thin slabs and a depth-first walk would leave a near one for last) until the ranges (to `list`)
+// hold knn_near_points(K) points.  An entry is a node's first child and their depth, or a range's node and depth 255.
+// Returns when the list is full; the state is carried from call to call.
+__host__ __device__ constexpr uint32_t knn_near_points(uint32_t K) { return K <= 256 ? 2 * K : K + K / 2; }
+struct KnnNear {
+    int open;        // open entries
+    uint32_t taken;  // points of the ranges so far
+    uint32_t m;      // ranges of this call
+};
+__device__ __noinline__ KnnNear knn_near_ranges(const uint32_t* offsets, const uint2* ranges, const double* centers,
+                                                const double (*radii)[3], double x, double y, double z, uint32_t K,
+                                                uint32_t bucket, KnnNear st, uint32_t* fcs, uint8_t* depths,
+                                                uint16_t* keys, uint2* list) {
+    const int lane = threadIdx.x & 31;
+    const double p[3] = {x, y, z};
+    st.m = 0;
+#pragma unroll 1
+    while (st.open > 0 && st.taken < knn_near_points(K) && st.m < kGrpRanges) {
+        uint32_t key = 0xffffffffu;
+        int at = 0;
+#pragma unroll 1
+        for (int t = lane; t < st.open; t += 32)
+            if (keys[t] < key) {
+                key = keys[t];
+                at = t;
+            }
+        const uint32_t least = __reduce_min_sync(0xffffffffu, key);
+        at = __shfl_sync(0xffffffffu, at, __ffs(__ballot_sync(0xffffffffu, key == least)) - 1);
+        const uint32_t fc = fcs[at], depth = depths[at];
+        --st.open;
+        __syncwarp();
+        if (lane == 0) {  // the last entry takes its place
+            fcs[at] = fcs[st.open];
+            depths[at] = depths[st.open];
+            keys[at] = keys[st.open];
+        }
+        if (depth == 255u) {
+            const uint2 rg = ranges[fc];
+            if (lane == 0) list[st.m] = rg;
+            ++st.m;
+            st.taken += rg.y - rg.x;
+            __syncwarp();
+            continue;
+        }
+        const uint32_t child = fc + (lane & 7);
+        const uint2 rg = ranges[child];
+        const uint32_t cfc = offsets[child], n = rg.y - rg.x;
+        const float lb = (float)dist_po(p, centers + 3ull * child, radii[depth]);
+        const bool some = lane < 8 && n, whole = cfc == 0 || n <= bucket;
+        const uint32_t sm = __ballot_sync(0xffffffffu, some);
+        __syncwarp();
+        if (some) {
+            const int to = st.open + __popc(sm & lanemask_lt());
+            fcs[to] = whole ? child : cfc;
+            depths[to] = whole ? (uint8_t)255 : (uint8_t)(depth + 1);
+            keys[to] = (uint16_t)(__float_as_uint(lb) >> 16);
+        }
+        st.open += __popc(sm);
+        __syncwarp();
+        if (st.open + 7 > kGrpStack) {
+            // no room for the next node's children: the far entries go (any K points bound the K-th distance)
+            uint32_t most = 0;
+#pragma unroll 1
+            for (int t = lane; t < st.open; t += 32) most = max(most, (uint32_t)keys[t]);
+            float limit = __uint_as_float(__reduce_max_sync(0xffffffffu, most) << 16);
+#pragma unroll 1
+            for (int tries = 0; st.open > kGrpStack / 2 && tries < 64; ++tries) {
+                limit *= 0.5f;
+                int left = 0;
+#pragma unroll 1
+                for (int t = 0; t < st.open; t += 32) {
+                    uint32_t f = 0;
+                    uint16_t k = 0xffff;
+                    uint8_t d = 0;
+                    if (t + lane < st.open) {
+                        f = fcs[t + lane];
+                        d = depths[t + lane];
+                        k = keys[t + lane];
+                    }
+                    const bool stay = __uint_as_float((uint32_t)k << 16) <= limit;  // (0xffff is no number)
+                    const uint32_t sb = __ballot_sync(0xffffffffu, stay);
+                    if (stay) {  // at or below the lanes' own positions
+                        const int to = left + __popc(sb & lanemask_lt());
+                        fcs[to] = f;
+                        depths[to] = d;
+                        keys[to] = k;
+                    }
+                    left += __popc(sb);
+                    __syncwarp();
+                }
+                st.open = left;
+            }
+            if (st.open + 7 > kGrpStack) st.open = kGrpStack - 8;
+        }
+    }
+    return st;
+}
+
+template <int MULTI, bool F32>
+__global__ void __launch_bounds__(kGrpThreads, 7) k_knn_group(KnnGroupArgs a) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ uint32_t s_n[kGrpWarps];               // pairs in the buffer
+    __shared__ uint32_t st_fc[kGrpWarps][kGrpStack];  // first child of a node
+    __shared__ uint8_t st_d[kGrpWarps][kGrpStack];    // its children's depth
+    __shared__ uint16_t st_key[kGrpWarps][kGrpStack];  // its bound (upper half of the FP32 bits), for cold queries
+    __shared__ uint2 s_rg[kGrpWarps][kGrpRanges];
+    // the nodes that the warp's last walks passed one by one from the root (centre, first child), by
+    // depth: a walk starts at the deepest that holds its whole ball
+    __shared__ double s_pc[kGrpWarps][kMaxDepth + 1][3];
+    __shared__ uint32_t s_pf[kGrpWarps][kMaxDepth + 1];
     // level radii: per warp for a table of clouds, once per block for one cloud
     __shared__ double s_rad[MULTI == 1 ? kGrpWarps : 1][kMaxDepth + 1][3];
     __shared__ CloudView s_view[MULTI == 1 ? kGrpWarps : 1];
@@ -827,27 +1113,26 @@ __global__ void __launch_bounds__(kGrpThreads, kGrpMinBlocks) k_knn_group(KnnGro
     double (*s_radii)[3] = s_rad[MULTI == 1 ? warp : 0];
     if (MULTI != 1) {
         const double* gr = &a.single.cv.geom->radii[0][0];
+#pragma unroll 1
         for (int t = threadIdx.x; t < (kMaxDepth + 1) * 3; t += kGrpThreads) (&s_rad[0][0][0])[t] = gr[t];
         __syncthreads();
     }
-    double (*ld)[LC] = s_ld[warp];
-    uint32_t (*li)[LC] = s_li[warp];
-    double (*bd)[32] = s_bd[warp];
-    uint32_t (*bi)[32] = s_bi[warp];
-    double (*qs)[3] = s_q[warp];
-    double* thr = s_thr[warp];
-    uint32_t* thri = s_thri[warp];
-    uint32_t* nls = s_nl[warp];
-    uint32_t* nbs = s_nb[warp];
-    uint32_t* sa = st_a[warp];
-    uint32_t* sb = st_b[warp];
-    __half (*slb)[G] = st_lb[warp];
+    const uint32_t cap = a.cap, bins = a.bins;
+    unsigned char* mine = smem + (size_t)warp * knn_group_bytes(cap, bins);
+    double* bd = reinterpret_cast<double*>(mine);
+    uint32_t* bi = reinterpret_cast<uint32_t*>(mine + (size_t)cap * 8);
+    uint32_t* hist = bi + cap;
+    uint16_t* ord = reinterpret_cast<uint16_t*>(hist + bins);
+    uint32_t* sf = st_fc[warp];
     uint8_t* sdp = st_d[warp];
-    uint8_t* smk = st_m[warp];
+    uint16_t* sk = st_key[warp];
+    uint2* list = s_rg[warp];
+    uint32_t* np = &s_n[warp];
+    unsigned long long f_tests = 0, f_64 = 0, f_band = 0;
     uint32_t cur_cloud = 0xffffffffu;
     const SearchReq* reqs = nullptr;
     uint32_t nreq = 1;
-    // query positions and group indices of a launch fit 32 bits (positions are u32 in the order arrays)
+    // query positions of a launch fit 32 bits (positions are u32 in the order arrays)
     uint32_t packets = (uint32_t)a.packets;
     uint32_t fb_base = 0;  // the fallback entries of a batch group start at its first position
     if (MULTI) {
@@ -856,28 +1141,30 @@ __global__ void __launch_bounds__(kGrpThreads, kGrpMinBlocks) k_knn_group(KnnGro
         packets = (uint32_t)a.grp->packets;
         fb_base = (uint32_t)a.grp->q_begin;
     }
-    // lane roles at an internal node: LPQ lanes per query qj, CPL children each
-    constexpr int LPQ = 32 / G, CPL = 8 / LPQ;
-    static_assert(G == 4 || G == 8, "4 or 8 queries per warp");
-    const int qj = lane / LPQ, cs = lane % LPQ;
-    // heads (every S-th group) go out first, one at a time; the other groups are
-    // slots: slot s is the s-th group that is not a head (every group without heads)
-    const uint32_t S = a.head_stride;
-    const uint32_t n_heads = S ? (packets + S - 1) / S : 0;
+    // heads (every S-th query) go out first, one at a time; the others are slots:
+    // slot s is the s-th query that is not a head (every query without heads)
+    constexpr uint32_t S = kKnnHeadStride;
+    const bool heads = a.heads != 0;
+    const uint32_t n_heads = heads ? (packets + S - 1) / S : 0;
     const uint32_t slots = packets - n_heads;
     bool heads_left = n_heads != 0;
     // slots [0, p_chunked) go out in chunks, the rest one at a time
     const uint32_t nw = gridDim.x * kGrpWarps;
-    const uint32_t chunk = a.chunk;
+    // (runs no longer than leave every warp four of them)
+    const uint32_t chunk = max(1u, min(2 * a.chunk, slots / (4 * nw)));
     const uint32_t p_chunked = (chunk > 1 && slots > 2 * nw) ? (slots - 2 * nw) / chunk * chunk : 0;
     uint32_t next = 0, chunk_end = 0;
-    // seed: the previous group's largest k-th distance (< 0: none), its slot and request
-    double seed_thr = -1.0;
-    uint32_t seed_slot = 0;
-    uint32_t seed_ri = 0;
+    double (*pc)[3] = s_pc[warp];
+    uint32_t* pf = s_pf[warp];
+    uint32_t path_len = 0;
+    // the warp's last slot and request; the query after it on the curve, read ahead (lane t < 3: coordinate t)
+    uint32_t seed_slot = 0xfffffffeu, seed_ri = 0;
+    uint32_t ahead_pos = 0xffffffffu, ahead_q = 0;
+    double ahead_c = 0.0;
+    double run_kth = -1.0;  // the largest recent k-th distance of the run (< 0: none)
 
     for (;;) {
-        uint32_t slot = 0xffffffffu;  // the head's group index when a head
+        uint32_t slot = 0xffffffffu;  // the head's number when a head
         bool head = false;
         if (heads_left) {
             uint32_t h = 0;
@@ -909,10 +1196,11 @@ __global__ void __launch_bounds__(kGrpThreads, kGrpMinBlocks) k_knn_group(KnnGro
             }
             if (slot >= slots) break;
         }
-        const uint32_t packet = head ? slot * S : !S ? slot : slot + slot / (S - 1) + 1;
+        const uint32_t packet = head ? slot * S : !heads ? slot : slot + slot / (S - 1) + 1;
         uint32_t ri = 0;
-        if (MULTI) {  // the request of this group (packet_begin ascending over the table)
+        if (MULTI) {  // the request of this query (packet_begin ascending over the table)
             uint32_t lo = 0, hi = nreq;
+#pragma unroll 1
             while (hi - lo > 1) {
                 const uint32_t mid = (lo + hi) >> 1;
                 if (reqs[mid].packet_begin <= packet) lo = mid;
@@ -920,357 +1208,359 @@ __global__ void __launch_bounds__(kGrpThreads, kGrpMinBlocks) k_knn_group(KnnGro
             }
             ri = lo;
         }
-        if (MULTI == 1 && reqs[ri].cloud_id != cur_cloud) {  // this warp's level radii and cloud follow the group's
+        if (MULTI == 1 && reqs[ri].cloud_id != cur_cloud) {  // this warp's level radii and cloud follow the query's
             __syncwarp();
             const double* gr = &reqs[ri].cv.geom->radii[0][0];
+#pragma unroll 1
             for (int t = lane; t < (kMaxDepth + 1) * 3; t += 32) (&s_radii[0][0])[t] = gr[t];
             if (lane == 0) s_view[warp] = reqs[ri].cv;
             cur_cloud = reqs[ri].cloud_id;
+            path_len = 0;
             __syncwarp();
         }
         const uint32_t K = KRQ(k);
         const uint32_t q_begin = (uint32_t)KRQ(q_begin);
-        const uint32_t pos0 = q_begin + (uint32_t)G * (packet - (uint32_t)KRQ(packet_begin));
-        const uint32_t q_end = (uint32_t)KRQ(q_end);
-        // seed: the group before this one in the warp's run, else (between heads) the
+        const uint32_t pos = q_begin + (packet - (uint32_t)KRQ(packet_begin));
+        // seed: the queries before this one in the warp's run, else (between heads) the
         // nearest head of the same request
-        // heads start from the density estimate
-        double seed = (a.est > 0.0 && !head && seed_thr >= 0.0 && slot == seed_slot + 1 && ri == seed_ri)
-                          ? seed_thr : -1.0;
-        if (seed < 0.0 && a.est > 0.0 && S && !head) {
+        if (head || slot != seed_slot + 1 || ri != seed_ri) run_kth = -1.0;
+        double seed = run_kth;
+        if (seed < 0.0 && heads && !head) {
             const uint32_t pb = (uint32_t)KRQ(packet_begin);
-            const uint32_t pe = pb + (uint32_t)((KRQ(q_end) - KRQ(q_begin) + G - 1) / G);
+            const uint32_t pe = pb + (uint32_t)(KRQ(q_end) - KRQ(q_begin));
             const uint32_t hlo = packet / S, hhi = hlo + 1;  // heads hlo S < packet < hhi S
             const bool lo_ok = hlo * S >= pb, hi_ok = hhi < n_heads && hhi * S < pe;
             const bool use_hi = hi_ok && (!lo_ok || hhi * S - packet < packet - hlo * S);
             // a head not finished yet reads NaN: no seed (nothing waits for it)
             if (use_hi || lo_ok) seed = __ldcg(&a.head_kth[use_hi ? hhi : hlo]);
-            if (!(seed >= 0.0)) seed = -1.0;
         }
-        const bool seeded = seed >= 0.0;
-        // lanes j < G: load query j, reset its state
-        bool valid = false;
-        if (lane < G) {
-            const uint64_t pos = pos0 + lane;
-            valid = pos < q_end;
-            const uint64_t q = valid ? (uint64_t)a.order[pos] : q_begin;
-            const uint64_t ql = q - q_begin;
-            const double* qc = KRQ(centers);
-            qs[lane][0] = qc[3 * ql];
-            qs[lane][1] = qc[3 * ql + 1];
-            qs[lane][2] = qc[3 * ql + 2];
-            thr[lane] = seeded ? kGrpSeed * seed : (double)INFINITY;
-            thri[lane] = 0xffffffffu;  // with the pair order a provisional threshold accepts d <= thr
-            nls[lane] = 0;
-            nbs[lane] = 0;
-            s_qg[warp][lane] = (uint32_t)q;
-            if constexpr (F32) {
-                const BoxD* bx = KRQV(box);
-                const double bqx = dsub(qc[3 * ql], bx->center[0]);
-                const double bqy = dsub(qc[3 * ql + 1], bx->center[1]);
-                const double bqz = dsub(qc[3 * ql + 2], bx->center[2]);
-                const double A = smax(smax(bx->radii[0], bx->radii[1]), bx->radii[2]);
-                const double B = smax(smax(fabs(bqx), fabs(bqy)), fabs(bqz));
-                const double ab = (A + B) * (1.0 + 1.0e-12);
-                s_qab[warp][lane] = ab;
-                s_qf[warp][lane] = make_float4((float)bqx, (float)bqy, (float)bqz, knn_f32_threshold(thr[lane], ab));
-            }
+        bool cold = !(a.est > 0.0 && seed >= 0.0);
+        if (pos != ahead_pos) {
+            ahead_q = a.order ? a.order[pos] : pos;
+            ahead_c = lane < 3 ? KRQ(centers)[3ull * (ahead_q - q_begin) + lane] : 0.0;
         }
-        for (int t = lane; t < G * LC; t += 32) {
-            (&ld[0][0])[t] = INFINITY;
-            (&li[0][0])[t] = 0xffffffffu;
+        const uint64_t q = ahead_q;
+        const uint64_t ql = q - q_begin;
+        const double p[3] = {__shfl_sync(0xffffffffu, ahead_c, 0), __shfl_sync(0xffffffffu, ahead_c, 1),
+                             __shfl_sync(0xffffffffu, ahead_c, 2)};
+        ahead_pos = next < chunk_end && pos + 1 < (uint32_t)KRQ(q_end) && (!heads || (packet + 1) % S) ? pos + 1 : 0xffffffffu;
+        if (ahead_pos != 0xffffffffu) ahead_q = a.order ? a.order[ahead_pos] : ahead_pos;
+        double thr = cold ? (double)INFINITY : kGrpSeed * seed;
+        // FP32 filter: query - box centre in FP32, the FP32 threshold, and A + B (box radius +
+        // |query - centre|_inf) for new thresholds
+        float qx = 0.0f, qy = 0.0f, qz = 0.0f, tf = 0.0f;
+        double ab = 0.0;
+        if constexpr (F32) {
+            const BoxD* bx = KRQV(box);
+            const double bqx = dsub(p[0], bx->center[0]);
+            const double bqy = dsub(p[1], bx->center[1]);
+            const double bqz = dsub(p[2], bx->center[2]);
+            const double A = smax(smax(bx->radii[0], bx->radii[1]), bx->radii[2]);
+            const double B = smax(smax(fabs(bqx), fabs(bqy)), fabs(bqz));
+            ab = (A + B) * (1.0 + 1.0e-12);
+            qx = (float)bqx;
+            qy = (float)bqy;
+            qz = (float)bqz;
         }
-        const uint32_t vm = __ballot_sync(0xffffffffu, valid) & ((1u << G) - 1u);
-        uint32_t est_pend = (a.est > 0.0 && !seeded) ? vm : 0u, est_used = seeded ? vm : 0u;
-        bool failed = false;
-
-        // Merge query j's buffer (nb > 0 pairs) into its list (warp-uniform call).
-        auto merge = [&](int j, uint32_t nb) {
-            const double cdv = (lane < (int)nb) ? bd[j][lane] : (double)INFINITY;
-            const uint32_t civ = (lane < (int)nb) ? bi[j][lane] : 0xffffffffu;
-            RegList<R> L;
-            if (nls[j] == 0) {  // an empty list (every entry +inf): the sorted candidates are the merge
-                double sd = cdv;
-                uint32_t si = civ;
-                warp_sort32(sd, si);
-                L.d[0] = sd;
-                L.i[0] = si;
-#pragma unroll
-                for (int r = 1; r < R; ++r) {
-                    L.d[r] = INFINITY;
-                    L.i[r] = 0xffffffffu;
-                }
-            } else {
-#pragma unroll
-                for (int r = 0; r < R; ++r) {
-                    L.d[r] = ld[j][r * 32 + lane];
-                    L.i[r] = li[j][r * 32 + lane];
-                }
-                reglist_merge32<R>(L, cdv, civ);
-            }
-#pragma unroll
-            for (int r = 0; r < R; ++r) {
-                ld[j][r * 32 + lane] = L.d[r];
-                li[j][r * 32 + lane] = L.i[r];
-            }
-            uint32_t nl = nls[j] + nb;
-            if (nl > K) nl = K;
-            double td = 0.0;
-            uint32_t ti = 0;
-            if (nl == K) reglist_kth<R>(L, K, td, ti);
-            __syncwarp();
-            if (lane == 0) {
-                nls[j] = nl;
-                nbs[j] = 0;
-                if (nl == K) {
-                    thr[j] = td;
-                    thri[j] = ti;
-                    if constexpr (F32) s_qf[warp][j].w = knn_f32_threshold(td, s_qab[warp][j]);
-                }
-            }
-            __syncwarp();
-        };
-
-        // root (bound 0)
-        {
-            const uint32_t fc0 = KRQV(offsets)[0];
-            const uint2 rg0 = KRQV(ranges)[0];
-            const bool scan0 = fc0 == 0 || rg0.y - rg0.x <= a.bucket;
-            if (lane == 0) {
-                sa[0] = scan0 ? rg0.x : fc0;
-                sb[0] = scan0 ? rg0.y : 0xffffffffu;
-                sdp[0] = 0;
-                smk[0] = (uint8_t)vm;
-            }
-            if (lane < G) slb[0][lane] = __float2half_rz(0.0f);
-        }
-        __syncwarp();
-        int sp = vm ? 1 : 0;
-        while (sp > 0) {
-            --sp;
-            const uint32_t ea = sa[sp], eb = sb[sp];
-            const uint32_t depth = sdp[sp];
-            bool act = false;
-            if (lane < G) act = ((smk[sp] >> lane) & 1u) && !((double)__half2float(slb[sp][lane]) > thr[lane]);
-            const uint32_t m = __ballot_sync(0xffffffffu, act) & ((1u << G) - 1u);
-            __syncwarp();
-            if (!m) continue;
-            if (eb != 0xffffffffu) {
-                // a range [ea, eb)
-                const uint32_t pend = est_pend & m;
-                if (pend) {
-                    const double area = 4.0 * s_radii[depth][0] * s_radii[depth][1];
-                    if (area > 0.0) {
-                        if (lane < G && ((pend >> lane) & 1u)) {
-                            thr[lane] = a.est * (double)K * area / (3.14159265358979323846 * (double)(eb - ea));
-                            thri[lane] = 0xffffffffu;  // with the pair order this accepts d <= thr
-                            if constexpr (F32) s_qf[warp][lane].w = knn_f32_threshold(thr[lane], s_qab[warp][lane]);
+        bool ok = true;       // false: left to the fallback
+        double kth = -1.0;    // the k-th distance, when k pairs were found
+#pragma unroll 1
+        for (int attempt = 0; attempt < 2; ++attempt) {
+            // phase 0 (cold): the points of the query's own node, for a threshold; phase 1: every point
+            // within the threshold
+#pragma unroll 1
+            for (int phase = cold ? 0 : 1; phase < 2; ++phase) {
+                int sp = 0;
+                uint32_t m = 0, taken = 0;  // ranges gathered; points of phase 0
+                uint2 rg0 = make_uint2(0u, 0u);
+                uint32_t fc0 = 0, depth0 = 1;  // children to judge first, and their depth
+                if (phase == 0) {
+                    thr = (double)INFINITY;
+                    fc0 = KRQV(offsets)[0];
+                    if (fc0) {  // the root
+                        if (lane == 0) {
+                            sf[0] = fc0;
+                            sdp[0] = 1;
+                            sk[0] = 0;
                         }
-                        est_used |= pend;
+                        sp = 1;
                     }
-                    est_pend &= ~pend;
+                } else if (path_len) {
+                    // the deepest node of the path that holds the whole ball, by a margin far above the rounding
+                    // of coordinates and node boxes: nothing outside it can be within the threshold
+                    const double r = (double)(sqrtf((float)thr) * 1.000001f);
+                    bool holds = (uint32_t)lane < path_len;
+                    if (holds && lane) {
+#pragma unroll
+                        for (int t = 0; t < 3; ++t) {
+                            const double h = s_radii[lane][t], c = pc[lane][t];
+                            holds = holds && fabs(p[t] - c) + r + 1.0e-12 * (fabs(p[t]) + fabs(c) + h) <= h;
+                        }
+                    }
+                    path_len = 32 - __clz(__ballot_sync(0xffffffffu, holds));
+                    fc0 = pf[path_len - 1];
+                    depth0 = path_len;
+                } else {
+                    rg0 = KRQV(ranges)[0];
+                    fc0 = KRQV(offsets)[0];
+                    if (fc0) {  // the root
+                        if (lane == 0) pf[0] = fc0;
+                        path_len = 1;
+                    }
+                }
+                if constexpr (F32) tf = knn_f32_threshold(thr, ab);
+                if (phase == 0) {
+                } else if (fc0 == 0) {
+                    if (lane == 0) list[0] = rg0;
+                    m = 1;
+                } else {
+                    if (lane == 0) {
+                        sf[0] = fc0;
+                        sdp[0] = (uint8_t)depth0;
+                    }
+                    sp = 1;
+                }
+                if (lane == 0) *np = 0;
+                __syncwarp();
+#pragma unroll 1
+                for (;;) {
+                    if (phase == 0) {
+                        const KnnNear st = knn_near_ranges(KRQV(offsets), KRQV(ranges), KRQV(centers), s_radii, p[0], p[1],
+                                                           p[2], K, a.bucket, KnnNear{sp, taken, 0}, sf, sdp, sk, list);
+                        sp = st.taken < knn_near_points(K) ? st.open : 0;
+                        taken = st.taken;
+                        m = st.m;
+                    }
+                    if (phase == 0 || sp == 0 || m > kGrpRanges - 32) {
+                        // the gathered ranges, 32 of them at a time as one run of points: lane l's range holds
+                        // [first, end) of the run, starting at point first + base
+#pragma unroll 1
+                        for (uint32_t r0 = 0; r0 < m; r0 += 32) {
+                            const uint2 rg = r0 + lane < m ? list[r0 + lane] : make_uint2(0u, 0u);
+                            const uint32_t len = rg.y - rg.x;
+                            uint32_t end = len;
+#pragma unroll
+                            for (int off = 1; off < 32; off <<= 1) {
+                                const uint32_t y = __shfl_up_sync(0xffffffffu, end, off);
+                                if (lane >= off) end += y;
+                            }
+                            const uint32_t first = end - len, base = rg.x - first;
+                            const uint32_t total = __shfl_sync(0xffffffffu, end, 31);
+#pragma unroll 1
+                            for (uint32_t b = 0; b < total; b += 32 * kScanBlocks) {
+                                const uint32_t have = *np;
+                                __syncwarp();  // read by every lane before any adds to it
+                                uint32_t i[kScanBlocks];
+                                double px[kScanBlocks], py[kScanBlocks], pz[kScanBlocks];
+                                float4 pt[kScanBlocks];
+#pragma unroll
+                                for (int u = 0; u < kScanBlocks; ++u) {
+                                    const uint32_t bu = b + 32 * u;
+                                    if (u && bu >= total) break;
+                                    // the lane's range: ranges begun before bu, plus those that begin at or below it
+                                    const uint32_t before = __popc(__ballot_sync(0xffffffffu, first < bu));
+                                    const uint32_t starts = __reduce_or_sync(
+                                        0xffffffffu, (len && first - bu < 32u) ? 1u << (first - bu) : 0u);
+                                    const int r = (int)(before + __popc(starts & (2u * (1u << lane) - 1u))) - 1;
+                                    // (lanes past the end read the last point again)
+                                    i[u] = __shfl_sync(0xffffffffu, base, r) + min(bu + lane, total - 1);
+                                    if constexpr (F32) {
+                                        pt[u] = KRQV(crel)[i[u]];
+                                    } else {
+                                        px[u] = KRQV(xs)[i[u]];
+                                        py[u] = KRQV(ys)[i[u]];
+                                        pz[u] = KRQV(zs)[i[u]];
+                                    }
+                                }
+                                if (have + 32 * kScanBlocks > cap) {
+                                    // no room for a whole step: the K smallest pairs (to a bin) are kept, the threshold
+                                    // drops to the largest of them
+                                    KnnCut c = knn_cut(bd, bi, have, thr, K, cap - 32 * kScanBlocks, hist, bins);
+                                    if (c.n + 32 * kScanBlocks > cap) {  // equal distances that fill the buffer
+                                        ok = false;
+                                        c.n = 0;
+                                        c.top = -1.0;  // takes no more points
+                                    }
+                                    __syncwarp();
+                                    if (lane == 0) *np = c.n;
+                                    thr = c.top;
+                                    if constexpr (F32) tf = knn_f32_threshold(thr, ab);
+                                    __syncwarp();
+                                }
+#pragma unroll
+                                for (int u = 0; u < kScanBlocks; ++u) {
+                                    if (u && b + 32 * u >= total) break;
+                                    const bool in = b + 32 * u + lane < total;
+                                    double d = 0.0;
+                                    bool cand = false;
+                                    if constexpr (F32) {
+                                        const float dx = pt[u].x - qx, dy = pt[u].y - qy, dz = pt[u].z - qz;
+                                        const float df = __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmul_rn(dx, dx)));
+                                        if (in) {
+                                            ++f_tests;
+                                            if (!(df > tf)) {  // near the threshold or inside: the exact FP64 test
+                                                d = dist_pp(p[0], p[1], p[2], KRQV(xs)[i[u]], KRQV(ys)[i[u]],
+                                                            KRQV(zs)[i[u]]);
+                                                cand = d <= thr;
+                                                ++f_64;
+                                                f_band += cand ? 0u : 1u;
+                                            }
+                                        }
+                                    } else {
+                                        d = dist_pp(p[0], p[1], p[2], px[u], py[u], pz[u]);
+                                        cand = in && d <= thr;
+                                    }
+                                    if (cand) {
+                                        const uint32_t at = atomicAdd(np, 1u);
+                                        bd[at] = d;
+                                        bi[at] = i[u];
+                                    }
+                                }
+                                __syncwarp();
+                            }
+                        }
+                        m = 0;
+                        if (sp == 0) break;
+                        __syncwarp();
+                        if (phase == 0) continue;
+                    }
+                    // up to four nodes: lane (node lane / 8, child lane % 8)
+                    const int take = sp > 32 ? 1 : sp < 4 ? sp : 4;
+                    const int from = sp - 1 - (lane >> 3);
+                    bool near = false;
+                    uint32_t cfc = 0, cd = 0;
+                    uint2 rg = make_uint2(0u, 0u);
+                    double oc[3] = {0.0, 0.0, 0.0};
+                    if ((lane >> 3) < take) {
+                        cd = sdp[from];
+                        const uint32_t child = sf[from] + (lane & 7);
+                        cfc = KRQV(offsets)[child];
+                        rg = KRQV(ranges)[child];
+#pragma unroll
+                        for (int t = 0; t < 3; ++t) oc[t] = KRQV(centers)[3ull * child + t];
+                        near = !(dist_po(p, oc, s_radii[cd]) > thr) && rg.y != rg.x;
+                    }
+                    const bool whole = cfc == 0 || rg.y - rg.x <= a.bucket;
+                    const uint32_t mr = __ballot_sync(0xffffffffu, near && whole);
+                    const uint32_t mn = __ballot_sync(0xffffffffu, near && !whole);
+                    sp -= take;
+                    if (sp + __popc(mn) > kGrpStack) {
+                        ok = false;
+                        break;
+                    }
+                    if (near) {
+                        if (whole) {
+                            list[m + __popc(mr & lanemask_lt())] = rg;
+                        } else {
+                            const int at = sp + __popc(mn & lanemask_lt());
+                            sf[at] = cfc;
+                            sdp[at] = (uint8_t)(cd + 1);
+                        }
+                    }
+                    if (sp == 0 && m == 0 && mr == 0 && __popc(mn) == 1) {
+                        // one node still, below the path's last: the path goes on with it
+                        const int from_lane = __ffs(mn) - 1;
+                        if (__shfl_sync(0xffffffffu, cd, from_lane) == path_len) {
+                            if (lane == from_lane) {
+                                pf[path_len] = cfc;
+#pragma unroll
+                                for (int t = 0; t < 3; ++t) pc[path_len][t] = oc[t];
+                            }
+                            ++path_len;
+                        }
+                    }
+                    m += __popc(mr);
+                    sp += __popc(mn);
                     __syncwarp();
                 }
-                for (uint32_t b = ea; b < eb; b += 32) {
-                    const uint32_t i = b + lane;
-                    const bool in = i < eb;
-                    double px = 0.0, py = 0.0, pz = 0.0;
-                    float4 pf = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                    bool have64 = !F32;  // the FP32 form reads FP64 coordinates only for points near a threshold
-                    if (in) {
-                        if constexpr (F32) {
-                            pf = KRQV(crel)[i];
-                        } else {
-                            px = KRQV(xs)[i];
-                            py = KRQV(ys)[i];
-                            pz = KRQV(zs)[i];
-                        }
-                    }
-                    if (F32 && lane == 0) f_tests += (unsigned long long)__popc(m) * ((eb - b < 32u) ? (eb - b) : 32u);
-                    uint32_t rem = m;
-                    while (rem) {
-                        const int j = __ffs(rem) - 1;
-                        rem &= rem - 1;
-                        double d = (double)INFINITY;
-                        bool cand = false;
-                        if constexpr (F32) {
-                            const float4 q4 = s_qf[warp][j];
-                            const float dx = pf.x - q4.x, dy = pf.y - q4.y, dz = pf.z - q4.z;
-                            const float df = __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmul_rn(dx, dx)));
-                            if (in && !(df > q4.w)) {  // near the threshold or inside: the exact FP64 test
-                                if (!have64) {
-                                    px = KRQV(xs)[i];
-                                    py = KRQV(ys)[i];
-                                    pz = KRQV(zs)[i];
-                                    have64 = true;
-                                }
-                                d = dist_pp(qs[j][0], qs[j][1], qs[j][2], px, py, pz);
-                                cand = pair_less(d, i, thr[j], thri[j]);
-                                ++f_64;
-                                f_band += cand ? 0u : 1u;
-                            }
-                        } else {
-                            d = dist_pp(qs[j][0], qs[j][1], qs[j][2], px, py, pz);
-                            cand = in && pair_less(d, i, thr[j], thri[j]);
-                        }
-                        uint32_t hb = __ballot_sync(0xffffffffu, cand);
-                        if (!hb) continue;
-                        uint32_t nb = nbs[j];
-                        if (nb + __popc(hb) > 32u) {
-                            merge(j, nb);
-                            nb = 0;
-                            cand = cand && pair_less(d, i, thr[j], thri[j]);
-                            hb = __ballot_sync(0xffffffffu, cand);
-                        }
-                        if (cand) {
-                            const uint32_t slot = nb + __popc(hb & lanemask_lt());
-                            bd[j][slot] = d;
-                            bi[j][slot] = i;
-                        }
-                        __syncwarp();
-                        if (lane == 0) nbs[j] = nb + __popc(hb);
-                        __syncwarp();
-                    }
+                __syncwarp();
+                if (phase == 0) {
+                    if (*np >= K) thr = knn_cut(bd, bi, *np, thr, K, cap - 32 * kScanBlocks, hist, bins).top;
+                    __syncwarp();
                 }
+            }
+            if (!ok) break;
+            const uint32_t n = *np;
+            if (n < K && thr < (double)INFINITY) {  // the seeded threshold was too small
+                ok = attempt == 0;
+                cold = true;
+                __syncwarp();
                 continue;
             }
-            // internal node: lane (qj, cs) judges children cs CPL .. cs CPL + CPL - 1 for query qj
-            const uint32_t fc = ea;
-            const uint32_t cd = depth + 1;
-            const bool qa = (m >> qj) & 1u;
-            double lb[CPL];
-            bool kp[CPL];
-            uint32_t B[CPL];
-            double v[CPL];
-#pragma unroll
-            for (int w = 0; w < CPL; ++w) {
-                lb[w] = INFINITY;
-                kp[w] = false;
-            }
-            if (qa) {
-                const double* c0 = KRQV(centers) + 3ull * (fc + CPL * cs);
-                const double t = thr[qj];
-#pragma unroll
-                for (int w = 0; w < CPL; ++w) {
-                    lb[w] = dist_po(qs[qj], c0 + 3 * w, s_radii[cd]);
-                    kp[w] = !(lb[w] > t);
+            if (ahead_pos != 0xffffffffu && lane < 3) ahead_c = KRQ(centers)[3ull * (ahead_q - q_begin) + lane];
+            const uint64_t o = KRQ(out_begin) + ql * (uint64_t)K;
+            if (lane == 0 && a.counts) a.counts[q] = n < K ? n : K;
+            if (n <= 32) {  // a pair a lane, ranked against each of the others
+                const double dd = (uint32_t)lane < n ? bd[lane] : (double)INFINITY;
+                const uint32_t ii = (uint32_t)lane < n ? bi[lane] : 0xffffffffu;
+                uint32_t rank = 0;
+#pragma unroll 1
+                for (uint32_t t = 0; t < n; ++t)
+                    rank += pair_less(__shfl_sync(0xffffffffu, dd, t), __shfl_sync(0xffffffffu, ii, t), dd, ii);
+                if ((uint32_t)lane >= n) rank = lane;  // empty slots
+                if (rank < K) {
+                    a.idx[o + rank] = ii;
+                    a.d2[o + rank] = dd;
                 }
-            }
-            // smallest accepting bound per child, over the lanes judging the same children
-#pragma unroll
-            for (int w = 0; w < CPL; ++w) {
-                B[w] = __ballot_sync(0xffffffffu, kp[w]);
-                v[w] = kp[w] ? lb[w] : (double)INFINITY;
-            }
-#pragma unroll
-            for (int off = LPQ; off < 32; off <<= 1)
-#pragma unroll
-                for (int w = 0; w < CPL; ++w) v[w] = fmin(v[w], __shfl_xor_sync(0xffffffffu, v[w], off));
-            // lane c < 8: child c's query mask, bound and record
-            const int cc = lane & 7;
-            double key = INFINITY;
-            uint32_t Bw = 0;
-#pragma unroll
-            for (int w = 0; w < CPL; ++w) {
-                const double x = __shfl_sync(0xffffffffu, v[w], cc / CPL);
-                if (cc % CPL == w) {
-                    key = x;
-                    Bw = B[w];
+#pragma unroll 1
+                for (uint32_t t = 32 + lane; t < K; t += 32) {
+                    a.idx[o + t] = 0xffffffffu;
+                    a.d2[o + t] = (double)INFINITY;
                 }
-            }
-            uint32_t cm = 0;
-            uint32_t ca = 0, cb = 0;
-            if (lane < 8) {
-#pragma unroll
-                for (int j = 0; j < G; ++j) cm |= ((Bw >> (LPQ * j + cc / CPL)) & 1u) << j;
-                const uint32_t child = fc + lane;
-                const uint32_t cfc = KRQV(offsets)[child];
-                const uint2 rg = KRQV(ranges)[child];
-                if (cfc && rg.y - rg.x > a.bucket) {
-                    ca = cfc;
-                    cb = 0xffffffffu;
-                } else {
-                    ca = rg.x;
-                    cb = rg.y;
-                    if (rg.y == rg.x) cm = 0;  // an empty leaf holds no candidate
-                }
-            } else {
-                key = INFINITY;
-            }
-            const uint32_t pushm = __ballot_sync(0xffffffffu, lane < 8 && cm != 0);
-            const int np = __popc(pushm);
-            if (sp + np > kGrpStack) {
-                failed = true;
+                const uint32_t kb = __ballot_sync(0xffffffffu, rank == K - 1 && (uint32_t)lane < n);
+                kth = kb ? __shfl_sync(0xffffffffu, dd, 31 - __clz(kb)) : -1.0;
                 break;
             }
-            // nearest on top: slot below every farther (or equal and higher octant) child
-            int pos = 0;
-#pragma unroll
-            for (int o = 0; o < 8; ++o) {
-                const double ol = __shfl_sync(0xffffffffu, key, o);
-                if (((pushm >> o) & 1u) && o != lane && ((ol > key) || (ol == key && o > lane))) ++pos;
-            }
-            const int slot = sp + pos;
-            if (lane < 8 && cm != 0) {
-                sa[slot] = ca;
-                sb[slot] = cb;
-                sdp[slot] = (uint8_t)cd;
-                smk[slot] = (uint8_t)cm;
-            }
-            // per-query bounds of the pushed children, rounded down
-#pragma unroll
-            for (int w = 0; w < CPL; ++w) {
-                const int c = CPL * cs + w;
-                const int sw = __shfl_sync(0xffffffffu, slot, c);
-                if (kp[w] && ((pushm >> c) & 1u)) slb[sw][qj] = __float2half_rd(__double2float_rd(lb[w]));
-            }
+            // rank the pairs and write the K best
+            const BinMap bm = knn_bin_pairs(bd, n, thr, hist, bins);
+#pragma unroll 1
+            for (uint32_t e = lane; e < n; e += 32) ord[atomicAdd(&hist[bm.bin(bd[e], bins)], 1u)] = (uint16_t)e;
             __syncwarp();
-            sp += np;
-        }
-        __syncwarp();
-        // flush the buffers, then write each query's pairs or hand it to the fallback
-        uint32_t rem = vm;
-        while (rem) {
-            const int j = __ffs(rem) - 1;
-            rem &= rem - 1;
-            const uint32_t nb = nbs[j];
-            if (nb) merge(j, nb);
-            const uint32_t nl = nls[j];
-            const uint64_t q = s_qg[warp][j];
-            if (failed || (((est_used >> j) & 1u) && nl < K)) {
-                if (lane == 0) {
-                    const unsigned long long f = atomicAdd(a.fb_count, 1ull);
-                    a.fb_list[fb_base + f] = (uint32_t)q;
-                }
-                continue;
-            }
-            const uint64_t o = KRQ(out_begin) + (q - q_begin) * (uint64_t)K;
-#pragma unroll
-            for (int r = 0; r < R; ++r) {
-                const uint32_t jj = (uint32_t)(r * 32 + lane);
-                if (jj < K) {
-                    a.idx[o + jj] = (jj < nl) ? li[j][jj] : 0xffffffffu;
-                    a.d2[o + jj] = (jj < nl) ? ld[j][jj] : (double)INFINITY;
+#pragma unroll 1
+            for (uint32_t t = lane; t < n; t += 32) {
+                const uint32_t e = ord[t];
+                const double dd = bd[e];
+                const uint32_t ii = bi[e];
+                const uint32_t b = bm.bin(dd, bins);
+                const uint32_t f = b ? hist[b - 1] : 0u, l = hist[b];  // the bin's pairs in ord
+                uint32_t rank = f;
+                if (f < K && l - f > 1)
+#pragma unroll 1
+                    for (uint32_t x = f; x < l; ++x) {
+                        const uint32_t g = ord[x];
+                        rank += pair_less(bd[g], bi[g], dd, ii) ? 1u : 0u;
+                    }
+                if (rank < K) {
+                    a.idx[o + rank] = ii;
+                    a.d2[o + rank] = dd;
+                    if (rank == K - 1) kth = dd;
                 }
             }
-            if (lane == 0 && a.counts) a.counts[q] = nl;
+#pragma unroll 1
+            for (uint32_t t = n + lane; t < K; t += 32) {
+                a.idx[o + t] = 0xffffffffu;
+                a.d2[o + t] = (double)INFINITY;
+            }
+            const uint32_t kb = __ballot_sync(0xffffffffu, kth >= 0.0);
+            kth = kb ? __shfl_sync(0xffffffffu, kth, 31 - __clz(kb)) : -1.0;
+            break;
         }
-        // seed of the next group: the largest k-th distance of the queries that found k pairs
-        double mx = -1.0;
-        if (lane < G && ((vm >> lane) & 1u) && !failed && nls[lane] == K) mx = thr[lane];
-#pragma unroll
-        for (int off = 4; off > 0; off >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, off));
-        mx = __shfl_sync(0xffffffffu, mx, 0);
-        seed_thr = mx;
+        if (!ok && lane == 0) {
+            const unsigned long long f = atomicAdd(a.fb_count, 1ull);
+            a.fb_list[fb_base + f] = (uint32_t)q;
+        }
+        if (!ok) ahead_pos = 0xffffffffu;  // not read
+        run_kth = fmax(kth, kSeedFade * run_kth);
         seed_slot = head ? 0xfffffffeu : slot;  // a head seeds no slot of the run
         seed_ri = ri;
-        if (head && lane == 0) __stcg(&a.head_kth[slot], mx);
+        if (head && lane == 0) __stcg(&a.head_kth[slot], kth);
         __syncwarp();
     }
     if constexpr (F32) {
         if (a.stats) {
 #pragma unroll
             for (int off = 16; off > 0; off >>= 1) {
+                f_tests += __shfl_xor_sync(0xffffffffu, f_tests, off);
                 f_64 += __shfl_xor_sync(0xffffffffu, f_64, off);
                 f_band += __shfl_xor_sync(0xffffffffu, f_band, off);
             }
@@ -1283,24 +1573,27 @@ __global__ void __launch_bounds__(kGrpThreads, kGrpMinBlocks) k_knn_group(KnnGro
     }
 }
 
-// Blocks per SM of a group-kNN instantiation (its shared memory sets it).
-template <int R, int MULTI, bool F32>
-int group_blocks_per_sm() {
-    static int per = 0;
-    if (per == 0) {
-        int v = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, k_knn_group<R, MULTI, F32>, kGrpThreads, 0) !=
-            cudaSuccess)
-            v = 1;
-        per = v > 0 ? v : 1;
-    }
-    return per;
-}
+// Buffer pairs and bins for lists of up to k pairs: a seeded walk collects about 1.4 k.
+uint32_t knn_group_cap(uint32_t k) { return (knn_near_points(k) + 32 * kScanBlocks + 31) / 32 * 32; }
+uint32_t knn_group_bins(uint32_t k) { return k <= 128 ? 128 : k <= 256 ? 256 : k <= 512 ? 512 : 1024; }
 
 // blocks_per_sm > 0 caps the resident blocks (room for a kernel running beside it).
-template <int R, int MULTI, bool F32>
-cudaError_t launch_group(const KnnGroupArgs& g, int sms, cudaStream_t s, int blocks_per_sm = 0) {
-    int per = group_blocks_per_sm<R, MULTI, F32>();
+template <int MULTI, bool F32>
+cudaError_t launch_group(KnnGroupArgs g, uint32_t kmax, int sms, cudaStream_t s, int blocks_per_sm) {
+    g.cap = knn_group_cap(kmax);
+    g.bucket /= 4;
+    g.bins = knn_group_bins(kmax);
+    const size_t smem = kGrpWarps * knn_group_bytes(g.cap, g.bins);
+    cudaError_t e;
+    if (smem > (32u << 10) &&
+        (e = cudaFuncSetAttribute(k_knn_group<MULTI, F32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)(kGrpWarps * knn_group_bytes(knn_group_cap(1024), 1024)))) != cudaSuccess)
+        return e;
+    int per = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_knn_group<MULTI, F32>, kGrpThreads, smem) !=
+            cudaSuccess ||
+        per < 1)
+        per = 1;
     if (blocks_per_sm > 0 && blocks_per_sm < per) per = blocks_per_sm;
     uint64_t grid = (uint64_t)sms * per;
     if (!g.grp) {
@@ -1308,27 +1601,27 @@ cudaError_t launch_group(const KnnGroupArgs& g, int sms, cudaStream_t s, int blo
         if (want < grid) grid = want;
     }
     if (grid == 0) return cudaSuccess;
-    k_knn_group<R, MULTI, F32><<<(int)grid, kGrpThreads, 0, s>>>(g);
+    k_knn_group<MULTI, F32><<<(int)grid, kGrpThreads, smem, s>>>(g);
     return cudaGetLastError();
 }
 
-// The group search of a launch.  With seeding, every kKnnHeadStride-th group
-// is a head: the heads go out first and start from the density estimate; every
-// other group starts from its run's previous group or, when it leads its run,
-// from the nearest head that has finished.  packet_ctr holds 3 counters (zeroed);
+// The search of a launch.  With seeding, every kKnnHeadStride-th query is a
+// head: the heads go out first and start from their own nodes; every other
+// query starts from those before it in its run or, when it leads its run, from
+// the nearest head that has finished.  packet_ctr holds 3 counters (zeroed);
 // head_kth one double per head, set to NaN here.  fp32: the FP32-filter form
 // (every cloud of the launch has its centre-relative FP32 copy).
-template <int R, int MULTI>
-cudaError_t launch_group_seeded(KnnGroupArgs g, int sms, cudaStream_t s, int blocks_per_sm, double* head_kth,
-                                size_t head_bytes, bool fp32) {
-    g.head_stride = (g.est > 0.0 && head_kth) ? kKnnHeadStride : 0;
+template <int MULTI>
+cudaError_t launch_group_seeded(KnnGroupArgs g, uint32_t kmax, int sms, cudaStream_t s, int blocks_per_sm,
+                                double* head_kth, size_t head_bytes, bool fp32) {
+    g.heads = g.est > 0.0 && head_kth ? 1 : 0;
     g.head_kth = head_kth;
-    if (g.head_stride) {
+    if (g.heads) {
         const cudaError_t e = cudaMemsetAsync(head_kth, 0xff, head_bytes, s);
         if (e != cudaSuccess) return e;
     }
-    if (fp32) return launch_group<R, MULTI, true>(g, sms, s, blocks_per_sm);
-    return launch_group<R, MULTI, false>(g, sms, s, blocks_per_sm);
+    if (fp32) return launch_group<MULTI, true>(g, kmax, sms, s, blocks_per_sm);
+    return launch_group<MULTI, false>(g, kmax, sms, s, blocks_per_sm);
 }
 
 int sm_count_k(int device) {
@@ -1390,7 +1683,7 @@ cudaError_t launch_knn_group_table(int device, cudaStream_t s, const DynGroup* d
                                    uint32_t* d_packet_ctr, uint32_t* d_fb_list, double est, uint32_t chunk,
                                    int blocks_per_sm, double* d_head_kth, size_t head_bytes, bool fp32,
                                    unsigned long long* d_stats) {
-    if (kmax > 64) return cudaErrorInvalidValue;
+    if (kmax > 1024) return cudaErrorInvalidValue;
     cudaError_t e;
     if ((e = cudaMemsetAsync(d_packet_ctr, 0, 12, s)) != cudaSuccess) return e;
     KnnGroupArgs g{};
@@ -1410,12 +1703,8 @@ cudaError_t launch_knn_group_table(int device, cudaStream_t s, const DynGroup* d
     g.fb_count = reinterpret_cast<unsigned long long*>(&d_fb->nq);
     const int sms = sm_count_k(device);
     const int bps = blocks_per_sm;
-    if (single)
-        e = (kmax <= 32) ? launch_group_seeded<1, 2>(g, sms, s, bps, d_head_kth, head_bytes, fp32)
-                         : launch_group_seeded<2, 2>(g, sms, s, bps, d_head_kth, head_bytes, fp32);
-    else
-        e = (kmax <= 32) ? launch_group_seeded<1, 1>(g, sms, s, bps, d_head_kth, head_bytes, fp32)
-                         : launch_group_seeded<2, 1>(g, sms, s, bps, d_head_kth, head_bytes, fp32);
+    e = single ? launch_group_seeded<2>(g, kmax, sms, s, bps, d_head_kth, head_bytes, fp32)
+               : launch_group_seeded<1>(g, kmax, sms, s, bps, d_head_kth, head_bytes, fp32);
     if (e != cudaSuccess) return e;
     // the queries handed back, exactly and without the provisional threshold
     return launch_knn_table(device, s, d_fb, single, 0, kmax, d_fb_list, bucket, d_idx, d_d2, d_counts, d_err,
@@ -1435,6 +1724,25 @@ cudaError_t prepare_knn_dyn() {
         return e;
     return cudaFuncSetAttribute(k_knn<1024, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)knn_smem<1024>());
+}
+
+static SearchReq knn_request(const Cloud& c, const double* d_centers, uint64_t nq, uint32_t k) {
+    SearchReq r{};
+    r.cv = cloud_view(c);
+    r.centers = d_centers;
+    r.q_begin = 0;
+    r.q_end = nq;
+    r.k = k;
+    return r;
+}
+
+static cudaError_t launch_list(const KnnArgs& a, uint32_t k, int grid, cudaStream_t s, bool carry) {
+    if (k <= 32) return launch_l<32>(a, grid, s, carry);
+    if (k <= 64) return launch_l<64>(a, grid, s, carry);
+    if (k <= 128) return launch_l<128>(a, grid, s, carry);
+    if (k <= 256) return launch_l<256>(a, grid, s, carry);
+    if (k <= 512) return launch_l<512>(a, grid, s, carry);
+    return launch_l<1024>(a, grid, s, carry);
 }
 
 cudaError_t launch_knn(Cloud& c, const double* d_centers, uint64_t nq, uint32_t k, uint32_t* d_idx, double* d_d2,
@@ -1464,36 +1772,26 @@ cudaError_t launch_knn(Cloud& c, const double* d_centers, uint64_t nq, uint32_t 
     const uint64_t want = (nq + kKnnWarps - 1) / kKnnWarps;
     const uint64_t cap = (uint64_t)sm_count_k(c.device) * 16;
     const int grid = (int)(want < cap ? want : cap);
-    if (c.packet && k <= 64) {
-        // the FP32 filter (group kernel): centre-relative FP32 points, built on first use
-        const bool f32 = fp32_on_knn(c.fp32_filter) && c.knn_packet != 0;
+    if (c.packet && (k > 64 || c.knn_packet)) {
+        // the FP32 filter (k <= 64): centre-relative FP32 points, built on first use
+        cudaError_t e;
+        const bool f32 = fp32_on_knn(c.fp32_filter) && k <= 64;
         if (f32 && !c.crel_built) {
-            cudaError_t e;
             if ((e = launch_center_rel(c)) != cudaSuccess) return e;
             c.crel_built = true;
         }
-        SearchReq r{};
-        r.cv = cloud_view(c);
-        r.centers = d_centers;
-        r.q_begin = 0;
-        r.q_end = nq;
-        r.k = k;
-        if (!c.knn_packet)
-            return launch_knn_table(c.device, c.stream, nullptr, &r, nq, k, a.order, c.knn_bucket, d_idx, d_d2,
-                                    d_counts, c.d_err.as<uint32_t>(), 0, c.knn_est);
-        // groups of curve-ordered queries, then the exact per-query kernel for the queries they hand back
-        cudaError_t e;
+        const SearchReq r = knn_request(c, d_centers, nq, k);
+        // the curve-ordered search, then the exact sorted-list kernels for the queries it hands back
         if ((e = c.packet_ctr.reserve(256)) != cudaSuccess) return e;
         if ((e = c.knn_fb.reserve(16 + 4 * nq)) != cudaSuccess) return e;
-        const uint64_t n_groups = (nq + kGrpQ - 1) / kGrpQ;
-        const size_t head_bytes = 8 * (n_groups / kKnnHeadStride + 1);
+        const size_t head_bytes = 8 * (nq / kKnnHeadStride + 1);
         if ((e = c.knn_heads.reserve(head_bytes)) != cudaSuccess) return e;
         if ((e = cudaMemsetAsync(c.packet_ctr.ptr, 0, 12, c.stream)) != cudaSuccess) return e;
         if ((e = cudaMemsetAsync(c.knn_fb.ptr, 0, 8, c.stream)) != cudaSuccess) return e;
         KnnGroupArgs g{};
         g.single = r;
         g.grp = nullptr;
-        g.packets = (nq + kGrpQ - 1) / kGrpQ;
+        g.packets = nq;
         g.order = a.order;
         g.bucket = c.knn_bucket;
         g.idx = d_idx;
@@ -1509,10 +1807,14 @@ cudaError_t launch_knn(Cloud& c, const double* d_centers, uint64_t nq, uint32_t 
         const int sms = sm_count_k(c.device);
         double* heads = c.knn_heads.as<double>();
         KernelClock clk(c, 1);
-        e = (k <= 32) ? launch_group_seeded<1, 0>(g, sms, c.stream, 0, heads, head_bytes, f32)
-                      : launch_group_seeded<2, 0>(g, sms, c.stream, 0, heads, head_bytes, f32);
+        e = launch_group_seeded<0>(g, k, sms, c.stream, 0, heads, head_bytes, f32);
         clk.stop();
         if (e != cudaSuccess) return e;
+        if (k > 64) {
+            a.order = g.fb_list;
+            a.nq_dev = g.fb_count;
+            return launch_list(a, k, grid, c.stream, true);
+        }
         KnnTableArgs f{};
         f.single = r;
         f.nq = nq;
@@ -1524,17 +1826,16 @@ cudaError_t launch_knn(Cloud& c, const double* d_centers, uint64_t nq, uint32_t 
         f.counts = d_counts;
         f.err = g.err;
         f.est = 0.0;  // exact without the provisional threshold
-        const int fgrid = sms * 16;
-        if (k <= 32) k_knn_reg<1, 0><<<fgrid, kKnnThreads, 0, c.stream>>>(f);
-        else k_knn_reg<2, 0><<<fgrid, kKnnThreads, 0, c.stream>>>(f);
+        if (k <= 32) k_knn_reg<1, 0><<<grid, kKnnThreads, 0, c.stream>>>(f);
+        else k_knn_reg<2, 0><<<grid, kKnnThreads, 0, c.stream>>>(f);
         return cudaGetLastError();
     }
-    if (k <= 32) return launch_l<32>(a, grid, c.stream, c.packet != 0);
-    if (k <= 64) return launch_l<64>(a, grid, c.stream, c.packet != 0);
-    if (k <= 128) return launch_l<128>(a, grid, c.stream, c.packet != 0);
-    if (k <= 256) return launch_l<256>(a, grid, c.stream, c.packet != 0);
-    if (k <= 512) return launch_l<512>(a, grid, c.stream, c.packet != 0);
-    return launch_l<1024>(a, grid, c.stream, c.packet != 0);
+    if (c.packet) {  // k <= 64, one query per warp
+        const SearchReq r = knn_request(c, d_centers, nq, k);
+        return launch_knn_table(c.device, c.stream, nullptr, &r, nq, k, a.order, c.knn_bucket, d_idx, d_d2, d_counts,
+                                c.d_err.as<uint32_t>(), 0, c.knn_est);
+    }
+    return launch_list(a, k, grid, c.stream, false);
 }
 
 // A kernel of this file's device code, for preload_kernels.

@@ -35,7 +35,7 @@ __device__ __forceinline__ unsigned long long mix64(unsigned long long z) {
 
 __device__ __forceinline__ uint32_t lanemask_lt() {
     uint32_t m;
-    asm volatile("mov.u32 %0, %%lanemask_lt;" : "=r"(m));
+    asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));
     return m;
 }
 
