@@ -401,7 +401,7 @@ std::vector<DevBuf*> cloud_bufs(Cloud& c) {
     return {&c.xyz_in,   &c.xs,        &c.ys,          &c.zs,          &c.keys,       &c.keys_alt,
             &c.perm,     &c.perm_alt,  &c.keys_hi,     &c.keys_hi_alt, &c.run_pv,     &c.run_pv_alt,
             &c.run_ctl,  &c.run_list,  &c.run_long,  &c.sort_status, &c.d_ctl,       &c.d_box,      &c.d_err,
-            &c.offsets,  &c.ranges,    &c.centers,     &c.frontier,    &c.masks,      &c.parts,
+            &c.offsets,  &c.ranges,    &c.centers,     &c.lv_counts,   &c.lv_rows,    &c.lv_list,    &c.parts,
             &c.d_build,  &c.q_centers, &c.q_radii,     &c.q_counts,    &c.q_offsets,  &c.q_out,
             &c.q_out2,   &c.q_scan_tmp, &c.qs_keys,    &c.qs_keys_alt, &c.qs_ord,     &c.qs_ord_alt,
             &c.qs_status, &c.qs_ctl,   &c.packet_ctr,  &c.knn_fb,      &c.knn_heads,  &c.stats,

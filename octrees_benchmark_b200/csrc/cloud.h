@@ -71,14 +71,11 @@ struct SortCtl {
 
 // Octree build bookkeeping written by the device.
 struct BuildCtl {
-    uint32_t level_start[kMaxDepth + 3];  // first node index of each level
-    uint32_t level_internal[kMaxDepth + 2];
+    uint32_t level_internal[kMaxDepth + 2];  // split nodes of each level
     uint32_t n_total;
     uint32_t n_internal;
     uint32_t max_depth_seen;
     uint32_t need_nodes;                  // nodes the tree needs (valid when kErrNodeCapacity)
-    uint32_t barrier_count;
-    uint32_t barrier_gen;
 };
 
 // Device pointers of one built cloud, as the search kernels read them.
@@ -171,9 +168,10 @@ struct Cloud {
     DevBuf offsets;  // u32, n_total + 1
     DevBuf ranges;   // uint2 (first, last) per node
     DevBuf centers;  // 3 x f64 per node (AoS)
-    DevBuf frontier; // build scratch: internal nodes of the current/next level
-    DevBuf masks;    // build scratch: ballots of internal children
-    DevBuf parts;    // build scratch: per-block counts
+    DevBuf lv_counts; // build scratch: split nodes per level and block of keys
+    DevBuf lv_rows;   // build scratch: rows of keys that begin split nodes, per warp
+    DevBuf lv_list;   // build scratch: the split nodes
+    DevBuf parts;     // bounding-box partials
     DevBuf d_build;  // BuildCtl
     uint32_t node_capacity = 0;
     uint32_t n_total = 0, n_internal = 0, n_leaf = 0, max_depth_seen = 0;

@@ -20,15 +20,23 @@
 // node are the lower_bounds of its start and end key in the sorted keys, and
 // its centre is PointEncoder::getCenter of its start key.
 //
-// Kernel: one cooperative, persistent launch.  Per level, phase A computes the
-// 8 children of every internal node (one lane per child: a binary search in the
-// parent's point range, the centre, the split flag) and ballots the split flags
-// per 32 children; phase B ranks the split children and writes the next
-// frontier and the offsets.  A block's phase B reads only what its own phase A
-// wrote, plus the number of split children of the blocks before it, which it
-// takes by decoupled look-back over per-block status words (flag | count) —
-// so one grid barrier per level (the next level reads every block's frontier)
-// instead of two.  Grid barriers and look-back waits are bounded.
+// Kernels: every level at once.  The sorted keys alone say which nodes split: the
+// octant of level l that holds key i has more than M = maxPointsLeaf points past
+// i's first if key i + M still lies in it, so with e the level to which key i
+// shares its octant with key i - 1 and d (at most 20) that to which it shares it
+// with key i + M, the split nodes whose first point is i are those of levels e + 1
+// to d.  Their number per level and block of keys (k_level_count), its scan over
+// the blocks (k_level_scan) and their order inside a block give every split node
+// its rank in its level, and so the place of its 8 children (k_level_list);
+// k_level_children finds the children's ranges by search from i on, 8 lanes a
+// node.  No level waits for another, as it did for a grid barrier and a dependent
+// search each when one cooperative launch went down level by level.
+//
+// Bound: latency below ~1M points (four launches of 3 to 12 us), above that the
+// two reads of the keys and the sectors of the searches.  Device time, level by
+// level -> now: 20k points (Hilbert, leaf 32) 61 -> 28 us, 1M (Morton, leaf 128)
+// 113 -> 30, 10M (Hilbert, leaf 64) 194 -> 132 (count 30, scan 7, list 41, children
+// 53; with the children searched by the warp that found their node 236 in all).
 #include "cloud.h"
 #include "sfc.cuh"
 
@@ -36,71 +44,23 @@ namespace octb {
 
 namespace {
 
-constexpr int kBuildThreads = 1024;
-constexpr int kBuildWarps = kBuildThreads / 32;
-
-struct FrontierNode {
-    unsigned long long key;  // start key of the node
-    uint32_t first, last;    // point range
-};
+constexpr int kLvWarps = 8;
+constexpr int kLvThreads = 32 * kLvWarps;
+constexpr int kLvRows = 8;                           // rows of 32 keys a warp takes
+constexpr uint32_t kLvTile = kLvThreads * kLvRows;   // keys of a block
+constexpr int kSplitLevels = (int)kMaxDepth;         // levels 0 .. 20 can split
 
 struct BoxGeom {
     BoxD box;
     LevelGeom geom;
 };
 
-__device__ __forceinline__ uint32_t ld_acquire_u32(const uint32_t* p) {
-    uint32_t v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
-
-__device__ __forceinline__ unsigned long long ld_acquire_u64(const unsigned long long* p) {
-    unsigned long long v;
-    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-    return v;
-}
-__device__ __forceinline__ void st_release_u64(unsigned long long* p, unsigned long long v) {
-    asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
-}
-
-// look-back status word of a block at one level: flag (bits 62-63) | split children (low 32 bits)
-constexpr unsigned long long kLbLocal = 1ull << 62;   // this block's count
-constexpr unsigned long long kLbPrefix = 2ull << 62;  // this block's and every earlier block's
-constexpr unsigned long long kLbFlags = 3ull << 62;
-
-// Grid-wide barrier for a cooperative launch; gives up after kSpinLimit polls.
-__device__ void grid_barrier(BuildCtl* ctl, uint32_t* err) {
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        const uint32_t gen = ld_acquire_u32(&ctl->barrier_gen);
-        __threadfence();
-        const uint32_t arrived = atomicAdd(&ctl->barrier_count, 1u) + 1u;
-        if (arrived == gridDim.x) {
-            atomicExch(&ctl->barrier_count, 0u);
-            __threadfence();
-            atomicAdd(&ctl->barrier_gen, 1u);
-        } else {
-            uint32_t spins = 0;
-            while (ld_acquire_u32(&ctl->barrier_gen) == gen) {
-                if (++spins > kSpinLimit) {
-                    set_err(err, kErrSpinLimit);
-                    break;
-                }
-                __nanosleep(64);
-            }
-        }
-        __threadfence();
-    }
-    __syncthreads();
-}
-
-// lower_bound over a child's parent range.  Ranges longer than kKaryMin are
+// lower_bound over [lo, hi).  Ranges longer than kKaryMin are
 // first narrowed kKaryWays-fold per step by kKaryWays - 1 independent probes
 // (one round trip each step instead of log2(kKaryWays) dependent ones: the top
 // levels' searches span millions of keys), then bisected.
 constexpr uint32_t kKaryWays = 8;
-constexpr uint32_t kKaryMin = 256;
+constexpr uint32_t kKaryMin = 32;
 static_assert(kKaryMin >= kKaryWays, "a k-ary step needs a stride of at least one key");
 
 __device__ __forceinline__ uint32_t lower_bound_keys(const uint64_t* __restrict__ keys, uint32_t lo, uint32_t hi,
@@ -123,213 +83,291 @@ __device__ __forceinline__ uint32_t lower_bound_keys(const uint64_t* __restrict_
     return lo;
 }
 
-// Block-wide sum of one value per thread.
-__device__ __forceinline__ uint32_t block_sum(uint32_t v, uint32_t* red) {
-    for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    __syncthreads();
-    if (lane == 0) red[warp] = v;
-    __syncthreads();
-    uint32_t s = 0;
-    for (int w = 0; w < kBuildWarps; ++w) s += red[w];
-    return s;
+// Levels to which two keys share their octant (0 .. 21).
+__device__ __forceinline__ int shared_levels(uint64_t a, uint64_t b) {
+    const uint64_t x = a ^ b;
+    if (x == 0) return (int)kMaxDepth;
+    const int top = 63 - __clzll((long long)x);  // a key has 63 bits
+    return top >= 62 ? 0 : (62 - top) / 3;
 }
 
-template <int ENC>
-__global__ void __launch_bounds__(kBuildThreads) k_build(const uint64_t* __restrict__ keys, uint32_t n,
-                                                         uint32_t max_leaf, const BoxGeom* __restrict__ bgp,
-                                                         uint32_t* __restrict__ offsets, uint2* __restrict__ ranges,
-                                                         double* __restrict__ centers, uint32_t node_cap,
-                                                         FrontierNode* __restrict__ fa, FrontierNode* __restrict__ fb,
-                                                         uint32_t* __restrict__ masks,
-                                                         unsigned long long* __restrict__ lb, BuildCtl* ctl,
-                                                         uint32_t* err) {
-    __shared__ BoxGeom bg;
-    __shared__ uint32_t red[kBuildWarps];
-    __shared__ uint32_t chunk_pre[kBuildThreads];
-    __shared__ uint32_t s_excl;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    if (tid == 0) bg = *bgp;
-    __syncthreads();
+// e and d of key i: the nodes of levels e + 1 .. d split and begin with it (none when d <= e).
+__device__ __forceinline__ void split_levels(uint64_t prev, uint64_t key, uint64_t far, bool first, bool reaches,
+                                             int& e, int& d) {
+    e = first ? -1 : shared_levels(prev, key);
+    d = reaches ? min(shared_levels(key, far), kSplitLevels - 1) : -1;
+}
 
-    // root (level 0): one block writes it
-    if (blockIdx.x == 0 && tid == 0) {
+// Per block of keys and level, the split nodes that begin in it (counts[level * blocks + block]); per warp, the
+// rows that begin any.  A key whose difference to key i + M is above that to key i - 1 begins none, so few keys
+// get to their levels: two reads of the keys bound this kernel.
+__global__ void __launch_bounds__(kLvThreads) k_level_count(const uint64_t* __restrict__ keys, uint64_t n, uint32_t M,
+                                                            uint32_t* __restrict__ counts, uint8_t* __restrict__ rows) {
+    __shared__ uint32_t s_cnt[kLvWarps][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint64_t base = (uint64_t)blockIdx.x * kLvTile + (uint64_t)warp * (32 * kLvRows) + lane;
+    uint64_t key[kLvRows], far[kLvRows];
+#pragma unroll
+    for (int r = 0; r < kLvRows; ++r) {
+        const uint64_t i = base + 32 * r;
+        key[r] = i < n ? keys[i] : 0ull;
+        far[r] = i + M < n ? keys[i + M] : 0ull;
+    }
+    uint64_t before = lane == 0 && base > 0 && base < n ? keys[base - 1] : 0ull;  // lane 0: the key before the row
+    uint32_t mine = 0, any = 0;  // lane l: split nodes of level l
+#pragma unroll
+    for (int r = 0; r < kLvRows; ++r) {
+        const uint64_t i = base + 32 * r;
+        uint64_t prev = __shfl_up_sync(0xffffffffu, key[r], 1);
+        if (lane == 0) prev = before;
+        before = __shfl_sync(0xffffffffu, key[r], 31);
+        const bool reaches = i + M < n;
+        if (!__any_sync(0xffffffffu, reaches && (i == 0 || (key[r] ^ far[r]) < (prev ^ key[r])))) continue;
+        int e, d;
+        split_levels(prev, key[r], far[r], i == 0, reaches, e, d);
+        const bool has = d > e;
+        if (!__any_sync(0xffffffffu, has)) continue;
+        any |= 1u << r;
+        const int lo = __reduce_min_sync(0xffffffffu, has ? e + 1 : kSplitLevels);
+        const int hi = __reduce_max_sync(0xffffffffu, has ? d : -1);
+#pragma unroll 1
+        for (int l = lo; l <= hi; ++l) {
+            const uint32_t m = __ballot_sync(0xffffffffu, e < l && l <= d);
+            if (lane == l) mine += __popc(m);
+        }
+    }
+    s_cnt[warp][lane] = mine;
+    if (lane == 0) rows[(uint64_t)blockIdx.x * kLvWarps + warp] = (uint8_t)any;
+    __syncthreads();
+    if (threadIdx.x < kSplitLevels) {
+        uint32_t c = 0;
+#pragma unroll
+        for (int w = 0; w < kLvWarps; ++w) c += s_cnt[w][threadIdx.x];
+        counts[(uint64_t)threadIdx.x * gridDim.x + blockIdx.x] = c;
+    }
+}
+
+// One block per level: its counts become exclusive prefixes over the blocks, its total goes to level_internal.
+__global__ void __launch_bounds__(1024) k_level_scan(uint32_t* __restrict__ counts, uint32_t blocks, BuildCtl* ctl) {
+    __shared__ uint32_t s_sum[32];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    uint32_t* c = counts + (uint64_t)blockIdx.x * blocks;
+    uint32_t carry = 0;
+    for (uint32_t b = 0; b < blocks; b += 1024) {
+        const uint32_t v = b + tid < blocks ? c[b + tid] : 0u;
+        uint32_t x = v;
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, x, off);
+            if (lane >= off) x += y;
+        }
+        if (lane == 31) s_sum[warp] = x;
+        __syncthreads();
+        uint32_t w = s_sum[lane];
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, w, off);
+            if (lane >= off) w += y;
+        }
+        const uint32_t before = warp ? __shfl_sync(0xffffffffu, w, warp - 1) : 0u;
+        if (b + tid < blocks) c[b + tid] = carry + before + x - v;
+        carry += __shfl_sync(0xffffffffu, w, 31);
+        __syncthreads();
+    }
+    if (tid == 0) ctl->level_internal[blockIdx.x] = carry;
+}
+
+// Where the levels begin, from the split nodes of each: the first node of level l (start[l]) and the split nodes
+// of the levels before it (split[l]).  One warp; returns the nodes of the tree.
+__device__ __forceinline__ unsigned long long level_table(const BuildCtl* ctl, uint32_t* start, uint32_t* split) {
+    const int lane = threadIdx.x & 31;
+    const uint32_t c = lane < kSplitLevels ? ctl->level_internal[lane] : 0u;
+    unsigned long long x = c;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+        const unsigned long long y = __shfl_up_sync(0xffffffffu, x, off);
+        if (lane >= off) x += y;
+    }
+    const unsigned long long all = __shfl_sync(0xffffffffu, x, 31);
+    if (lane == 0) start[0] = 0;
+    if (lane < kSplitLevels) {
+        start[lane + 1] = (uint32_t)(1 + 8 * (x - c));
+        split[lane] = (uint32_t)(x - c);
+    }
+    if (lane == kSplitLevels) split[lane] = (uint32_t)all;
+    return 1 + 8 * all;
+}
+
+// Every split node, in the order of the nodes: its first point and its own place (x, y of list[]).
+__global__ void __launch_bounds__(kLvThreads) k_level_list(const uint64_t* __restrict__ keys, uint64_t n, uint32_t M,
+                                                           const uint32_t* __restrict__ counts,
+                                                           const uint8_t* __restrict__ rows, uint2* __restrict__ list,
+                                                           uint32_t node_cap, BuildCtl* ctl, uint32_t* err) {
+    __shared__ uint32_t s_start[kMaxDepth + 2], s_split[kMaxDepth + 2];
+    __shared__ unsigned long long s_total;
+    __shared__ uint32_t s_cnt[kLvWarps][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (warp == 0) {
+        const unsigned long long total = level_table(ctl, s_start, s_split);
+        const uint32_t used = __ballot_sync(0xffffffffu, lane < kSplitLevels && ctl->level_internal[lane] != 0);
+        if (lane == 0) {
+            s_total = total;
+            if (blockIdx.x == 0) {
+                if (total > node_cap) {
+                    ctl->need_nodes = (uint32_t)(total < 0xffffffffull ? total : 0xffffffffull);
+                    set_err(err, kErrNodeCapacity);
+                } else {
+                    ctl->n_total = (uint32_t)total;
+                    ctl->n_internal = (uint32_t)(total / 8);
+                    ctl->max_depth_seen = 32 - __clz(used);  // the deepest split level + 1
+                }
+            }
+        }
+    }
+    // split nodes per level of the warp's rows, and of those before them
+    const uint64_t base = (uint64_t)blockIdx.x * kLvTile + (uint64_t)warp * (32 * kLvRows) + lane;
+    const uint32_t any = base - lane < n ? rows[(uint64_t)blockIdx.x * kLvWarps + warp] : 0u;
+    auto levels = [&](int r, uint64_t& key, int& e, int& d) {
+        const uint64_t i = base + 32 * r;
+        key = i < n ? keys[i] : 0ull;
+        const uint64_t far = i + M < n ? keys[i + M] : 0ull;
+        uint64_t prev = __shfl_up_sync(0xffffffffu, key, 1);
+        if (lane == 0 && i > 0 && i < n) prev = keys[i - 1];
+        split_levels(prev, key, far, i == 0, i + M < n, e, d);
+    };
+    uint32_t mine = 0;
+#pragma unroll 1
+    for (uint32_t rem = any; rem; rem &= rem - 1) {
+        uint64_t key;
+        int e, d;
+        levels(__ffs(rem) - 1, key, e, d);
+        const bool has = d > e;
+        const int lo = __reduce_min_sync(0xffffffffu, has ? e + 1 : kSplitLevels);
+        const int hi = __reduce_max_sync(0xffffffffu, has ? d : -1);
+#pragma unroll 1
+        for (int l = lo; l <= hi; ++l) {
+            const uint32_t m = __ballot_sync(0xffffffffu, e < l && l <= d);
+            if (lane == l) mine += __popc(m);
+        }
+    }
+    s_cnt[warp][lane] = mine;
+    __syncthreads();
+    if (!any || s_total > node_cap) return;  // (the host grows the node arrays and runs again)
+    uint32_t pre = lane < kSplitLevels ? counts[(uint64_t)lane * gridDim.x + blockIdx.x] : 0u;
+    for (int w = 0; w < warp; ++w) pre += s_cnt[w][lane];
+#pragma unroll 1
+    for (uint32_t rem = any; rem; rem &= rem - 1) {
+        const int r = __ffs(rem) - 1;
+        uint64_t key;
+        int e, d;
+        levels(r, key, e, d);
+        const bool has = d > e;
+        const int lo = __reduce_min_sync(0xffffffffu, has ? e + 1 : kSplitLevels);
+        const int hi = __reduce_max_sync(0xffffffffu, has ? d : -1);
+        // the level above: its split nodes before the row, and those of the row up to the lane
+        uint32_t up = lo > 0 ? __shfl_sync(0xffffffffu, pre, lo - 1) : 0u;
+#pragma unroll 1
+        for (int l = lo; l <= hi; ++l) {
+            const bool begins = e < l && l <= d;
+            const uint32_t m = __ballot_sync(0xffffffffu, begins);
+            const uint32_t at = __shfl_sync(0xffffffffu, pre, l) + __popc(m & lanemask_lt());
+            if (begins) {
+                // child `digit` of the last split node of the level above that begins at or before the key
+                const uint32_t digit = (uint32_t)((key >> (3 * (kMaxDepth - l))) & 7u);
+                const uint32_t node = l ? s_start[l] + 8u * (up - 1u) + digit : 0u;
+                list[s_split[l] + at] = make_uint2((uint32_t)(base + 32 * r), node);
+            }
+            up = at + (begins ? 1u : 0u);
+            if (lane == l) pre += __popc(m);
+        }
+    }
+}
+
+// The children of every split node, 8 lanes a node.
+template <int ENC>
+__global__ void __launch_bounds__(kLvThreads) k_level_children(const uint64_t* __restrict__ keys, uint64_t n,
+                                                               uint32_t M, const BoxGeom* __restrict__ bgp,
+                                                               const uint2* __restrict__ list,
+                                                               uint32_t* __restrict__ offsets,
+                                                               uint2* __restrict__ ranges,
+                                                               double* __restrict__ centers, uint32_t node_cap,
+                                                               const BuildCtl* __restrict__ ctl) {
+    __shared__ BoxGeom bg;
+    __shared__ uint32_t s_start[kMaxDepth + 2], s_split[kMaxDepth + 2];
+    __shared__ unsigned long long s_total;
+    for (uint32_t t = threadIdx.x; t < sizeof(BoxGeom) / 8; t += kLvThreads)
+        reinterpret_cast<double*>(&bg)[t] = reinterpret_cast<const double*>(bgp)[t];
+    if (threadIdx.x < 32) {
+        const unsigned long long total = level_table(ctl, s_start, s_split);
+        if (threadIdx.x == 0) s_total = total;
+    }
+    __syncthreads();
+    if (s_total > node_cap) return;
+    const uint32_t total = (uint32_t)s_total, splits = total / 8;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
         double c[3];
         node_center<ENC>(0ull, 0, bg.box, bg.geom, c);
-        centers[0] = c[0]; centers[1] = c[1]; centers[2] = c[2];
-        ranges[0] = make_uint2(0u, n);
-        const bool split = n > max_leaf;  // level 0 < 21
-        offsets[0] = split ? 1u : 0u;
-        ctl->level_start[0] = 0;
-        ctl->level_start[1] = 1;
-        ctl->level_internal[0] = split ? 1u : 0u;
-        ctl->n_internal = split ? 1u : 0u;
-        ctl->max_depth_seen = split ? 1u : 0u;
-        ctl->n_total = 1;
-        if (split) {
-            FrontierNode r;
-            r.key = 0ull; r.first = 0u; r.last = n;
-            fa[0] = r;
-        }
+        centers[0] = c[0];
+        centers[1] = c[1];
+        centers[2] = c[2];
+        ranges[0] = make_uint2(0u, (uint32_t)n);
+        if (splits == 0) offsets[0] = 0u;
     }
-    grid_barrier(ctl, err);
-
-    FrontierNode* cur = fa;
-    FrontierNode* nxt = fb;
-    uint32_t F = ld_acquire_u32(&ctl->level_internal[0]);
-    uint32_t n_internal = F;
-    // first node of the level being created, kept by every block (block 0 writes the
-    // level starts for the host after the level's barrier, so they are not read back here)
-    uint32_t level_first = 1;
-    for (uint32_t l = 0; l < kMaxDepth && F > 0; ++l) {
-        const uint32_t child_level = l + 1;
-        const uint32_t lstart = level_first;
-        const uint64_t nchild = 8ull * F;
-        const uint64_t next_start = (uint64_t)lstart + nchild;
-        if (next_start > node_cap) {  // uniform across blocks: every block sees the same values
-            if (blockIdx.x == 0 && tid == 0) {
-                ctl->need_nodes = (uint32_t)(next_start < 0xffffffffull ? next_start : 0xffffffffull);
-                set_err(err, kErrNodeCapacity);
-            }
-            break;
-        }
-        const uint64_t crange = node_range(child_level);
-        const uint32_t W = (uint32_t)((nchild + 31) / 32);
-        const uint32_t C = (W + gridDim.x - 1) / gridDim.x;
-        const uint32_t w0 = blockIdx.x * C;
-        const uint32_t w1 = (w0 + C < W) ? (w0 + C) : W;
-        // ---- phase A: children, their ranges and centres, split ballots ----
-        uint32_t my_count = 0;
-        for (uint32_t w = w0 + warp; w < w1; w += kBuildWarps) {
-            const uint64_t t = 32ull * w + lane;
-            const bool valid = t < nchild;
-            uint32_t first = 0, last = 0;
-            bool split = false;
-            if (valid) {
-                const uint32_t j = (uint32_t)(t >> 3), c = (uint32_t)(t & 7);
-                const FrontierNode p = cur[j];
-                const uint64_t ck = p.key + (uint64_t)c * crange;
-                first = (c == 0) ? p.first : lower_bound_keys(keys, p.first, p.last, ck);
-                const uint32_t node = lstart + (uint32_t)t;
-                double cc[3];
-                node_center<ENC>(ck, child_level, bg.box, bg.geom, cc);
-                centers[3ull * node] = cc[0];
-                centers[3ull * node + 1] = cc[1];
-                centers[3ull * node + 2] = cc[2];
-                last = p.last;  // child 7; others take the next child's first below
-            }
-            const uint32_t nf = __shfl_down_sync(0xffffffffu, first, 1);
-            if (valid) {
-                const uint32_t c = (uint32_t)(t & 7);
-                if (c != 7) last = nf;
-                const uint32_t node = lstart + (uint32_t)t;
-                ranges[node] = make_uint2(first, last);
-                split = (last - first > max_leaf) && (child_level < kMaxDepth);
-                offsets[node] = 0u;
-            }
-            const uint32_t m = __ballot_sync(0xffffffffu, split);
-            if (lane == 0) {
-                masks[w] = m;
-                my_count += __popc(m);
-            }
-        }
-        const uint32_t bsum = block_sum(my_count, red);
-        // ---- the split children of the blocks before this one: decoupled look-back ----
-        unsigned long long* st = lb + (uint64_t)l * gridDim.x;
-        if (warp == 0) {
-            if (lane == 0)
-                st_release_u64(&st[blockIdx.x], (blockIdx.x == 0 ? kLbPrefix : kLbLocal) | bsum);
-            uint32_t excl = 0;
-            int64_t t = (int64_t)blockIdx.x - 1;  // the nearest predecessor not summed yet
-            uint32_t spins = 0;
-            while (t >= 0) {
-                const int64_t ti = t - lane;  // lane 0: the nearest
-                const unsigned long long v = ti >= 0 ? ld_acquire_u64(&st[ti]) : kLbPrefix;
-                const uint32_t ready = __ballot_sync(0xffffffffu, (v & kLbFlags) != 0);
-                const uint32_t pref = __ballot_sync(0xffffffffu, (v & kLbFlags) == kLbPrefix);
-                // lanes up to the nearest prefix must all have published; else wait for them
-                const uint32_t upto = pref ? ((pref & (0u - pref)) << 1) - 1u : 0xffffffffu;
-                if ((ready & upto) != upto) {
-                    if (++spins > kSpinLimit) {
-                        if (lane == 0) set_err(err, kErrSpinLimit);
+    const int c = threadIdx.x & 7;
+    const uint32_t stride = gridDim.x * (kLvThreads / 8);
+    const uint32_t rounds = (splits + stride - 1) / stride;  // whole warps: the lanes of a node shuffle
+    uint32_t t = blockIdx.x * (kLvThreads / 8) + (threadIdx.x >> 3);
+#pragma unroll 1
+    for (uint32_t round = 0; round < rounds; ++round, t += stride) {
+        const bool on = t < splits;
+        const uint2 me = on ? list[t] : make_uint2(0u, 0u);
+        const uint32_t first = me.x;
+        int l = 0;  // the last level that begins at or before t
+#pragma unroll
+        for (int b = 16; b > 0; b >>= 1)
+            if (l + b < kSplitLevels && s_split[l + b] <= t) l += b;
+        const uint64_t key = on ? keys[first] : 0ull;
+        const uint64_t step = node_range(l + 1);
+        const uint64_t start = key & ~(8ull * step - 1ull);
+        // where child c ends
+        const uint64_t v = start + (uint64_t)(c + 1) * step;
+        uint32_t end = first;
+        if (on && key < v) {
+            // the first few levels' nodes are a large part of the keys; else a bracket first: seven doublings
+            // of M / 8 keys at once, as most split nodes hold up to 8 M
+            uint64_t lo = (uint64_t)first + 1, hi = n;
+            if (l > 4) {
+                uint64_t at = first, s = M / 8 + 1;
+#pragma unroll 1
+                for (;;) {
+                    uint32_t below = 0;
+#pragma unroll
+                    for (int q = 0; q < 7; ++q) below += at + (s << q) < n && keys[at + (s << q)] < v ? 1u : 0u;
+                    if (below) lo = at + (s << (below - 1)) + 1;
+                    if (below < 7) {
+                        hi = min(n, at + (s << below));
                         break;
                     }
-                    __nanosleep(32);
-                    continue;
-                }
-                uint32_t c = ((upto >> lane) & 1u) && ti >= 0 ? (uint32_t)(v & 0xffffffffull) : 0u;
-#pragma unroll
-                for (int off = 16; off > 0; off >>= 1) c += __shfl_xor_sync(0xffffffffu, c, off);
-                excl += c;
-                if (pref) break;
-                t -= 32;
-            }
-            if (lane == 0) {
-                if (blockIdx.x > 0) st_release_u64(&st[blockIdx.x], kLbPrefix | (excl + bsum));
-                s_excl = excl;
-            }
-        }
-        __syncthreads();
-        // ---- phase B: rank split children, next frontier, offsets ----
-        const uint32_t pre = s_excl;
-        const uint32_t next_level_start = (uint32_t)next_start;
-        uint32_t carry = pre;
-        for (uint32_t seg = w0; seg < w1; seg += kBuildThreads) {
-            const uint32_t i = seg + tid;
-            const uint32_t v = (i < w1) ? __popc(((volatile uint32_t*)masks)[i]) : 0u;
-            // block exclusive scan of v
-            uint32_t x = v;
-            for (int off = 1; off < 32; off <<= 1) {
-                const uint32_t y = __shfl_up_sync(0xffffffffu, x, off);
-                if (lane >= off) x += y;
-            }
-            __syncthreads();
-            if (lane == 31) red[warp] = x;
-            __syncthreads();
-            uint32_t wp = 0, segsum = 0;
-            for (int ww = 0; ww < kBuildWarps; ++ww) {
-                if (ww < warp) wp += red[ww];
-                segsum += red[ww];
-            }
-            chunk_pre[tid] = carry + wp + x - v;
-            __syncthreads();
-            const uint32_t seg_end = (seg + kBuildThreads < w1) ? seg + kBuildThreads : w1;
-            for (uint32_t w = seg + warp; w < seg_end; w += kBuildWarps) {
-                const uint32_t m = ((volatile uint32_t*)masks)[w];
-                if (m & (1u << lane)) {
-                    const uint32_t rank = chunk_pre[w - seg] + __popc(m & lanemask_lt());
-                    const uint64_t t = 32ull * w + lane;
-                    const uint32_t node = lstart + (uint32_t)t;
-                    const FrontierNode p = cur[t >> 3];
-                    const uint2 rg = ranges[node];
-                    FrontierNode q;
-                    q.key = p.key + (t & 7) * crange;
-                    q.first = rg.x;
-                    q.last = rg.y;
-                    nxt[rank] = q;
-                    offsets[node] = next_level_start + 8u * rank;
+                    at += s << 6;
+                    s <<= 6;
                 }
             }
-            carry += segsum;
-            __syncthreads();
+            end = lower_bound_keys(keys, (uint32_t)lo, (uint32_t)hi, v);
         }
-        grid_barrier(ctl, err);
-        // every block has published its inclusive prefix before the barrier: the last one's is the total
-        const uint32_t tot = (uint32_t)(ld_acquire_u64(&st[gridDim.x - 1]) & 0xffffffffull);
-        if (blockIdx.x == 0 && tid == 0) {
-            ctl->level_start[l + 2] = next_level_start;
-            ctl->level_internal[l + 1] = tot;
-            ctl->n_total = next_level_start;
-            if (tot > 0) ctl->max_depth_seen = l + 2;
-        }
-        n_internal += tot;
-        level_first = next_level_start;
-        FrontierNode* tmp = cur;
-        cur = nxt;
-        nxt = tmp;
-        F = tot;
+        const uint32_t prev = __shfl_up_sync(0xffffffffu, end, 1);
+        if (!on) continue;
+        const uint32_t child = s_start[l + 1] + 8u * (t - s_split[l]) + c;
+        const uint32_t begin = c ? prev : first;
+        double cc[3];
+        node_center<ENC>(start + (uint64_t)c * step, l + 1, bg.box, bg.geom, cc);
+        ranges[child] = make_uint2(begin, end);
+        centers[3ull * child] = cc[0];
+        centers[3ull * child + 1] = cc[1];
+        centers[3ull * child + 2] = cc[2];
+        // a child that splits is in the list itself, and gets its link there
+        if (!(end - begin > M && l + 1 < kSplitLevels)) offsets[child] = 0u;
+        if (c == 0 && me.y < total) offsets[me.y] = child;
     }
-    if (blockIdx.x == 0 && tid == 0) ctl->n_internal = n_internal;
 }
 
 int sm_count_b(int device) {
@@ -353,55 +391,35 @@ cudaError_t launch_build(Cloud& c, bool* capacity_ok) {
         c.node_capacity = (uint32_t)cap;
     }
     const uint64_t cap = c.node_capacity;
-    const uint64_t fcap = n / ((uint64_t)M + 1) + 2;
+    const uint32_t blocks = (uint32_t)(n ? (n + kLvTile - 1) / kLvTile : 1);
     if ((e = c.offsets.reserve(4 * (cap + 1))) != cudaSuccess) return e;
     if ((e = c.ranges.reserve(8 * cap)) != cudaSuccess) return e;
     if ((e = c.centers.reserve(24 * cap)) != cudaSuccess) return e;
-    if ((e = c.frontier.reserve(2 * sizeof(FrontierNode) * fcap)) != cudaSuccess) return e;
-    if ((e = c.masks.reserve(4 * ((8 * fcap + 31) / 32 + 1))) != cudaSuccess) return e;
-
-    int dev = c.device;
-    int per_sm = 0;
-    void (*kfn)(const uint64_t*, uint32_t, uint32_t, const BoxGeom*, uint32_t*, uint2*, double*, uint32_t,
-                FrontierNode*, FrontierNode*, uint32_t*, unsigned long long*, BuildCtl*, uint32_t*) =
-        (c.params.encoder == OCT_ENC_HILBERT_3D) ? k_build<5> : k_build<1>;
-    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kfn, kBuildThreads, 0)) != cudaSuccess)
-        return e;
-    if (per_sm < 1) per_sm = 1;
-    if (per_sm > 4) per_sm = 4;
-    unsigned grid = (unsigned)(sm_count_b(dev) * per_sm);
-    // small trees need few blocks; keep at least one
-    const uint64_t max_useful = (8 * fcap + 31) / 32 / kBuildWarps + 1;
-    if (grid > max_useful) grid = (unsigned)max_useful;
-    if (grid < 1) grid = 1;
-    // BuildCtl, then the look-back status words of every level and block (zeroed: no flag)
-    const size_t ctl_bytes = (sizeof(BuildCtl) + 255) / 256 * 256;
-    const size_t lb_bytes = sizeof(unsigned long long) * (kMaxDepth + 1) * (size_t)grid;
-    if ((e = c.d_build.reserve(ctl_bytes + lb_bytes)) != cudaSuccess) return e;
-    if ((e = cudaMemsetAsync(c.d_build.ptr, 0, ctl_bytes + lb_bytes, c.stream)) != cudaSuccess) return e;
-
+    if ((e = c.lv_counts.reserve(4ull * kSplitLevels * blocks)) != cudaSuccess) return e;
+    if ((e = c.lv_rows.reserve((uint64_t)kLvWarps * blocks)) != cudaSuccess) return e;
+    if ((e = c.lv_list.reserve(sizeof(uint2) * (cap / 8 + 1))) != cudaSuccess) return e;
+    if ((e = c.d_build.reserve(sizeof(BuildCtl))) != cudaSuccess) return e;
+    if ((e = cudaMemsetAsync(c.d_build.ptr, 0, sizeof(BuildCtl), c.stream)) != cudaSuccess) return e;
     const uint64_t* keys = c.keys.as<uint64_t>();
-    uint32_t nn = (uint32_t)n;
-    uint32_t ml = M;
-    const BoxGeom* bg = c.d_box.as<BoxGeom>();
-    uint32_t* offs = c.offsets.as<uint32_t>();
-    uint2* rng = c.ranges.as<uint2>();
-    double* ctr = c.centers.as<double>();
-    uint32_t ncap = (uint32_t)cap;
-    FrontierNode* fa = c.frontier.as<FrontierNode>();
-    FrontierNode* fb = fa + fcap;
-    uint32_t* masks = c.masks.as<uint32_t>();
+    uint32_t* counts = c.lv_counts.as<uint32_t>();
+    uint8_t* rows = c.lv_rows.as<uint8_t>();
     BuildCtl* ctl = c.d_build.as<BuildCtl>();
-    unsigned long long* lb = reinterpret_cast<unsigned long long*>(static_cast<unsigned char*>(c.d_build.ptr) +
-                                                                   ctl_bytes);
-    uint32_t* err = c.d_err.as<uint32_t>();
-    void* args[] = {(void*)&keys, &nn, &ml, (void*)&bg, &offs, &rng, &ctr, &ncap, &fa, &fb, &masks, &lb,
-                    &ctl, &err};
-    e = cudaLaunchCooperativeKernel((const void*)kfn, dim3(grid), dim3(kBuildThreads), args, 0, c.stream);
-    return e;
+    uint2* list = c.lv_list.as<uint2>();
+    const uint64_t most = cap / 8 + 1;  // split nodes
+    const uint64_t want = (8 * most + kLvThreads - 1) / kLvThreads;
+    const uint64_t full = (uint64_t)sm_count_b(c.device) * 8;
+    const unsigned grid = (unsigned)(want < full ? want : full);
+    k_level_count<<<blocks, kLvThreads, 0, c.stream>>>(keys, n, M, counts, rows);
+    k_level_scan<<<kSplitLevels, 1024, 0, c.stream>>>(counts, blocks, ctl);
+    k_level_list<<<blocks, kLvThreads, 0, c.stream>>>(keys, n, M, counts, rows, list, (uint32_t)cap, ctl,
+                                                      c.d_err.as<uint32_t>());
+    auto children = c.params.encoder == OCT_ENC_HILBERT_3D ? k_level_children<5> : k_level_children<1>;
+    children<<<grid, kLvThreads, 0, c.stream>>>(keys, n, M, c.d_box.as<BoxGeom>(), list, c.offsets.as<uint32_t>(),
+                                                c.ranges.as<uint2>(), c.centers.as<double>(), (uint32_t)cap, ctl);
+    return cudaGetLastError();
 }
 
 // A kernel of this file's device code, for preload_kernels.
-const void* kernel_anchor_octree_build() { return reinterpret_cast<const void*>(&k_build<1>); }
+const void* kernel_anchor_octree_build() { return reinterpret_cast<const void*>(&k_level_children<1>); }
 
 }  // namespace octb
