@@ -248,31 +248,31 @@ __global__ void __launch_bounds__(kEncThreads) k_encode(const double* __restrict
     }
 }
 
-// Exclusive scans of the 8 histograms; pass p is skipped when one digit holds
-// every key.  One block of 256 threads.
+// Exclusive scans of the 8 histograms, a block of 256 threads each (one block for
+// all of them took 8.7 us of every sort and query order, 8 blocks 2.7); pass p is
+// skipped when one digit holds every key.
+constexpr int kScanHistBlocks = 8;
 __global__ void __launch_bounds__(256) k_scan_hist(SortCtl* ctl, uint64_t n, const uint64_t* d_n = nullptr) {
     __shared__ unsigned long long warp_sum[8];
     if (d_n) n = *d_n;
     const int d = threadIdx.x, lane = d & 31, warp = d >> 5;
-    for (int p = 0; p < 8; ++p) {
-        const unsigned long long v = ctl->hist[p][d];
-        unsigned long long x = v;
+    const int p = blockIdx.x;
+    const unsigned long long v = ctl->hist[p][d];
+    unsigned long long x = v;
 #pragma unroll
-        for (int off = 1; off < 32; off <<= 1) {
-            const unsigned long long y = __shfl_up_sync(0xffffffffu, x, off);
-            if (lane >= off) x += y;
-        }
-        if (lane == 31) warp_sum[warp] = x;
-        const bool full = (v == n);
-        const int any_full = __syncthreads_or(full);
-        unsigned long long base = 0;
-        for (int w = 0; w < warp; ++w) base += warp_sum[w];
-        ctl->offs[p][d] = base + x - v;
-        if (d == 0) {
-            ctl->skip[p] = any_full ? 1u : 0u;
-            ctl->tile_ctr[p] = 0;
-        }
-        __syncthreads();
+    for (int off = 1; off < 32; off <<= 1) {
+        const unsigned long long y = __shfl_up_sync(0xffffffffu, x, off);
+        if (lane >= off) x += y;
+    }
+    if (lane == 31) warp_sum[warp] = x;
+    const bool full = (v == n);
+    const int any_full = __syncthreads_or(full);
+    unsigned long long base = 0;
+    for (int w = 0; w < warp; ++w) base += warp_sum[w];
+    ctl->offs[p][d] = base + x - v;
+    if (d == 0) {
+        ctl->skip[p] = any_full ? 1u : 0u;
+        ctl->tile_ctr[p] = 0;
     }
 }
 
@@ -637,6 +637,7 @@ __global__ void __launch_bounds__(kRunMidThreads) k_runs_mid(const uint32_t* __r
     __shared__ uint32_t s_r;
     const int tid = threadIdx.x;
     const uint32_t count = rc->b_count;
+    if (blockIdx.x >= count) return;  // no more blocks than runs
     for (;;) {
         if (tid == 0) s_r = atomicAdd(&rc->b_next, 1u);
         __syncthreads();
@@ -685,6 +686,8 @@ __global__ void __launch_bounds__(kRunWarpThreads) k_runs_warp(const uint32_t* _
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     unsigned long long* s = sw[warp];
     const uint32_t count = rc->w_count;
+    // no more warps than runs: 9.5k warps asking the counter for one of a few runs took 9 us
+    if (blockIdx.x * (kRunWarpThreads / 32) + warp >= count) return;
     for (;;) {
         uint32_t r = 0;
         if (lane == 0) r = atomicAdd(&rc->w_next, 1u);
@@ -850,7 +853,7 @@ cudaError_t launch_bbox_encode(Cloud& c, const double* d_xyz, bool upper_hist_on
         else if (!upper_hist_only) k_encode<1><<<grid, kEncThreads, 0, c.stream>>>(d_xyz, n, bg, keys, ctl);
         else if (hil) k_encode<5, false><<<grid, kEncThreads, 0, c.stream>>>(d_xyz, n, bg, keys, ctl);
         else k_encode<1, false><<<grid, kEncThreads, 0, c.stream>>>(d_xyz, n, bg, keys, ctl);
-        k_scan_hist<<<1, 256, 0, c.stream>>>(ctl, n);
+        k_scan_hist<<<kScanHistBlocks, 256, 0, c.stream>>>(ctl, n);
     }
     return cudaGetLastError();
 }
@@ -1042,7 +1045,7 @@ cudaError_t launch_sort_long(Cloud& c, const double* d_xyz, uint32_t l_count, ui
     const uint64_t want = (T + 255) / 256;
     const int grid = (int)(want < (uint64_t)sms * 4 ? want : (uint64_t)sms * 4);
     k_hist_all<<<grid, 256, 0, c.stream>>>(kb[0]->as<uint64_t>(), rc, ctl);
-    k_scan_hist<<<1, 256, 0, c.stream>>>(ctl, T);
+    k_scan_hist<<<kScanHistBlocks, 256, 0, c.stream>>>(ctl, T);
     int slot_bytes = 0;
     for (uint32_t v = l_count - 1; v; v >>= 8) ++slot_bytes;
     int sel = 0;
@@ -1114,7 +1117,7 @@ cudaError_t launch_sort_dyn(int device, cudaStream_t s, uint64_t* k0, uint64_t* 
     const uint64_t max_tiles = (max_n + kSortTile - 1) / kSortTile;
     const uint64_t resident = (uint64_t)sm_count(device) * kSortBlocksPerSM;
     const unsigned grid = (unsigned)(max_tiles < resident ? (max_tiles ? max_tiles : 1) : resident);
-    k_scan_hist<<<1, 256, 0, s>>>(ctl, 0, d_n);
+    k_scan_hist<<<kScanHistBlocks, 256, 0, s>>>(ctl, 0, d_n);
     uint64_t* kb[2] = {k0, k1};
     uint32_t* vb[2] = {v0, v1};
     for (int p = 0; p < passes; ++p) {
@@ -1188,7 +1191,7 @@ cudaError_t launch_query_order(Cloud& c, const double* d_centers, uint64_t nq, c
         k_query_keys<5><<<grid, kEncThreads, 0, c.stream>>>(d_centers, nq, bg, c.qs_keys.as<uint64_t>(), ctl);
     else
         k_query_keys<1><<<grid, kEncThreads, 0, c.stream>>>(d_centers, nq, bg, c.qs_keys.as<uint64_t>(), ctl);
-    k_scan_hist<<<1, 256, 0, c.stream>>>(ctl, nq);
+    k_scan_hist<<<kScanHistBlocks, 256, 0, c.stream>>>(ctl, nq);
     DevBuf* kb[2] = {&c.qs_keys, &c.qs_keys_alt};
     DevBuf* vb[2] = {&c.qs_ord, &c.qs_ord_alt};
     int sel = 0;
@@ -1317,7 +1320,7 @@ extern "C" int oct_encode_sort_noalloc(int encoder, const double* d_xyz, uint64_
         const int grid = (int)(want < (uint64_t)kNoAllocBboxGrid ? want : (uint64_t)kNoAllocBboxGrid);
         if (encoder == OCT_ENC_HILBERT_3D) k_encode<5><<<grid, kEncThreads, 0, s>>>(d_xyz, n, &sc->bg, d_keys, ctl);
         else k_encode<1><<<grid, kEncThreads, 0, s>>>(d_xyz, n, &sc->bg, d_keys, ctl);
-        k_scan_hist<<<1, 256, 0, s>>>(ctl, n);
+        k_scan_hist<<<kScanHistBlocks, 256, 0, s>>>(ctl, n);
         // all 8 digit passes (no host readback of the skip flags), so the result
         // ends in the caller's buffers: caller -> scratch -> caller ...
         const size_t smem = onesweep_smem();
