@@ -302,6 +302,48 @@ cudaMemPool_t cloud_pool(int device) {
     return pools[device];
 }
 
+static std::mutex g_stream_mu;
+static std::vector<cudaStream_t> g_streams[64];  // idle, per device
+
+cudaError_t stream_get(int device, cudaStream_t* out) {
+    if (device >= 0 && device < 64) {
+        std::lock_guard<std::mutex> lk(g_stream_mu);
+        if (!g_streams[device].empty()) {
+            *out = g_streams[device].back();
+            g_streams[device].pop_back();
+            return cudaSuccess;
+        }
+    }
+    return cudaStreamCreateWithFlags(out, cudaStreamNonBlocking);
+}
+
+void stream_put(int device, cudaStream_t s) {
+    if (!s) return;
+    if (device >= 0 && device < 64) {
+        std::lock_guard<std::mutex> lk(g_stream_mu);
+        if (g_streams[device].size() < kIdleStreams) {
+            try {
+                g_streams[device].push_back(s);
+                return;
+            } catch (...) {
+            }
+        }
+    }
+    cudaStreamDestroy(s);
+}
+
+void idle_streams_drop(int device) {
+    std::vector<cudaStream_t> drop;
+    if (device >= 0 && device < 64) {
+        std::lock_guard<std::mutex> lk(g_stream_mu);
+        drop.swap(g_streams[device]);
+    }
+    for (cudaStream_t s : drop) {
+        cudaStreamSynchronize(s);  // its last cloud's arrays are free then
+        cudaStreamDestroy(s);
+    }
+}
+
 static std::mutex g_pinned_mu;
 static std::vector<void*> g_pinned_free;
 
@@ -458,12 +500,13 @@ int oct_cloud_create(const oct_params* p, oct_cloud* out) {
     c.device = p->device;
     c.split_sort = (p->flags & OCT_CLOUD_SORT_8PASS) ? 0 : 1;
     DeviceGuard g(c.device);
-    cudaError_t e = cudaStreamCreateWithFlags(&c.stream, cudaStreamNonBlocking);
+    cudaError_t e = stream_get(c.device, &c.stream);
     if (e == cudaSuccess) {
         c.own_stream = true;
         cudaMemPool_t pool = cloud_pool(c.device);
         if (!pool) e = cudaErrorMemoryAllocation;
         for (DevBuf* b : cloud_bufs(c)) b->bind(pool, &c.stream);
+        c.slab.bind(pool, &c.stream);
     }
     if (e == cudaSuccess) e = c.d_err.reserve(256);
     if (e == cudaSuccess) e = cudaMemsetAsync(c.d_err.ptr, 0, 256, c.stream);
@@ -473,7 +516,6 @@ int oct_cloud_create(const oct_params* p, oct_cloud* out) {
         c.pinned = pinned_block_get();
         if (!c.pinned) e = cudaErrorMemoryAllocation;
     }
-    if (e == cudaSuccess) e = cudaStreamSynchronize(c.stream);
     if (e != cudaSuccess) {
         cudaGetLastError();
         oct_cloud_destroy(h);
@@ -490,12 +532,13 @@ int oct_cloud_destroy(oct_cloud h) {
         DeviceGuard g(c.device);
         if (c.stream) cudaStreamSynchronize(c.stream);
         for (DevBuf* b : cloud_bufs(c)) b->release();  // in the stream's order: waits for nothing else
-        if (c.stream) cudaStreamSynchronize(c.stream);
+        c.slab.release();
+        if (c.stream && !c.own_stream) cudaStreamSynchronize(c.stream);
         pinned_block_put(c.pinned);
         for (auto& v : c.ev_pend)
             for (auto& pr : v) c.ev_free.insert(c.ev_free.end(), {pr.first, pr.second});
         for (cudaEvent_t ev : c.ev_free) cudaEventDestroy(ev);
-        if (c.own_stream && c.stream) cudaStreamDestroy(c.stream);
+        if (c.own_stream) stream_put(c.device, c.stream);  // (what it still frees, its next cloud may take at once)
     }
     delete h;
     return OCT_OK;
@@ -506,7 +549,7 @@ int oct_cloud_set_stream(oct_cloud h, void* stream) {
     Cloud& c = h->c;
     DeviceGuard g(c.device);
     CK(cudaStreamSynchronize(c.stream));
-    if (c.own_stream) cudaStreamDestroy(c.stream);
+    if (c.own_stream) stream_put(c.device, c.stream);
     c.own_stream = false;
     c.stream = static_cast<cudaStream_t>(stream);
     return OCT_OK;
@@ -636,6 +679,7 @@ int oct_trim_cloud_memory(int device) {
     cudaMemPool_t pool = cloud_pool(device);
     if (!pool) return OCT_ERR_CUDA;
     DeviceGuard g(device);
+    idle_streams_drop(device);
     if (cudaMemPoolTrimTo(pool, 0) != cudaSuccess) {
         cudaGetLastError();
         return OCT_ERR_CUDA;
@@ -649,17 +693,26 @@ int oct_set_points(oct_cloud h, const double* xyz, uint64_t n, uint32_t flags) {
     if (n && !xyz) return set_error(c, OCT_ERR_INVALID_ARG, "xyz is NULL");
     if (n >= 0xffffffffull) return set_error(c, OCT_ERR_INVALID_ARG, "more than 2^32 - 2 points");
     DeviceGuard g(c.device);
+    // the old points are gone from here on, whatever fails
+    c.n = 0;
+    c.sorted = false;
+    c.built = false;
+    c.rel_built = false;
+    c.crel_built = false;
+    c.node_capacity = 0;
+    if (n && c.split_sort && c.xyz_in.bytes < 24 * n) {
+        // more points than before: new arrays, cut from one slab (the old slab goes with all that is cut from it)
+        for (DevBuf* b : cloud_bufs(c))
+            if (b->slice) b->release();
+        c.slab.release();
+        reserve_point_arrays(c, n);
+    }
     CK(c.xyz_in.reserve(24 * (n ? n : 1)));
     if (n) {
         CK(cudaMemcpyAsync(c.xyz_in.ptr, xyz, 24 * n,
                            (flags & OCT_MEM_DEVICE) ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, c.stream));
     }
     c.n = n;
-    c.sorted = false;
-    c.built = false;
-    c.rel_built = false;
-    c.crel_built = false;
-    c.node_capacity = 0;
     if (!(flags & OCT_MEM_DEVICE)) CK(cudaStreamSynchronize(c.stream));
     return OCT_OK;
 }

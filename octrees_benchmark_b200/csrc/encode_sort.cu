@@ -912,6 +912,40 @@ cudaError_t launch_sort_passes(Cloud& c, const uint32_t skip[8], int* final_sel)
     return cudaGetLastError();
 }
 
+void reserve_point_arrays(Cloud& c, uint64_t n) {
+    const struct {
+        DevBuf* b;
+        size_t bytes;
+    } part[] = {{&c.xyz_in, 24 * n},
+                {&c.keys, 8 * n},
+                {&c.keys_alt, 8 * n},
+                {&c.perm, 4 * n},
+                {&c.keys_hi, 4 * n},
+                {&c.keys_hi_alt, 4 * n},
+                {&c.run_pv, 8 * n},
+                {&c.run_pv_alt, 8 * n},
+                {&c.xs, 8 * n},
+                {&c.ys, 8 * n},
+                {&c.zs, 8 * n},
+                {&c.run_ctl, sizeof(RunCtl)},
+                {&c.run_list, 8 * (n / (kRunSmall + 1) + 1)},
+                {&c.run_long, sizeof(LongRun) * (n / (kRunMid + 1) + 1)},
+                {&c.d_ctl, sizeof(SortCtl)},
+                {&c.d_box, sizeof(BoxGeom)}};
+    auto up = [](size_t b) { return (b + 255) / 256 * 256; };
+    size_t total = 0;
+    for (const auto& p : part) total += up(p.bytes);
+    if (c.slab.reserve(total) != cudaSuccess) {
+        cudaGetLastError();
+        return;
+    }
+    unsigned char* at = static_cast<unsigned char*>(c.slab.ptr);
+    for (const auto& p : part) {
+        p.b->take_slice(at, up(p.bytes));
+        at += up(p.bytes);
+    }
+}
+
 // The split sort (upper halves, then runs): the sorted keys go to c.keys_alt,
 // the permutation to c.perm, the sorted coordinates to xs / ys / zs.  The
 // passes carry each key's lower half with its input position (one 64-bit
@@ -936,9 +970,11 @@ cudaError_t launch_sort_split(Cloud& c, const uint32_t skip[8], const double* d_
     if ((e = c.ys.reserve(8 * nn)) != cudaSuccess) return e;
     if ((e = c.zs.reserve(8 * nn)) != cudaSuccess) return e;
     RunCtl* rc = c.run_ctl.as<RunCtl>();
-    RunCtl rc0{};
-    rc0.cap = (uint32_t)(n / (kRunSmall + 1) + 1);
-    if ((e = cudaMemcpyAsync(rc, &rc0, sizeof(RunCtl), cudaMemcpyHostToDevice, c.stream)) != cudaSuccess) return e;
+    // (a pinned source: the copy is queued, where one from the stack is staged first)
+    RunCtl* rc0 = reinterpret_cast<RunCtl*>(static_cast<unsigned char*>(c.pinned) + kPinnedRunOffset);
+    *rc0 = RunCtl{};
+    rc0->cap = (uint32_t)(n / (kRunSmall + 1) + 1);
+    if ((e = cudaMemcpyAsync(rc, rc0, sizeof(RunCtl), cudaMemcpyHostToDevice, c.stream)) != cudaSuccess) return e;
     if (n == 0) return cudaSuccess;
     const uint64_t tiles = (n + kSortTile - 1) / kSortTile;
     const size_t status_bytes = tiles * 256 * sizeof(unsigned long long);
