@@ -157,7 +157,7 @@ cudaError_t radius_pass(Cloud& c, int kernel, int algo, bool fill, const double*
 }
 
 // Radius search in one traversal (packet path, FP64 or FP32 filter): every query's results go
-// to its chain of result chunks, the counts are scanned, and the chains are
+// to its chain of result chunks, the counts are scanned, and the chunks are
 // compacted into the CSR output.  A pool that turned out too small leaves the
 // counts exact: it is sized from the total and the traversal runs once more.
 // d_points (neighborsStruct ranges): every query's points; else NULL, and neighborsStruct searches its index set.
@@ -167,7 +167,6 @@ int radius_chunks(Cloud& c, int kernel, int algo, const double* dq, uint64_t nq,
     const int pass_algo = (algo == OCT_NEIGHBORS_STRUCT && !d_points) ? OCT_NEIGHBORS_PRUNE : algo;  // same index set
     unsigned long long* dc = c.q_counts.as<unsigned long long>();
     CK(c.stats.reserve(64));
-    CK(c.ck_first.reserve(4 * nq));
     CK(c.ck_ctr.reserve(256));
     const uint32_t* order = nullptr;
     if (packet_width(nq, c.device) > 1) CK(launch_query_order(c, dq, nq, &order));
@@ -183,10 +182,10 @@ int radius_chunks(Cloud& c, int kernel, int algo, const double* dq, uint64_t nq,
         if (want > 0xfffffff0ull) return set_error(c, OCT_ERR_INVALID_ARG, "too many results for one call");
         if (want > c.ck_cap) {
             CK(c.ck_pool.reserve(4ull * kResultChunk * want));
-            CK(c.ck_next.reserve(4ull * want));
+            CK(c.ck_rec.reserve(sizeof(uint2) * want));
             c.ck_cap = (uint32_t)want;
         }
-        ChunkArgs ck{c.ck_pool.as<uint32_t>(), c.ck_next.as<uint32_t>(), c.ck_first.as<uint32_t>(),
+        ChunkArgs ck{c.ck_pool.as<uint32_t>(), c.ck_rec.as<uint2>(),
                      c.ck_ctr.as<uint32_t>(), c.ck_cap};
         CK(cudaMemsetAsync(ck.ctr, 0, 4, c.stream));
         CK(launch_radius_packet(c, kernel, pass_algo, 2, fp32_on_radius(c.fp32_filter), dq, nq, dr, radius, order,
@@ -205,7 +204,7 @@ int radius_chunks(Cloud& c, int kernel, int algo, const double* dq, uint64_t nq,
     return OCT_OK;
 }
 
-// One pass into result chunks (radius_chunks), then the chains compacted into the CSR output.
+// One pass into result chunks (radius_chunks), then the chunks compacted into the CSR output.
 int radius_one_pass(Cloud& c, int kernel, int algo, const double* dq, uint64_t nq, const double* dr, double radius,
                     unsigned long long* doffs, uint64_t* offsets, uint32_t* idx, uint64_t idx_capacity,
                     uint64_t* total, bool dev) {
@@ -224,7 +223,7 @@ int radius_one_pass(Cloud& c, int kernel, int algo, const double* dq, uint64_t n
         CK(c.q_out.reserve(4 * (tot ? tot : 1)));
         dout = c.q_out.as<uint32_t>();
     }
-    ChunkArgs ck{c.ck_pool.as<uint32_t>(), c.ck_next.as<uint32_t>(), c.ck_first.as<uint32_t>(),
+    ChunkArgs ck{c.ck_pool.as<uint32_t>(), c.ck_rec.as<uint2>(),
                  c.ck_ctr.as<uint32_t>(), c.ck_cap};
     CK(launch_chunk_compact(c.device, c.stream, dc, doffs, ck, dout, tot, nq, nullptr, c.d_err.as<uint32_t>()));
     if (!dev && tot) CK(cudaMemcpyAsync(idx, dout, 4 * tot, cudaMemcpyDeviceToHost, c.stream));
@@ -460,7 +459,7 @@ std::vector<DevBuf*> cloud_bufs(Cloud& c) {
             &c.d_build,  &c.q_centers, &c.q_radii,     &c.q_counts,    &c.q_offsets,  &c.q_out,
             &c.q_out2,   &c.q_scan_tmp, &c.qs_keys,    &c.qs_keys_alt, &c.qs_ord,     &c.qs_ord_alt,
             &c.qs_status, &c.qs_ctl,   &c.packet_ctr,  &c.knn_fb,      &c.knn_heads,  &c.stats,
-            &c.rel,      &c.crel,      &c.q_axes,      &c.ck_pool,     &c.ck_next,    &c.ck_first,
+            &c.rel,      &c.crel,      &c.q_axes,      &c.ck_pool,     &c.ck_rec,
             &c.ck_ctr};
 }
 }  // namespace
@@ -1071,7 +1070,7 @@ int oct_radius_hash(oct_cloud h, int kernel, int algo, const double* centers, ui
     int st = radius_common(c, kernel, algo, centers, nq, radii, radius, dev, &dq, &dr);
     if (st != OCT_OK || nq == 0) return st;
     // the one-pass search into result chunks (whatever the cloud's search configuration: the sets are the same),
-    // then per query the sum over its chain instead of the CSR lists
+    // then per query the sum over its chunks instead of the CSR lists
     CK(c.q_counts.reserve(8 * nq));
     CK(c.q_offsets.reserve(8 * (nq + 1)));
     uint64_t tot = 0;
@@ -1082,7 +1081,7 @@ int oct_radius_hash(oct_cloud h, int kernel, int algo, const double* centers, ui
         CK(c.q_out2.reserve(8 * nq));
         dh = c.q_out2.as<unsigned long long>();
     }
-    ChunkArgs ck{c.ck_pool.as<uint32_t>(), c.ck_next.as<uint32_t>(), c.ck_first.as<uint32_t>(),
+    ChunkArgs ck{c.ck_pool.as<uint32_t>(), c.ck_rec.as<uint2>(),
                  c.ck_ctr.as<uint32_t>(), c.ck_cap};
     const unsigned long long* dc = c.q_counts.as<unsigned long long>();
     CK(launch_chunk_hash(c.device, c.stream, dc, ck, dh, nq, c.d_err.as<uint32_t>()));
@@ -1213,7 +1212,7 @@ static int ranges_search(oct_cloud h, int kernel, const double* centers, uint64_
         dout = c.q_out.as<uint32_t>();
     }
     if (one_pass) {
-        const ChunkArgs ck{c.ck_pool.as<uint32_t>(), c.ck_next.as<uint32_t>(), c.ck_first.as<uint32_t>(),
+        const ChunkArgs ck{c.ck_pool.as<uint32_t>(), c.ck_rec.as<uint2>(),
                            c.ck_ctr.as<uint32_t>(), c.ck_cap};
         CK(launch_chunk_compact(c.device, c.stream, dranges, doffs, ck, dout, 2 * tot, nq, nullptr,
                                 c.d_err.as<uint32_t>(), 2));

@@ -225,8 +225,8 @@ struct Cloud {
     DevBuf q_axes;
     double knn_est = kKnnEstimate;  // register kNN: provisional-threshold factor (0: off)
     uint32_t knn_chunk = kKnnGroupChunk;  // group kNN: consecutive groups per warp fetch
-    // one-pass radius search: result chunk pool, links, first chunk per query, counter
-    DevBuf ck_pool, ck_next, ck_first, ck_ctr;
+    // one-pass radius search: result chunk pool, each chunk's query and place in its chain, counter
+    DevBuf ck_pool, ck_rec, ck_ctr;
     uint32_t ck_cap = 0;
 
     // pinned host staging for small readbacks
@@ -297,12 +297,11 @@ cudaError_t launch_radius_packet(Cloud& c, int kernel, int algo, int mode, bool 
                                  unsigned long long* d_counts, unsigned long long* d_counts2,
                                  const unsigned long long* d_offsets, uint32_t* d_out, uint64_t out_capacity,
                                  const ChunkArgs* chunks = nullptr);
-// Result chunks of the one-pass radius search: `cap` chunks of 64 entries, the
-// next-chunk links, each query's first chunk, and the hand-out counter.
+// Result chunks of the one-pass radius search: `cap` chunks of 64 entries, the query each belongs to and its
+// number in that query's chain (chunk k holds entries 64 k on), and the hand-out counter.
 struct ChunkArgs {
     uint32_t* pool;
-    uint32_t* next;
-    uint32_t* first;
+    uint2* rec;  // query, number in the chain
     uint32_t* ctr;
     uint32_t cap;
 };
@@ -315,18 +314,18 @@ uint32_t packet_width(uint64_t nq, int device);
 // both, every request of the group is on the cloud `single->cv` (kernel
 // parameters instead of per-request views).
 // mode: 0 count, 1 fill at d_offsets, 2 one pass into `chunks` (counts and
-// first chunks written; neighborsStruct also writes d_counts2).
+// the chunks' records written; neighborsStruct also writes d_counts2).
 cudaError_t launch_radius_table(int device, cudaStream_t s, int kernel, int algo, int mode, bool fp32,
                                 const DynGroup* d_grp, const SearchReq* single, uint64_t packets, uint32_t width,
                                 const uint32_t* d_order, unsigned long long* d_counts, unsigned long long* d_counts2,
                                 const unsigned long long* d_offsets, uint32_t* d_out, uint64_t out_capacity,
                                 uint32_t* d_packet_ctr, unsigned long long* d_stats, uint32_t* d_err,
                                 int blocks_per_sm = 0, const ChunkArgs* chunks = nullptr);
-// Chains of result chunks into CSR (after the counts are scanned into d_offsets);
-// per = 2 for ranges (two entries a result; d_out and out_capacity count entries).
-// Per query, the sum of splitmix64's output function over its result chain.
+// Per query, the sum of splitmix64's output function over its result chunks.
 cudaError_t launch_chunk_hash(int device, cudaStream_t s, const unsigned long long* d_counts, const ChunkArgs& chunks,
                               unsigned long long* d_hashes, uint64_t n, uint32_t* d_err);
+// Result chunks into CSR (after the counts are scanned into d_offsets);
+// per = 2 for ranges (two entries a result; d_out and out_capacity count entries).
 cudaError_t launch_chunk_compact(int device, cudaStream_t s, const unsigned long long* d_counts,
                                  const unsigned long long* d_offsets, const ChunkArgs& chunks, uint32_t* d_out,
                                  uint64_t out_capacity, uint64_t n, const uint64_t* d_n, uint32_t* d_err,

@@ -279,7 +279,7 @@ struct oct_engine_s {
     DevBuf counts, offs, part, out;
     DevBuf knn_idx, knn_d2, knn_counts;
     DevBuf ctrs, stats, summary, totals;
-    DevBuf ck_pool, ck_next, ck_first, ck_ctr;  // one-pass radius: result chunks (ck_next has one word per chunk)
+    DevBuf ck_pool, ck_rec, ck_ctr;  // one-pass radius: result chunks, their queries and places
     DevBuf knn_fb;  // group kNN fallback list, one entry per query position
     DevBuf knn_heads;  // group kNN: the heads' largest k-th distances (f64 per head)
     DevBuf hash_out;   // oct_engine_copy_radius_hash's counts and hashes before they go to the host
@@ -383,8 +383,8 @@ int grow_pinned(oct_engine e, size_t bytes) {
 size_t table_offset() { return (sizeof(EngineDyn) + 255) & ~(size_t)255; }
 
 ChunkArgs chunk_args(oct_engine e) {
-    const uint64_t cap = std::min<uint64_t>(e->ck_next.bytes / 4, e->ck_pool.bytes / (4ull * kResultChunk));
-    return ChunkArgs{e->ck_pool.as<uint32_t>(), e->ck_next.as<uint32_t>(), e->ck_first.as<uint32_t>(),
+    const uint64_t cap = std::min<uint64_t>(e->ck_rec.bytes / sizeof(uint2), e->ck_pool.bytes / (4ull * kResultChunk));
+    return ChunkArgs{e->ck_pool.as<uint32_t>(), e->ck_rec.as<uint2>(),
                      e->ck_ctr.as<uint32_t>(), (uint32_t)std::min<uint64_t>(cap, 0xfffffff0ull)};
 }
 
@@ -456,7 +456,7 @@ cudaError_t enqueue_work(oct_engine e) {
             k_escan_top<<<1, kScanThreads, 0, s>>>(part, kScanBlocks, sum);
             k_escan_apply<<<kScanBlocks, kScanThreads, 0, s>>>(counts, &dyn->n_radius, part, offs);
         };
-        // one traversal: results into chunk chains, scan, chains compacted into the result array
+        // one traversal: results into chunks, scan, chunks compacted into the result array
         const ChunkArgs ck = chunk_args(e);
         if ((r = cudaMemsetAsync(ck.ctr, 0, 4, s)) != cudaSuccess) return r;
         for (int v = 0; v < kRadiusVariants; ++v) {
@@ -540,7 +540,7 @@ int launch_batch(oct_engine e, bool record_start) {
 int grow_chunks(oct_engine e, uint64_t chunks) {
     if (chunks > 0xfffffff0ull) return fail(e, OCT_ERR_INVALID_ARG, "too many radius results for one batch");
     int st;
-    if ((st = grow(e, e->ck_next, 4 * chunks)) != OCT_OK) return st;
+    if ((st = grow(e, e->ck_rec, sizeof(uint2) * chunks)) != OCT_OK) return st;
     return grow(e, e->ck_pool, 4ull * kResultChunk * chunks);
 }
 
@@ -685,8 +685,7 @@ int submit(oct_engine e, const oct_request* rq, uint32_t n) {
         if ((st = grow(e, e->knn_heads, 8 * (groups / kKnnHeadStride + 2))) != OCT_OK) return st;
     }
     if ((st = grow(e, e->totals, sizeof(ReqTotal) * std::max<uint32_t>(m, 1))) != OCT_OK) return st;
-    if (n_radius) {  // one-pass radius: a first chunk per query, a pool of at least 3 chunks per query
-        if ((st = grow(e, e->ck_first, 4 * n_radius)) != OCT_OK) return st;
+    if (n_radius) {  // one-pass radius: a pool of at least 3 chunks per query
         if ((st = grow(e, e->ck_ctr, 256)) != OCT_OK) return st;
         const uint64_t have = chunk_args(e).cap;
         const uint64_t want = std::max<uint64_t>(3 * n_radius + 1024, e->out.bytes / (4ull * kResultChunk) + n_radius);
@@ -861,7 +860,7 @@ int oct_engine_create(const oct_engine_params* p, oct_engine* out) {
         DevBuf* per_q8[] = {&e->keys[0], &e->keys[1], &e->counts, &e->offs};
         for (DevBuf* b : per_q8)
             if (r == cudaSuccess && grow(e, *b, 8 * (q + 1)) != OCT_OK) r = cudaErrorMemoryAllocation;
-        DevBuf* per_q4[] = {&e->ord[0], &e->ord[1], &e->knn_counts, &e->knn_fb, &e->ck_first};
+        DevBuf* per_q4[] = {&e->ord[0], &e->ord[1], &e->knn_counts, &e->knn_fb};
         for (DevBuf* b : per_q4)
             if (r == cudaSuccess && grow(e, *b, 4 * (q + 1)) != OCT_OK) r = cudaErrorMemoryAllocation;
         // kNN results of up to 256 neighbours per centre, the request table of 1024 requests, the sort's
@@ -905,7 +904,7 @@ int oct_engine_destroy(oct_engine e) {
         for (DevBuf* b : fixed) b->release();
         DevBuf* pooled[] = {&e->desc, &e->keys[0], &e->keys[1], &e->ord[0], &e->ord[1], &e->sort_status,
                             &e->counts, &e->offs, &e->out, &e->knn_idx, &e->knn_d2, &e->knn_counts, &e->totals,
-                            &e->ck_pool, &e->ck_next, &e->ck_first, &e->ck_ctr, &e->knn_fb, &e->knn_heads,
+                            &e->ck_pool, &e->ck_rec, &e->ck_ctr, &e->knn_fb, &e->knn_heads,
                             &e->hash_out};
         for (DevBuf* b : pooled) {
             if (b->ptr && e->stream) cudaFreeAsync(b->ptr, e->stream);
@@ -1142,7 +1141,7 @@ int oct_engine_memory(oct_engine e, uint64_t* bytes) {
     const DevBuf* bufs[] = {&e->desc, &e->keys[0], &e->keys[1], &e->ord[0], &e->ord[1], &e->sort_ctl,
                             &e->sort_status, &e->epoch, &e->counts, &e->offs, &e->part, &e->out, &e->knn_idx,
                             &e->knn_d2, &e->knn_counts, &e->ctrs, &e->stats, &e->summary, &e->totals,
-                            &e->ck_pool, &e->ck_next, &e->ck_first, &e->ck_ctr, &e->knn_fb,
+                            &e->ck_pool, &e->ck_rec, &e->ck_ctr, &e->knn_fb,
                             &e->knn_heads, &e->hash_out};
     uint64_t s = 0;
     for (const DevBuf* b : bufs) s += b->bytes;

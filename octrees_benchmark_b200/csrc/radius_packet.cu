@@ -47,6 +47,7 @@
 // Cube / square: per axis, the interval bounds bmin = c - r and bmax = c + r
 // (FP64) are made leaf-relative and rounded to FP32; an axis is certain when
 // its margin exceeds 2^-22 (|p_i| + |bound_i|).
+#include <algorithm>
 #include <cfloat>
 
 #include "cloud.h"
@@ -82,8 +83,7 @@ struct PacketArgs {
     uint32_t* err;
     // one-pass mode: each query's results go to its own chain of kChunk-entry chunks
     uint32_t* chunk_pool;       // chunk_cap x kChunk entries
-    uint32_t* chunk_next;       // next chunk of a chain (chunk_cap)
-    uint32_t* chunk_first;      // first chunk of each query (per query position)
+    uint2* chunk_rec;           // the query position a chunk belongs to, its number in the query's chain (chunk_cap)
     uint32_t* chunk_ctr;        // chunks handed out
     uint32_t chunk_cap;
 };
@@ -290,9 +290,10 @@ __device__ __forceinline__ bool inside_of(const double (*q)[kQpRow], int j, doub
 
 // MODE 0 counts, 1 fills at scanned offsets, 2 (one pass) appends each query's
 // results to its own chain of kChunk-entry chunks taken from a pool (contiguous
-// chunks for one long range, so positions stay linear); per query the count and
-// the first chunk are written, and k_chunk_compact moves every chain into the CSR
-// array after the scan.  A neighborsStruct range takes two entries.
+// chunks for one long range, so positions stay linear); per query the count is
+// written, per chunk its query and its number in the chain, and k_chunk_compact
+// moves every chunk into the CSR array after the scan.  A neighborsStruct range
+// takes two entries.
 //
 // Leaves are tested in groups: up to kLeafGroup leaves that are next on the stack
 // (ascending, possibly with gaps) form one run of points, 32 of them on the lanes
@@ -383,8 +384,9 @@ __global__ void __launch_bounds__(kPkThreads) k_radius_packet(PacketArgs a) {
         if (MODE == 1 && valid) base = a.offs[qi];
         bool overflow = false;
         uint32_t open_at = kNotOpen;  // neighborsStruct: first point of the run that crosses into the next 32 points
-        // one-pass mode: this lane's chain (current chunk, entries used in it, first chunk)
-        uint32_t ck_cur = kNoChunk, ck_fill = kChunk, ck_first = kNoChunk;
+        // one-pass mode: this lane's chain (current chunk, entries used in it); its chunks are full up to the
+        // current one, so the count says how many there are
+        uint32_t ck_cur = kNoChunk, ck_fill = kChunk;
         bool ck_over = false;
 
         // Reserve n > 0 entries at the end of lane j's chain (warp-uniform call):
@@ -395,6 +397,9 @@ __global__ void __launch_bounds__(kPkThreads) k_radius_packet(PacketArgs a) {
         struct ChunkPos {
             uint32_t cur, fill, room, nc;
         };
+        auto chain_len = [&]() -> uint32_t {  // before the results being added are counted
+            return kRanges ? (cnt + kChunk / 2 - 1) / (kChunk / 2) : (cnt + kChunk - 1) / kChunk;
+        };
         auto chunk_reserve = [&](int j, uint32_t n) -> ChunkPos {
             ChunkPos p;
             p.cur = __shfl_sync(0xffffffffu, ck_cur, j);
@@ -404,19 +409,23 @@ __global__ void __launch_bounds__(kPkThreads) k_radius_packet(PacketArgs a) {
             if (n > p.room) {
                 const uint32_t m = (n - p.room + kChunk - 1) / kChunk;
                 uint32_t nc = 0;
-                if (lane == 0) nc = atomicAdd(a.chunk_ctr, m);
-                nc = __shfl_sync(0xffffffffu, nc, 0);
+                if (lane == j) nc = atomicAdd(a.chunk_ctr, m);
+                nc = __shfl_sync(0xffffffffu, nc, j);
                 const bool fits = (uint64_t)nc + m <= a.chunk_cap;
                 if (fits) {
                     p.nc = nc;
-                    if (lane == 0 && p.cur != kNoChunk) a.chunk_next[p.cur] = nc;
-                    for (uint32_t t = lane; t + 1 < m; t += 32) a.chunk_next[nc + t] = nc + t + 1;
+                    if (m > 1) {  // the chunks after the first, which is lane j's to record
+                        const uint32_t owner = __shfl_sync(0xffffffffu, qi, j), num = __shfl_sync(0xffffffffu, chain_len(), j);
+                        for (uint32_t t = 1 + lane; t < m; t += 32) {
+                            a.chunk_rec[nc + t] = make_uint2(owner, num + t);
+                        }
+                    }
                 } else {
                     ck_over = true;
                 }
                 if (lane == j) {
                     if (fits) {
-                        if (ck_cur == kNoChunk) ck_first = nc;
+                        a.chunk_rec[nc] = make_uint2(qi, chain_len());
                         ck_cur = nc + m - 1;
                         ck_fill = n - p.room - (m - 1) * kChunk;
                     } else {
@@ -448,8 +457,7 @@ __global__ void __launch_bounds__(kPkThreads) k_radius_packet(PacketArgs a) {
                 if (!room) {
                     const uint32_t nc = atomicAdd(a.chunk_ctr, 1u);
                     if (nc < a.chunk_cap) {
-                        if (ck_cur != kNoChunk) a.chunk_next[ck_cur] = nc;
-                        else ck_first = nc;
+                        a.chunk_rec[nc] = make_uint2(qi, chain_len());
                         ck_cur = nc;
                         ck_fill = 0;
                         room = true;
@@ -799,7 +807,6 @@ __global__ void __launch_bounds__(kPkThreads) k_radius_packet(PacketArgs a) {
         if (kChain && ck_over) set_err(a.err, kErrChunkCapacity);
         if (MODE != 1 && valid) {
             a.counts[qi] = cnt;
-            if (kChain) a.chunk_first[qi] = ck_first;
             if (kRanges) a.counts2[qi] = cnt2;
         }
         __syncwarp();
@@ -883,128 +890,97 @@ cudaError_t launch_pk_a(const PacketArgs& a, int algo, int mode, bool fp32, int 
     }
 }
 
-// Each radius query's chain of result chunks into its CSR slot.  A warp takes
-// S queries at a time (S from 4 up to 32, as many as keep every warp busy):
-// their counts, offsets and first chunks come in one coalesced round trip; then
-// the chains of kCompactBatch queries are walked in lockstep, each step loading
-// one chunk of every one of them (and their next links) before storing any, so
-// the four latency chains overlap.
+// Result chunks into the CSR array, every chunk by itself: its query's count and offset and its number in the
+// chain say where its entries go.  A warp takes up to 32 chunks at a time, their records in coalesced reads, and copies
+// kCompactBatch of them a step, the loads of all before any store.  Bound: HBM (8 bytes a result), and the
+// sectors that a query's last chunk leaves half empty.  Following each query's links from chunk to chunk, four
+// queries in lockstep, took 133 us for the 36.8M results of 500k queries, 195 for 59M in long chains and 981 for
+// a 16-cloud batch; this form takes 106, 118 and 661.
 constexpr int kCompactBatch = 4;
 static_assert(kChunk == 64, "a chunk is two 32-entry rows");
 
 __global__ void __launch_bounds__(256) k_chunk_compact(const unsigned long long* __restrict__ counts,
                                                        const unsigned long long* __restrict__ offs,
-                                                       const uint32_t* __restrict__ first,
-                                                       const uint32_t* __restrict__ next,
-                                                       const uint32_t* __restrict__ pool, uint64_t chunk_cap,
+                                                       const uint2* __restrict__ rec,
+                                                       const uint32_t* __restrict__ pool,
+                                                       const uint32_t* __restrict__ ctr, uint32_t chunk_cap,
                                                        uint32_t* __restrict__ out, uint64_t out_cap, uint64_t n,
                                                        const uint64_t* d_n, uint32_t per, uint32_t* err) {
     // per: entries of a result (1 index, or 2 for a range); counts and offsets count results
     if (d_n) n = *d_n;
     const int lane = threadIdx.x & 31;
+    const uint64_t chunks = min(*ctr, chunk_cap);
     const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    uint32_t S = kCompactBatch;
-    while (S < 32 && (uint64_t)S * nwarps < n) S <<= 1;
-    bool bad = false;  // a chain cut short by a pool overflow (reported by the search kernel), or no room
-    for (uint64_t q0 = (((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * S; q0 < n; q0 += nwarps * S) {
-        const uint64_t q = q0 + lane;
-        unsigned long long cnt = 0, o = 0;
-        uint32_t c0 = kNoChunk;
-        if ((uint32_t)lane < S && q < n) {
-            cnt = counts[q] * per;
-            if (cnt) {
-                o = offs[q] * per;
-                c0 = first[q];
+    uint32_t S = kCompactBatch;  // chunks a warp takes at a time: as many as keep every warp busy
+    while (S < 32 && S * nwarps < chunks) S <<= 1;
+    bool bad = false;  // a chunk without a query (the pool ran over, which the search reported), or no room
+    for (uint64_t c0 = (((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * S; c0 < chunks; c0 += nwarps * S) {
+        const uint64_t c = c0 + lane;
+        uint32_t len = 0;
+        unsigned long long dst = 0;
+        if ((uint32_t)lane < S && c < chunks) {
+            const uint2 r = rec[c];
+            const uint32_t q = r.x;
+            if (q < n) {
+                const unsigned long long total = counts[q] * per, at = (unsigned long long)r.y * kChunk;
+                if (at < total) {
+                    len = total - at < kChunk ? (uint32_t)(total - at) : kChunk;
+                    dst = offs[q] * per + at;
+                    if (dst + len > out_cap) {
+                        bad = true;
+                        len = 0;
+                    }
+                }
+            } else {
+                bad = true;
             }
         }
-        uint32_t todo = __ballot_sync(0xffffffffu, cnt != 0);
-        while (todo) {
-            unsigned long long cj[kCompactBatch], dst[kCompactBatch], done[kCompactBatch];
-            uint32_t cur[kCompactBatch];
+        for (uint32_t t = 0; t < S && c0 + t < chunks; t += kCompactBatch) {
+            uint32_t v[kCompactBatch][2], m[kCompactBatch];
+            unsigned long long d[kCompactBatch];
 #pragma unroll
             for (int b = 0; b < kCompactBatch; ++b) {
-                const int j = todo ? __ffs(todo) - 1 : -1;
-                todo &= todo - 1;
-                const unsigned long long cb = __shfl_sync(0xffffffffu, cnt, j & 31);
-                cj[b] = j >= 0 ? cb : 0ull;
-                dst[b] = __shfl_sync(0xffffffffu, o, j & 31);
-                cur[b] = __shfl_sync(0xffffffffu, c0, j & 31);
-                done[b] = 0;
+                m[b] = __shfl_sync(0xffffffffu, len, t + b);
+                d[b] = __shfl_sync(0xffffffffu, dst, t + b);
+                const uint32_t* src = pool + (c0 + t + b) * kChunk + lane;
+                if ((uint32_t)lane < m[b]) v[b][0] = src[0];
+                if ((uint32_t)lane + 32 < m[b]) v[b][1] = src[32];
             }
-            for (;;) {  // one chunk of every unfinished chain per step (warp-uniform)
-                bool any = false;
 #pragma unroll
-                for (int b = 0; b < kCompactBatch; ++b) any = any || done[b] < cj[b];
-                if (!any) break;
-                uint32_t v[kCompactBatch][2], nx[kCompactBatch];
-#pragma unroll
-                for (int b = 0; b < kCompactBatch; ++b) {
-                    v[b][0] = v[b][1] = 0;
-                    nx[b] = kNoChunk;
-                    if (done[b] < cj[b] && cur[b] < chunk_cap) {
-#pragma unroll
-                        for (int h = 0; h < 2; ++h) {
-                            const uint32_t t = 32u * h + lane;
-                            if (done[b] + t < cj[b]) v[b][h] = pool[(uint64_t)cur[b] * kChunk + t];
-                        }
-                        if (done[b] + kChunk < cj[b]) nx[b] = next[cur[b]];
-                    }
-                }
-#pragma unroll
-                for (int b = 0; b < kCompactBatch; ++b) {
-                    if (done[b] >= cj[b]) continue;
-                    if (cur[b] >= chunk_cap) {
-                        bad = true;
-                        done[b] = cj[b];
-                        continue;
-                    }
-#pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        const uint32_t t = 32u * h + lane;
-                        if (done[b] + t < cj[b]) {
-                            const unsigned long long w = dst[b] + done[b] + t;
-                            if (w < out_cap) out[w] = v[b][h];
-                            else bad = true;
-                        }
-                    }
-                    done[b] = (cj[b] - done[b] > kChunk) ? done[b] + kChunk : cj[b];
-                    cur[b] = nx[b];
-                }
+            for (int b = 0; b < kCompactBatch; ++b) {
+                uint32_t* to = out + d[b] + lane;
+                if ((uint32_t)lane < m[b]) to[0] = v[b][0];
+                if ((uint32_t)lane + 32 < m[b]) to[32] = v[b][1];
             }
         }
     }
     if (bad) set_err(err, kErrOutputCapacity);
 }
 
-// One warp per query: the sum of mix64 over the query's result chain (the
-// count is the search's), instead of moving the chain into a CSR array.
+// The sum of mix64 over each query's results (the count is the search's), a chunk a warp; hashes zeroed before.
 __global__ void __launch_bounds__(256) k_chunk_hash(const unsigned long long* __restrict__ counts,
-                                                    const uint32_t* __restrict__ first,
-                                                    const uint32_t* __restrict__ next,
-                                                    const uint32_t* __restrict__ pool, uint64_t chunk_cap,
+                                                    const uint2* __restrict__ rec,
+                                                    const uint32_t* __restrict__ pool,
+                                                    const uint32_t* __restrict__ ctr, uint32_t chunk_cap,
                                                     unsigned long long* __restrict__ hashes, uint64_t n,
                                                     uint32_t* err) {
     const int lane = threadIdx.x & 31;
     const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    for (uint64_t q = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; q < n; q += nwarps) {
-        const unsigned long long cnt = counts[q];
-        unsigned long long h = 0;
-        uint32_t c = first[q];
-        bool bad = false;
-        for (unsigned long long done = 0; done < cnt;) {
-            if (c >= chunk_cap) {  // a chain cut short by a pool overflow (reported by the search kernel)
-                bad = true;
-                break;
-            }
-            const unsigned long long m = (cnt - done < kChunk) ? (cnt - done) : kChunk;
-            for (uint32_t t = lane; t < m; t += 32) h += mix64(pool[(uint64_t)c * kChunk + t]);
-            done += m;
-            if (done < cnt) c = next[c];
+    const uint64_t chunks = min(*ctr, chunk_cap);
+    for (uint64_t c = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; c < chunks; c += nwarps) {
+        const uint2 r = rec[c];
+        const uint32_t q = r.x;
+        if (q >= n) {  // the pool ran over (reported by the search kernel)
+            if (lane == 0) set_err(err, kErrOutputCapacity);
+            continue;
         }
+        const unsigned long long total = counts[q], at = (unsigned long long)r.y * kChunk;
+        unsigned long long h = 0;
+        if (at + lane < total) h += mix64(pool[c * kChunk + lane]);
+        if (at + lane + 32 < total) h += mix64(pool[c * kChunk + lane + 32]);
 #pragma unroll
         for (int off = 16; off > 0; off >>= 1) h += __shfl_xor_sync(0xffffffffu, h, off);
-        if (lane == 0) hashes[q] = h;
-        if (bad && lane == 0) set_err(err, kErrOutputCapacity);
+        if (lane == 0) atomicAdd(&hashes[q], h);
     }
 }
 
@@ -1098,8 +1074,7 @@ cudaError_t launch_radius_table(int device, cudaStream_t s, int kernel, int algo
     a.stats = d_stats;
     a.err = d_err;
     a.chunk_pool = chunks ? chunks->pool : nullptr;
-    a.chunk_next = chunks ? chunks->next : nullptr;
-    a.chunk_first = chunks ? chunks->first : nullptr;
+    a.chunk_rec = chunks ? chunks->rec : nullptr;
     a.chunk_ctr = chunks ? chunks->ctr : nullptr;
     a.chunk_cap = chunks ? chunks->cap : 0;
     if (mode == 2 && (!chunks || (algo == kStruct && !d_counts2))) return cudaErrorInvalidValue;
@@ -1118,11 +1093,13 @@ cudaError_t launch_radius_table(int device, cudaStream_t s, int kernel, int algo
 cudaError_t launch_chunk_hash(int device, cudaStream_t s, const unsigned long long* d_counts, const ChunkArgs& chunks,
                               unsigned long long* d_hashes, uint64_t n, uint32_t* d_err) {
     if (n == 0) return cudaSuccess;
+    const cudaError_t e = cudaMemsetAsync(d_hashes, 0, 8 * n, s);
+    if (e != cudaSuccess) return e;
     const uint64_t cap = (uint64_t)sm_count_p(device) * 8;
-    const uint64_t want = (n + 7) / 8;
+    const uint64_t want = ((uint64_t)chunks.cap + 7) / 8;
     const int grid = (int)(want < cap ? want : cap);
-    k_chunk_hash<<<grid, 256, 0, s>>>(d_counts, chunks.first, chunks.next, chunks.pool, chunks.cap, d_hashes, n,
-                                      d_err);
+    k_chunk_hash<<<grid, 256, 0, s>>>(d_counts, chunks.rec, chunks.pool, chunks.ctr, chunks.cap, d_hashes,
+                                      n, d_err);
     return cudaGetLastError();
 }
 
@@ -1130,12 +1107,14 @@ cudaError_t launch_chunk_compact(int device, cudaStream_t s, const unsigned long
                                  const unsigned long long* d_offsets, const ChunkArgs& chunks, uint32_t* d_out,
                                  uint64_t out_capacity, uint64_t n, const uint64_t* d_n, uint32_t* d_err,
                                  uint32_t per) {
-    if (!d_n && n == 0) return cudaSuccess;
+    if ((!d_n && n == 0) || chunks.cap == 0) return cudaSuccess;
     const uint64_t cap = (uint64_t)sm_count_p(device) * 8;
-    const uint64_t want = d_n ? cap : (n + 31) / 32;  // 8 warps of at least 4 queries per block
-    const int grid = (int)(want < cap ? (want ? want : 1) : cap);
-    k_chunk_compact<<<grid, 256, 0, s>>>(d_counts, d_offsets, chunks.first, chunks.next, chunks.pool, chunks.cap,
-                                         d_out, out_capacity, n, d_n, per, d_err);
+    // a single search's chunks: its results' and a last one of every query
+    const uint64_t most = d_n ? chunks.cap : std::min<uint64_t>(chunks.cap, out_capacity / kChunk + n + 1);
+    const uint64_t want = (most + 31) / 32;  // 8 warps of at least kCompactBatch chunks a block
+    const int grid = (int)(want < cap ? want : cap);
+    k_chunk_compact<<<grid, 256, 0, s>>>(d_counts, d_offsets, chunks.rec, chunks.pool, chunks.ctr,
+                                         chunks.cap, d_out, out_capacity, n, d_n, per, d_err);
     return cudaGetLastError();
 }
 
