@@ -64,11 +64,11 @@ LAUNCHES_PER_STEP = {"plain": 6, "packet": 10 + 7, "packet_fp32": 10 + 7, "knn_p
                      "engine": 15}
 BUILD_BYTES_PER_POINT = 112  # encode 32 + sort 20 + reorder 52 + leaf counting 8
 BUILD_BYTES_PER_NODE = 36    # offsets 4 + ranges 8 + centers 24
-# DRAM bytes (read + write) per query of the search kernels, from ncu --set full of this script's
-# `--points 6000000 --queries 200000 --search packet --paths packet` case (6M points at this tile's density,
-# 200k queries each): k_knn_group k=50 511.8 + 143.8 MB, one-pass k_radius_packet r=2.5 342.3 + 58.8 MB
-KNN_DRAM_BYTES_PER_QUERY = (511.8e6 + 143.8e6) / 200_000
-RADIUS_DRAM_BYTES_PER_QUERY = (342.3e6 + 58.8e6) / 200_000
+# DRAM bytes (read + write) per query of the search kernels, from ncu captures of this script's
+# tile at 6M points (the same density, 200k queries each): k_knn_group k=50 355.6 + 125.2 MB, one-pass
+# k_radius_packet r=2.5 207.5 + 50.3 MB
+KNN_DRAM_BYTES_PER_QUERY = (355.6e6 + 125.2e6) / 200_000
+RADIUS_DRAM_BYTES_PER_QUERY = (207.5e6 + 50.3e6) / 200_000
 
 
 def measured_peak():
@@ -629,7 +629,7 @@ def run_b200(args, rank, world, local_rank):
     flush = torch.empty(L2_FLUSH_BYTES // 4, dtype=torch.float32, device="cuda")
     ev = [torch.cuda.Event(enable_timing=True) for _ in range(4)]
 
-    # (packet, fp32_filter, lanes, kNN in groups of 4 queries per warp)
+    # (packet, fp32_filter, lanes, kNN by collecting within a threshold)
     # (packet, fp32_filter, lanes, knn_packet); fp32_filter 1: the radius and kNN FP32 filters, 2: radius only
     SEARCH_PATHS = {"plain": (0, 0, args.radius_group, 0), "packet": (1, 0, 8, 1), "packet_fp32": (1, 1, 8, 1),
                     "packet_fp32_radius": (1, 2, 8, 1), "knn_per_query": (1, 0, 8, 0), "engine": (1, 0, 8, 1),
