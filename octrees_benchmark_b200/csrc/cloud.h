@@ -340,8 +340,8 @@ cudaError_t launch_knn_table(int device, cudaStream_t s, const DynGroup* d_grp, 
                              uint32_t kmax, const uint32_t* d_order, uint32_t bucket, uint32_t* d_idx, double* d_d2,
                              uint32_t* d_counts, uint32_t* d_err, int blocks_per_sm = 0, double est = 0.0);
 // Curve-ordered kNN of a batch group, then the sorted-list kernels over the queries it hands back.  d_fb: the
-// fallback group (requests, kmax and q_begin of d_grp, nq = 0 before the
-// launch); d_fb_list: one entry per query position of the batch; d_packet_ctr:
+// fallback group (requests, kmax and q_begin of d_grp; its nq is set to 0
+// here, so that the launch can be repeated); d_fb_list: one entry per query position of the batch; d_packet_ctr:
 // three counters; blocks_per_sm > 0 caps the resident blocks of both launches.
 cudaError_t launch_knn_group_table(int device, cudaStream_t s, const DynGroup* d_grp, DynGroup* d_fb,
                                    const SearchReq* single, uint32_t kmax, const uint32_t* d_order, uint32_t bucket,

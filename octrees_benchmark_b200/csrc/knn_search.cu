@@ -1686,6 +1686,9 @@ cudaError_t launch_knn_group_table(int device, cudaStream_t s, const DynGroup* d
     if (kmax > 1024) return cudaErrorInvalidValue;
     cudaError_t e;
     if ((e = cudaMemsetAsync(d_packet_ctr, 0, 12, s)) != cudaSuccess) return e;
+    // a batch whose radius results outgrew their arrays runs again from the same table: the queries handed back
+    // are counted from 0 each time (the list has one entry a query)
+    if ((e = cudaMemsetAsync(&d_fb->nq, 0, sizeof(d_fb->nq), s)) != cudaSuccess) return e;
     KnnGroupArgs g{};
     g.single = single ? *single : SearchReq{};
     g.grp = d_grp;
