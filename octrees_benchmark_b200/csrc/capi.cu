@@ -156,6 +156,8 @@ cudaError_t radius_pass(Cloud& c, int kernel, int algo, bool fill, const double*
                                 *order, counts, counts2, offs, out, cap);
 }
 
+ChunkArgs cloud_chunks(const Cloud& c) { return chunk_args(c.ck_pool, c.ck_rec, c.ck_ctr); }
+
 // Radius search in one traversal (packet path, FP64 or FP32 filter): every query's results go
 // to its chain of result chunks, the counts are scanned, and the chunks are
 // compacted into the CSR output.  A pool that turned out too small leaves the
@@ -177,16 +179,11 @@ int radius_chunks(Cloud& c, int kernel, int algo, const double* dq, uint64_t nq,
     uint64_t tot = 0;
     for (int attempt = 0; attempt < 2; ++attempt) {
         // pool: every query's partial last chunk plus the results (a guess of 128 per query at first)
-        const uint64_t want = attempt == 0 ? std::max<uint64_t>(c.ck_cap, 3 * nq + 1024)
-                                           : per * tot / kResultChunk + nq + 1024;
+        const uint64_t want = attempt == 0 ? 3 * nq + 1024 : per * tot / kResultChunk + nq + 1024;
         if (want > 0xfffffff0ull) return set_error(c, OCT_ERR_INVALID_ARG, "too many results for one call");
-        if (want > c.ck_cap) {
-            CK(c.ck_pool.reserve(4ull * kResultChunk * want));
-            CK(c.ck_rec.reserve(sizeof(uint2) * want));
-            c.ck_cap = (uint32_t)want;
-        }
-        ChunkArgs ck{c.ck_pool.as<uint32_t>(), c.ck_rec.as<uint2>(),
-                     c.ck_ctr.as<uint32_t>(), c.ck_cap};
+        CK(c.ck_pool.reserve(4ull * kResultChunk * want));
+        CK(c.ck_rec.reserve(sizeof(uint2) * want));
+        const ChunkArgs ck = cloud_chunks(c);
         CK(cudaMemsetAsync(ck.ctr, 0, 4, c.stream));
         CK(launch_radius_packet(c, kernel, pass_algo, 2, fp32_on_radius(c.fp32_filter), dq, nq, dr, radius, order,
                                 dc, d_points, nullptr, nullptr, 0, &ck));
@@ -223,8 +220,7 @@ int radius_one_pass(Cloud& c, int kernel, int algo, const double* dq, uint64_t n
         CK(c.q_out.reserve(4 * (tot ? tot : 1)));
         dout = c.q_out.as<uint32_t>();
     }
-    ChunkArgs ck{c.ck_pool.as<uint32_t>(), c.ck_rec.as<uint2>(),
-                 c.ck_ctr.as<uint32_t>(), c.ck_cap};
+    const ChunkArgs ck = cloud_chunks(c);
     CK(launch_chunk_compact(c.device, c.stream, dc, doffs, ck, dout, tot, nq, nullptr, c.d_err.as<uint32_t>()));
     if (!dev && tot) CK(cudaMemcpyAsync(idx, dout, 4 * tot, cudaMemcpyDeviceToHost, c.stream));
     if (!dev) return sync_and_check(c);
@@ -1081,8 +1077,7 @@ int oct_radius_hash(oct_cloud h, int kernel, int algo, const double* centers, ui
         CK(c.q_out2.reserve(8 * nq));
         dh = c.q_out2.as<unsigned long long>();
     }
-    ChunkArgs ck{c.ck_pool.as<uint32_t>(), c.ck_rec.as<uint2>(),
-                 c.ck_ctr.as<uint32_t>(), c.ck_cap};
+    const ChunkArgs ck = cloud_chunks(c);
     const unsigned long long* dc = c.q_counts.as<unsigned long long>();
     CK(launch_chunk_hash(c.device, c.stream, dc, ck, dh, nq, c.d_err.as<uint32_t>()));
     if (dev) {
@@ -1212,8 +1207,7 @@ static int ranges_search(oct_cloud h, int kernel, const double* centers, uint64_
         dout = c.q_out.as<uint32_t>();
     }
     if (one_pass) {
-        const ChunkArgs ck{c.ck_pool.as<uint32_t>(), c.ck_rec.as<uint2>(),
-                           c.ck_ctr.as<uint32_t>(), c.ck_cap};
+        const ChunkArgs ck = cloud_chunks(c);
         CK(launch_chunk_compact(c.device, c.stream, dranges, doffs, ck, dout, 2 * tot, nq, nullptr,
                                 c.d_err.as<uint32_t>(), 2));
     } else {

@@ -230,7 +230,6 @@ struct Cloud {
     uint32_t knn_chunk = kKnnGroupChunk;  // group kNN: consecutive groups per warp fetch
     // one-pass radius search: result chunk pool, each chunk's query and place in its chain, counter
     DevBuf ck_pool, ck_rec, ck_ctr;
-    uint32_t ck_cap = 0;
 
     // pinned host staging for small readbacks
     void* pinned = nullptr;
@@ -309,6 +308,13 @@ struct ChunkArgs {
     uint32_t cap;
 };
 constexpr uint32_t kResultChunk = 64;
+// The chunks of arrays as they are now: an array that could not be grown is empty, and so is the pool then.
+inline ChunkArgs chunk_args(const DevBuf& pool, const DevBuf& rec, const DevBuf& ctr) {
+    const uint64_t a = pool.bytes / (4ull * kResultChunk), b = rec.bytes / sizeof(uint2);
+    const uint64_t cap = a < b ? a : b;
+    return ChunkArgs{pool.as<uint32_t>(), rec.as<uint2>(), ctr.as<uint32_t>(),
+                     (uint32_t)(cap < 0xfffffff0ull ? cap : 0xfffffff0ull)};
+}
 
 // Queries per packet (1 to 32) of a packet radius launch over nq queries.
 uint32_t packet_width(uint64_t nq, int device);

@@ -382,11 +382,7 @@ int grow_pinned(oct_engine e, size_t bytes) {
 
 size_t table_offset() { return (sizeof(EngineDyn) + 255) & ~(size_t)255; }
 
-ChunkArgs chunk_args(oct_engine e) {
-    const uint64_t cap = std::min<uint64_t>(e->ck_rec.bytes / sizeof(uint2), e->ck_pool.bytes / (4ull * kResultChunk));
-    return ChunkArgs{e->ck_pool.as<uint32_t>(), e->ck_rec.as<uint2>(),
-                     e->ck_ctr.as<uint32_t>(), (uint32_t)std::min<uint64_t>(cap, 0xfffffff0ull)};
-}
+ChunkArgs chunk_args(oct_engine e) { return chunk_args(e->ck_pool, e->ck_rec, e->ck_ctr); }
 
 // Result chunks for `chunks` chunks (grows both arrays; a new address drops the graphs).
 int grow_chunks(oct_engine e, uint64_t chunks);
