@@ -192,7 +192,8 @@ int oct_search_kernel_times(oct_cloud cloud, double* radius_ms, uint64_t* radius
                             uint64_t* knn_launches, int reset);
 
 /* Upload n points (xyz AoS).  Replaces filling the reference's PointsAoS
- * container (inc/geometry/point_containers.hpp:32-65). */
+ * container (inc/geometry/point_containers.hpp:32-65).  If it fails for want
+ * of memory, a cloud that was sorted or built before answers as before. */
 int oct_set_points(oct_cloud cloud, const double* xyz, uint64_t n, uint32_t flags);
 
 /* Bounding box, SFC keys, stable key sort and point reorder.  Replaces

@@ -688,24 +688,27 @@ int oct_set_points(oct_cloud h, const double* xyz, uint64_t n, uint32_t flags) {
     if (n && !xyz) return set_error(c, OCT_ERR_INVALID_ARG, "xyz is NULL");
     if (n >= 0xffffffffull) return set_error(c, OCT_ERR_INVALID_ARG, "more than 2^32 - 2 points");
     DeviceGuard g(c.device);
-    // the old points are gone from here on, whatever fails
-    c.n = 0;
+    // the points as uploaded: no search reads them, so that a failure leaves a sorted (or built) cloud as it was;
+    // points that wait for their sort are gone
+    const uint64_t sorted_n = c.sorted ? c.n : 0;
+    const bool more = c.xyz_in.bytes < 24 * n;
+    c.n = sorted_n;
+    CK(c.xyz_in.reserve(24 * (n ? n : 1)));
+    if (n) {
+        CK(cudaMemcpyAsync(c.xyz_in.ptr, xyz, 24 * n,
+                           (flags & OCT_MEM_DEVICE) ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, c.stream));
+    }
     c.sorted = false;
     c.built = false;
     c.rel_built = false;
     c.crel_built = false;
     c.node_capacity = 0;
-    if (n && c.split_sort && c.xyz_in.bytes < 24 * n) {
+    if (more && c.split_sort) {
         // more points than before: new arrays, cut from one slab (the old slab goes with all that is cut from it)
         for (DevBuf* b : cloud_bufs(c))
             if (b->slice) b->release();
         c.slab.release();
         reserve_point_arrays(c, n);
-    }
-    CK(c.xyz_in.reserve(24 * (n ? n : 1)));
-    if (n) {
-        CK(cudaMemcpyAsync(c.xyz_in.ptr, xyz, 24 * n,
-                           (flags & OCT_MEM_DEVICE) ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, c.stream));
     }
     c.n = n;
     if (!(flags & OCT_MEM_DEVICE)) CK(cudaStreamSynchronize(c.stream));

@@ -916,8 +916,7 @@ void reserve_point_arrays(Cloud& c, uint64_t n) {
     const struct {
         DevBuf* b;
         size_t bytes;
-    } part[] = {{&c.xyz_in, 24 * n},
-                {&c.keys, 8 * n},
+    } part[] = {{&c.keys, 8 * n},
                 {&c.keys_alt, 8 * n},
                 {&c.perm, 4 * n},
                 {&c.keys_hi, 4 * n},

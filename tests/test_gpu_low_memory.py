@@ -1,4 +1,6 @@
 """Calls that run out of device memory return an error, and the calls after them answer as before."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -6,21 +8,19 @@ from octrees_benchmark_b200.synth import lidar_tile
 
 pytestmark = pytest.mark.gpu
 
-LEFT = 3 << 30  # bytes of device memory a test leaves free
-
 
 @pytest.fixture
 def scarce():
-    """All of the device's memory but LEFT bytes, and the clouds' own pool, taken by the program."""
+    """All of the device's memory but so many bytes, and the clouds' own pool, taken by the program."""
     import torch
 
     from octrees_benchmark_b200 import capi
 
-    def take():
+    def take(left):
         capi.check(capi.lib().oct_trim_cloud_memory(0), None)
         torch.cuda.synchronize()
         torch.cuda.empty_cache()
-        held.append(torch.empty(torch.cuda.mem_get_info()[0] - LEFT, dtype=torch.uint8, device="cuda"))
+        held.append(torch.empty(torch.cuda.mem_get_info()[0] - left, dtype=torch.uint8, device="cuda"))
 
     held = []
     yield take
@@ -44,9 +44,32 @@ def test_result_chunks_that_do_not_fit(scarce):
     q = xyz[::10].copy()
     oc = LinearOctree(xyz, max_points_leaf=64)
     want = oc.radius_search(q, 2.0, "sphere"), oc.neighborsStruct(q, 2.0, "square"), oc.radius_hash(q, 2.0, "cube")
-    scarce()
+    scarce(3 << 30)
     out_of_memory(lambda: oc.radius_hash(q, 1e3, "sphere"))  # 4e9 results
     got = oc.radius_search(q, 2.0, "sphere"), oc.neighborsStruct(q, 2.0, "square"), oc.radius_hash(q, 2.0, "cube")
     for w, g in zip(want, got):
         assert all(np.array_equal(a, b) for a, b in zip(w, g))
+    oc.close()
+
+
+def test_points_that_do_not_fit_leave_the_cloud(scarce):
+    from octrees_benchmark_b200 import LinearOctree, capi
+
+    L = capi.lib()
+    xyz = lidar_tile(50_000, 70.0, seed=4)
+    q = xyz[::50].copy()
+    oc = LinearOctree(xyz, max_points_leaf=64)
+    want = [*oc.sorted_points(), *oc.radius_search(q, 2.0, "sphere"), *oc.knn(q, 10)]
+    scarce(1 << 30)
+    big = np.zeros((60_000_000, 3))  # 1.4 GB (never read)
+    out_of_memory(lambda: capi.check(L.oct_set_points(oc.handle, big.ctypes.data, len(big), 0), oc.handle))
+    got = [*oc.sorted_points(), *oc.radius_search(q, 2.0, "sphere"), *oc.knn(q, 10)]
+    assert all(np.array_equal(a, b) for a, b in zip(want, got))
+    # points that were given but not sorted are gone with the failure: an empty cloud, not a stale one
+    capi.check(L.oct_set_points(oc.handle, xyz.ctypes.data, len(xyz), 0), oc.handle)
+    out_of_memory(lambda: capi.check(L.oct_set_points(oc.handle, big.ctypes.data, len(big), 0), oc.handle))
+    info = capi.OctTreeInfo()
+    capi.check(L.oct_encode_sort(oc.handle, None, None, None, None, 0), oc.handle)
+    capi.check(L.oct_build(oc.handle, C.byref(info)), oc.handle)
+    assert info.n_points == 0
     oc.close()
