@@ -682,27 +682,32 @@ int oct_trim_cloud_memory(int device) {
     return OCT_OK;
 }
 
+// Before the arrays that searches read are written or made anew: until that has succeeded there is no sorted cloud
+// (an array that could not be grown is empty).
+static void forget_points(Cloud& c) {
+    c.n = 0;
+    c.sorted = false;
+    c.built = false;
+    c.rel_built = false;
+    c.crel_built = false;
+    c.node_capacity = 0;
+}
+
 int oct_set_points(oct_cloud h, const double* xyz, uint64_t n, uint32_t flags) {
     if (!h) return OCT_ERR_INVALID_ARG;
     Cloud& c = h->c;
     if (n && !xyz) return set_error(c, OCT_ERR_INVALID_ARG, "xyz is NULL");
     if (n >= 0xffffffffull) return set_error(c, OCT_ERR_INVALID_ARG, "more than 2^32 - 2 points");
     DeviceGuard g(c.device);
-    // the points as uploaded: no search reads them, so that a failure leaves a sorted (or built) cloud as it was;
-    // points that wait for their sort are gone
-    const uint64_t sorted_n = c.sorted ? c.n : 0;
+    // the points as uploaded: no search reads them, so that a failure leaves a sorted (or built) cloud as it was
     const bool more = c.xyz_in.bytes < 24 * n;
-    c.n = sorted_n;
+    if (!c.sorted) c.n = 0;  // points that wait for their sort go with their array
     CK(c.xyz_in.reserve(24 * (n ? n : 1)));
     if (n) {
         CK(cudaMemcpyAsync(c.xyz_in.ptr, xyz, 24 * n,
                            (flags & OCT_MEM_DEVICE) ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, c.stream));
     }
-    c.sorted = false;
-    c.built = false;
-    c.rel_built = false;
-    c.crel_built = false;
-    c.node_capacity = 0;
+    forget_points(c);
     if (more && c.split_sort) {
         // more points than before: new arrays, cut from one slab (the old slab goes with all that is cut from it)
         for (DevBuf* b : cloud_bufs(c))
@@ -802,7 +807,9 @@ int oct_set_sorted_points(oct_cloud h, const double* sorted_xyz, const uint64_t*
         if (!(box12[3 + a] >= 0.0)) return set_error(c, OCT_ERR_INVALID_ARG, "negative or NaN box radii");
     DeviceGuard g(c.device);
     const auto kind = dev ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
+    if (!c.sorted) c.n = 0;  // points that wait for their sort go with their array
     CK(c.xyz_in.reserve(24 * (n ? n : 1)));
+    forget_points(c);
     CK(c.xs.reserve(8 * (n ? n : 1)));
     CK(c.ys.reserve(8 * (n ? n : 1)));
     CK(c.zs.reserve(8 * (n ? n : 1)));
@@ -967,6 +974,7 @@ int oct_tree_import(oct_cloud h, const oct_tree_info* info, const double* box12,
         for (int a = 0; a < 3; ++a)
             if (!(radii[3 * l + a] >= 0.0)) return set_error(c, OCT_ERR_INVALID_ARG, "negative or NaN radii");
     DeviceGuard g(c.device);
+    forget_points(c);
     CK(c.xs.reserve(8 * (n ? n : 1)));
     CK(c.ys.reserve(8 * (n ? n : 1)));
     CK(c.zs.reserve(8 * (n ? n : 1)));

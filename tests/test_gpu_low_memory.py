@@ -73,3 +73,37 @@ def test_points_that_do_not_fit_leave_the_cloud(scarce):
     capi.check(L.oct_build(oc.handle, C.byref(info)), oc.handle)
     assert info.n_points == 0
     oc.close()
+
+
+def test_sorted_points_and_trees_that_do_not_fit(scarce):
+    """Their arrays replace the cloud's one by one: a failure among them leaves no cloud, and says so."""
+    from octrees_benchmark_b200 import LinearOctree, capi
+
+    L = capi.lib()
+    n = 16_000_000
+    rng = np.random.default_rng(1)
+    big = LinearOctree(rng.random((n, 3)), max_points_leaf=4096)
+    ck = big.checkpoint()
+    big.close()
+    xyz = lidar_tile(50_000, 70.0, seed=4)
+    q = xyz[::50].copy()
+    clouds = [LinearOctree(xyz, encoder=int(ck["encoder"]), max_points_leaf=4096) for _ in range(2)]
+    want = clouds[0].knn(q, 10)
+    kinds = dict(box="f8", keys="u8", perm="u4", sorted_xyz="f8", offsets="u4", ranges="u8", centers="f8", radii="f8",
+                 half="f8")
+    arrays = {k: np.ascontiguousarray(ck[k], t) for k, t in kinds.items()}
+    ptr = {k: a.ctypes.data for k, a in arrays.items()}
+    info = capi.OctTreeInfo(*(int(v) for v in ck["info"]))
+    scarce(512 << 20)  # 32 bytes a point with the first, 36 with the second
+    calls = (lambda h: L.oct_set_sorted_points(h, ptr["sorted_xyz"], ptr["keys"], n, ptr["box"], 0),
+             lambda h: L.oct_tree_import(h, C.byref(info), *ptr.values(), 0))
+    for oc, call in zip(clouds, calls):
+        out_of_memory(lambda: capi.check(call(oc.handle), oc.handle))
+        with pytest.raises(capi.OctError) as e:
+            oc.knn(q, 10)
+        assert e.value.status == capi.OCT_ERR_STATE
+        capi.check(L.oct_set_points(oc.handle, xyz.ctypes.data, len(xyz), 0), oc.handle)
+        capi.check(L.oct_encode_sort(oc.handle, None, None, None, None, 0), oc.handle)
+        capi.check(L.oct_build(oc.handle, None), oc.handle)
+        assert all(np.array_equal(a, b) for a, b in zip(want, oc.knn(q, 10)))
+        oc.close()
