@@ -146,6 +146,11 @@ int oct_set_radius_group(oct_cloud cloud, int lanes);
  *               k best pairs.
  *  reserved[0]  1: packet radius searches count, then fill at the scanned
  *               offsets; 0 (default): one pass into per-query result chunks.
+ *               The chunks take at least 792 bytes a centre (264 for every 64
+ *               results, and three such chunks a centre to begin with) and
+ *               stay the cloud's for its next search.  oct_struct_search and
+ *               oct_approx_search take none when they are only asked for
+ *               sizes, and count and fill where there is no memory for them.
  *  reserved[1]  kNN (packet path) provisional threshold: < 0 = off (the
  *               collecting search then starts every query from the points
  *               next to it); otherwise, for knn_packet 0 and k <= 64, in

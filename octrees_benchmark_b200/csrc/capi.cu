@@ -163,8 +163,10 @@ ChunkArgs cloud_chunks(const Cloud& c) { return chunk_args(c.ck_pool, c.ck_rec, 
 // compacted into the CSR output.  A pool that turned out too small leaves the
 // counts exact: it is sized from the total and the traversal runs once more.
 // d_points (neighborsStruct ranges): every query's points; else NULL, and neighborsStruct searches its index set.
+// no_room (may be NULL: an error then): set when there is no memory for the pool, which is given back.
 int radius_chunks(Cloud& c, int kernel, int algo, const double* dq, uint64_t nq, const double* dr, double radius,
-                  unsigned long long* doffs, uint64_t* total, unsigned long long* d_points = nullptr) {
+                  unsigned long long* doffs, uint64_t* total, unsigned long long* d_points = nullptr,
+                  bool* no_room = nullptr) {
     const uint64_t per = d_points ? 2 : 1;  // chunk entries of a result
     const int pass_algo = (algo == OCT_NEIGHBORS_STRUCT && !d_points) ? OCT_NEIGHBORS_PRUNE : algo;  // same index set
     unsigned long long* dc = c.q_counts.as<unsigned long long>();
@@ -180,9 +182,18 @@ int radius_chunks(Cloud& c, int kernel, int algo, const double* dq, uint64_t nq,
     for (int attempt = 0; attempt < 2; ++attempt) {
         // pool: every query's partial last chunk plus the results (a guess of 128 per query at first)
         const uint64_t want = attempt == 0 ? 3 * nq + 1024 : per * tot / kResultChunk + nq + 1024;
-        if (want > 0xfffffff0ull) return set_error(c, OCT_ERR_INVALID_ARG, "too many results for one call");
-        CK(c.ck_pool.reserve(4ull * kResultChunk * want));
-        CK(c.ck_rec.reserve(sizeof(uint2) * want));
+        const bool too_many = want > 0xfffffff0ull;
+        if (too_many && !no_room) return set_error(c, OCT_ERR_INVALID_ARG, "too many results for one call");
+        cudaError_t e = too_many ? cudaErrorMemoryAllocation : c.ck_pool.reserve(4ull * kResultChunk * want);
+        if (e == cudaSuccess) e = c.ck_rec.reserve(sizeof(uint2) * want);
+        if (e == cudaErrorMemoryAllocation && no_room) {
+            cudaGetLastError();
+            c.ck_pool.release();
+            c.ck_rec.release();
+            *no_room = true;
+            return OCT_OK;
+        }
+        CK(e);
         const ChunkArgs ck = cloud_chunks(c);
         CK(cudaMemsetAsync(ck.ctr, 0, 4, c.stream));
         CK(launch_radius_packet(c, kernel, pass_algo, 2, fp32_on_radius(c.fp32_filter), dq, nq, dr, radius, order,
@@ -1193,11 +1204,17 @@ static int ranges_search(oct_cloud h, int kernel, const double* centers, uint64_
     }
     const uint32_t* order = nullptr;
     uint64_t tot;
-    const bool one_pass = c.packet && !c.two_pass && nq;
+    // one pass where there is somewhere to put the ranges and memory for their chunks; else the ranges are counted,
+    // which needs neither, and filled in by a second pass
+    bool one_pass = c.packet && !c.two_pass && nq && pairs && pair_capacity;
     if (one_pass) {
-        if ((st = radius_chunks(c, kernel, OCT_NEIGHBORS_STRUCT, dq, nq, dr, radius, doffs, &tot, dpoints)) != OCT_OK)
+        bool no_room = false;
+        if ((st = radius_chunks(c, kernel, OCT_NEIGHBORS_STRUCT, dq, nq, dr, radius, doffs, &tot, dpoints,
+                                &no_room)) != OCT_OK)
             return st;
-    } else {
+        one_pass = !no_room;
+    }
+    if (!one_pass) {
         CK(radius_pass(c, kernel, OCT_NEIGHBORS_STRUCT, false, dq, nq, dr, radius, dranges, dpoints, nullptr, nullptr,
                        0, &order));
         CK(launch_scan_u64(c, dranges, doffs, nq));

@@ -107,3 +107,29 @@ def test_sorted_points_and_trees_that_do_not_fit(scarce):
         capi.check(L.oct_build(oc.handle, None), oc.handle)
         assert all(np.array_equal(a, b) for a, b in zip(want, oc.knn(q, 10)))
         oc.close()
+
+
+def test_ranges_without_room_for_result_chunks(scarce):
+    from octrees_benchmark_b200 import LinearOctree, capi
+
+    import torch
+
+    L = capi.lib()
+    xyz = lidar_tile(100_000, 100.0, seed=4)
+    q = np.tile(xyz[:1_000], (2_000, 1))  # 2M centres: 1.6 GB of chunks
+    oc = LinearOctree(xyz, max_points_leaf=64)
+    oc.set_search_config(two_pass=True)
+    want = oc.neighborsStruct(q, 0.4), oc.neighborsApprox(q, 0.4, 4, True)
+    oc.set_search_config()
+    scarce(1 << 30)
+    for w, g in zip(want, (oc.neighborsStruct(q, 0.4), oc.neighborsApprox(q, 0.4, 4, True))):
+        assert all(np.array_equal(a, b) for a, b in zip(w, g))
+    # a call that asks for sizes only takes no chunks (158 MB for these centres)
+    few = LinearOctree(xyz, max_points_leaf=64)
+    few.radius_count(q[:200_000], 0.4)
+    total, free = C.c_uint64(0), torch.cuda.mem_get_info()[0]
+    st = L.oct_struct_search(few.handle, 2, q.ctypes.data, 200_000, None, 0.4, None, None, 0, C.byref(total), None, 0)
+    assert st == capi.OCT_ERR_CAPACITY and total.value == want[0][0][200_000]
+    assert free - torch.cuda.mem_get_info()[0] < (64 << 20)
+    few.close()
+    oc.close()
