@@ -723,7 +723,8 @@ __global__ void __launch_bounds__(kKnnThreads, 8) k_knn_reg(KnnTableArgs a) {
 // each; a pair's rank is its bin's start plus the pairs of the bin that precede
 // it by (distance, index), and the pair is written to that output slot.  (When a
 // bin holds more than kBinMany pairs the bins are taken again over the logarithm
-// of the distances, so far outliers do not press the others into one bin.)  A
+// of the distances, so far outliers do not press the others into one bin; if one
+// still does, the pairs are sorted.)  A
 // buffer that runs full keeps the bins that hold its k smallest pairs and the
 // threshold drops to the largest pair kept.
 //
@@ -818,6 +819,7 @@ struct BinMap {
     float scale;
     uint32_t lo;
     int shift;
+    bool crowded;  // a bin holds more than kBinMany pairs all the same
     __device__ __forceinline__ uint32_t bin(double d, uint32_t bins) const {
         if (shift < 0) {
             const int b = (int)((float)d * scale);  // NaN (inf * 0) converts to 0
@@ -837,6 +839,7 @@ __device__ __forceinline__ BinMap knn_bin_pairs(const double* d, uint32_t n, dou
     m.scale = top > 0.0 && top < (double)INFINITY ? (float)bins / (float)top : 0.0f;
     m.lo = 0;
     m.shift = -1;
+    m.crowded = false;
     uint4* h4 = reinterpret_cast<uint4*>(hist);  // 128 bins a step, four on a lane
 #pragma unroll 1
     for (int tries = 0;; ++tries) {
@@ -868,8 +871,9 @@ __device__ __forceinline__ BinMap knn_bin_pairs(const double* d, uint32_t n, dou
             c.x = ex;
             h4[b / 4 + lane] = c;
         }
-        if (tries == 0 && __any_sync(0xffffffffu, most > kBinMany)) {
-            // over the logarithm of the distances instead
+        m.crowded = __any_sync(0xffffffffu, most > kBinMany);
+        if (tries == 0 && m.crowded) {
+            // over the logarithm of the distances instead, unless they are all one (to FP32)
             uint32_t lo = 0xffffffffu, hi = 0;
 #pragma unroll 1
             for (uint32_t e = lane; e < n; e += 32) {
@@ -877,14 +881,61 @@ __device__ __forceinline__ BinMap knn_bin_pairs(const double* d, uint32_t n, dou
                 if (v) lo = v < lo ? v : lo;
                 hi = v > hi ? v : hi;
             }
-            m.lo = __reduce_min_sync(0xffffffffu, lo);
+            lo = __reduce_min_sync(0xffffffffu, lo);
             hi = __reduce_max_sync(0xffffffffu, hi);
-            m.shift = hi > m.lo ? 32 - __clz((hi - m.lo) / bins) : 0;  // (hi - lo) >> shift < bins
-            continue;
+            if (hi > lo) {
+                m.lo = lo;
+                m.shift = 32 - __clz((hi - lo) / bins);  // (hi - lo) >> shift < bins
+                continue;
+            }
         }
         __syncwarp();
         return m;
     }
+}
+
+// n pairs into ascending order by (distance, index), one warp: Batcher's odd-even merge sort, which takes any n.
+// For distances that crowd into one bin (points that are given many times), where ranking each pair against the
+// others of its bin is quadratic: 20k queries of k = 1000 on points given 1500 times 85.5 -> 3.1 ms, k = 250 on
+// points given 300 times 2.41 -> 0.63; other clouds take the time they took.
+__device__ __noinline__ void knn_sort_pairs(double* d, uint32_t* ix, uint32_t n) {
+    const uint32_t lane = threadIdx.x & 31;
+    __syncwarp();
+#pragma unroll 1
+    for (uint32_t p = 1; p < n; p <<= 1) {
+#pragma unroll 1
+        for (uint32_t k = p; k > 0; k >>= 1) {
+            const uint32_t off = k & (p - 1);  // (k mod p)
+#pragma unroll 1
+            for (uint32_t t = lane;; t += 32) {
+                const uint32_t x = off + (((t & ~(k - 1)) << 1) | (t & (k - 1))), y = x + k;
+                if (y >= n) break;
+                if (((x ^ y) & ~(2 * p - 1)) == 0) {  // of the same run of 2 p
+                    const double a = d[x], b = d[y];
+                    const uint32_t ia = ix[x], ib = ix[y];
+                    if (pair_less(b, ib, a, ia)) {
+                        d[x] = b;
+                        d[y] = a;
+                        ix[x] = ib;
+                        ix[y] = ia;
+                    }
+                }
+            }
+            __syncwarp();
+        }
+    }
+}
+
+// The K best of n pairs by that sort, to their output slots; returns the K-th distance (< 0: none).
+__device__ __noinline__ double knn_write_sorted(double* d, uint32_t* ix, uint32_t n, uint32_t K, uint32_t* idx,
+                                                double* d2) {
+    knn_sort_pairs(d, ix, n);
+#pragma unroll 1
+    for (uint32_t t = threadIdx.x & 31; t < K; t += 32) {
+        idx[t] = t < n ? ix[t] : 0xffffffffu;
+        d2[t] = t < n ? d[t] : (double)INFINITY;
+    }
+    return n >= K ? d[K - 1] : -1.0;
 }
 
 // The K-th smallest of the n squared distances at d as FP32 bits: radix selection, seven bits a pass.
@@ -1514,6 +1565,10 @@ __global__ void __launch_bounds__(kGrpThreads, 7) k_knn_group(KnnGroupArgs a) {
             }
             // rank the pairs and write the K best
             const BinMap bm = knn_bin_pairs(bd, n, thr, hist, bins);
+            if (bm.crowded) {
+                kth = knn_write_sorted(bd, bi, n, K, a.idx + o, a.d2 + o);
+                break;
+            }
 #pragma unroll 1
             for (uint32_t e = lane; e < n; e += 32) ord[atomicAdd(&hist[bm.bin(bd[e], bins)], 1u)] = (uint16_t)e;
             __syncwarp();
