@@ -151,8 +151,8 @@ constexpr double kKnnEstimate = 1.2;
 // ones start from the k-th distances of those before them).  10M-point tile, 500k
 // queries of k = 50: runs of 8 take 2.74 ms, of 16 2.87, of 32 3.23 (L2 and L1 hits).
 constexpr uint32_t kKnnGroupChunk = 4;
-// its heads: every kKnnHeadStride-th query is searched first, from its own node;
-// the others start from a neighbouring query's k-th distance
+// its heads: every kKnnHeadStride-th query (of k = 1 every fourth of those) is searched first,
+// from its own node; the others start from a neighbouring query's k-th distance
 constexpr uint32_t kKnnHeadStride = 16;
 struct Cloud {
     oct_params params{};

@@ -732,7 +732,7 @@ __global__ void __launch_bounds__(kKnnThreads, 8) k_knn_reg(KnnTableArgs a) {
 // after the first of a run starts at kGrpSeed x the largest k-th distance of those
 // before it, each faded by kSeedFade a query (the k-th distance varies slowly along the curve;
 // longer runs widen the stretch of the curve that the warps work on at once,
-// which costs L2 hits).  Every kKnnHeadStride-th query is a head: heads are handed
+// which costs L2 hits).  Every kKnnHeadStride-th query (of k = 1 every 64th) is a head: heads are handed
 // out first; the first query of a run (and each query handed out alone at the
 // end) starts from the nearest head of its request that has finished.  A query
 // without a seed, and a query that found fewer than k pairs within its seeded
@@ -756,8 +756,7 @@ __global__ void __launch_bounds__(kKnnThreads, 8) k_knn_reg(KnnTableArgs a) {
 // sorted lists for k <= 64, bitonic merges in shared memory above) and now:
 //   10M-point tile: 500k, k = 50 3700 -> 2787 us; 50k, k = 50 1069 -> 430; 5k, k = 50
 //   497 -> 195; 200, k = 50 345 -> 105; 5M: 30k, k = 250 2300 -> 710; 3k, k = 900
-//   2400 -> 610.  Only k = 1 in batches of 200k and more at cloud points is not
-//   faster (10M tile 500k 848 -> 863, 1M points at 20 a m^2 716 -> 789).
+//   2400 -> 610.  k = 1: see kHeadBitsOne.
 // ---------------------------------------------------------------------------
 
 constexpr int kGrpWarps = 4;
@@ -768,7 +767,13 @@ constexpr int kScanBlocks = 2;        // 32-point blocks in flight (k = 50, 500k
 constexpr double kGrpSeed = 1.5;      // provisional threshold / largest recent k-th distance of the run
 constexpr double kSeedFade = 0.95;    // what an earlier k-th distance counts for a query later (0.7: +8 % at k = 10)
 constexpr uint32_t kBinMany = 48;
-static_assert(kKnnHeadStride >= 2, "the groups between heads are numbered modulo kKnnHeadStride - 1");
+// Heads, as a power of two: every 16th query, of k = 1 every 64th.  A head starts cold, which for k = 1 costs several
+// times what the others do, and the head's distance is as good a start from further away (0 for centres at cloud
+// points).  200k, 500k and 1M centres at cloud points, every 16th -> every 64th, in us: 10M-point tile 429, 889,
+// 1655 -> 398, 798, 1476 (sorted lists of four queries a warp 442, 841, 1567), 1M points at 20 a m^2 363, 787, 1504
+// -> 338, 718, 1358 (357, 715, 1358); beside the points 749, 1660, 3096 -> 737, 1575, 2983.
+constexpr uint32_t kHeadBits = 4, kHeadBitsOne = 6;
+static_assert(kKnnHeadStride == 1u << kHeadBits, "every kKnnHeadStride-th query is a head");
 
 struct KnnGroupArgs {
     SearchReq single;                 // one request (grp == null)
@@ -1194,9 +1199,10 @@ __global__ void __launch_bounds__(kGrpThreads, 7) k_knn_group(KnnGroupArgs a) {
     }
     // heads (every S-th query) go out first, one at a time; the others are slots:
     // slot s is the s-th query that is not a head (every query without heads)
-    constexpr uint32_t S = kKnnHeadStride;
+    const bool far = (MULTI ? a.grp->kmax : a.single.k) == 1;
+    const uint32_t sbits = far ? kHeadBitsOne : kHeadBits, S = 1u << sbits;
     const bool heads = a.heads != 0;
-    const uint32_t n_heads = heads ? (packets + S - 1) / S : 0;
+    const uint32_t n_heads = heads ? (packets + S - 1) >> sbits : 0;
     const uint32_t slots = packets - n_heads;
     bool heads_left = n_heads != 0;
     // slots [0, p_chunked) go out in chunks, the rest one at a time
@@ -1247,7 +1253,7 @@ __global__ void __launch_bounds__(kGrpThreads, 7) k_knn_group(KnnGroupArgs a) {
             }
             if (slot >= slots) break;
         }
-        const uint32_t packet = head ? slot * S : !heads ? slot : slot + slot / (S - 1) + 1;
+        const uint32_t packet = head ? slot << sbits : !heads ? slot : slot + (far ? slot / ((1u << kHeadBitsOne) - 1) : slot / ((1u << kHeadBits) - 1)) + 1;
         uint32_t ri = 0;
         if (MULTI) {  // the request of this query (packet_begin ascending over the table)
             uint32_t lo = 0, hi = nreq;
@@ -1279,7 +1285,7 @@ __global__ void __launch_bounds__(kGrpThreads, 7) k_knn_group(KnnGroupArgs a) {
         if (seed < 0.0 && heads && !head) {
             const uint32_t pb = (uint32_t)KRQ(packet_begin);
             const uint32_t pe = pb + (uint32_t)(KRQ(q_end) - KRQ(q_begin));
-            const uint32_t hlo = packet / S, hhi = hlo + 1;  // heads hlo S < packet < hhi S
+            const uint32_t hlo = packet >> sbits, hhi = hlo + 1;  // heads hlo S < packet < hhi S
             const bool lo_ok = hlo * S >= pb, hi_ok = hhi < n_heads && hhi * S < pe;
             const bool use_hi = hi_ok && (!lo_ok || hhi * S - packet < packet - hlo * S);
             // a head not finished yet reads NaN: no seed (nothing waits for it)
@@ -1294,7 +1300,7 @@ __global__ void __launch_bounds__(kGrpThreads, 7) k_knn_group(KnnGroupArgs a) {
         const uint64_t ql = q - q_begin;
         const double p[3] = {__shfl_sync(0xffffffffu, ahead_c, 0), __shfl_sync(0xffffffffu, ahead_c, 1),
                              __shfl_sync(0xffffffffu, ahead_c, 2)};
-        ahead_pos = next < chunk_end && pos + 1 < (uint32_t)KRQ(q_end) && (!heads || (packet + 1) % S) ? pos + 1 : 0xffffffffu;
+        ahead_pos = next < chunk_end && pos + 1 < (uint32_t)KRQ(q_end) && (!heads || ((packet + 1) & (S - 1))) ? pos + 1 : 0xffffffffu;
         if (ahead_pos != 0xffffffffu) ahead_q = a.order ? a.order[ahead_pos] : ahead_pos;
         double thr = cold ? (double)INFINITY : kGrpSeed * seed;
         // FP32 filter: query - box centre in FP32, the FP32 threshold, and A + B (box radius +
