@@ -1345,14 +1345,17 @@ __global__ void __launch_bounds__(kGrpThreads, 7) k_knn_group(KnnGroupArgs a) {
                 } else if (path_len) {
                     // the deepest node of the path that holds the whole ball, by margins above what a squared distance
                     // loses below the FP64 range (3 x 2^-1075) and above the rounding of coordinates, keys and node
-                    // boxes (to the size of the cloud's box): every node outside it is beyond the threshold
-                    const double r = sqrt(thr) * 1.000001 + 4.0e-162;
+                    // boxes (to the size of the cloud's box): every node outside it is beyond the threshold.  Squares
+                    // are compared (an FP64 root: +0.4 % at k = 50); no square is above an infinite threshold
+                    const double r2 = thr * 1.000002 + 2.0e-323;
                     bool holds = (uint32_t)lane < path_len;
                     if (holds && lane) {
 #pragma unroll
                         for (int t = 0; t < 3; ++t) {
-                            const double h = s_radii[lane][t], c = pc[lane][t];
-                            holds = holds && fabs(p[t] - c) + r + 1.0e-12 * (fabs(p[t]) + fabs(c) + s_radii[0][t]) <= h;
+                            const double c = pc[lane][t];
+                            const double in = s_radii[lane][t] - fabs(p[t] - c) -
+                                              1.0e-12 * (fabs(p[t]) + fabs(c) + s_radii[0][t]);
+                            holds = holds && in > 0.0 && in * in > r2;
                         }
                     }
                     path_len = 32 - __clz(__ballot_sync(0xffffffffu, holds));
