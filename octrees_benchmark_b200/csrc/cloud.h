@@ -316,8 +316,8 @@ inline ChunkArgs chunk_args(const DevBuf& pool, const DevBuf& rec, const DevBuf&
                      (uint32_t)(cap < 0xfffffff0ull ? cap : 0xfffffff0ull)};
 }
 
-// Queries per packet (1 to 32) of a packet radius launch over nq queries.
-uint32_t packet_width(uint64_t nq, int device);
+// Queries per packet (1 to `widest`: 16, or 32 where FP32 searches count) of a packet radius launch over nq queries.
+uint32_t packet_width(uint64_t nq, int device, uint32_t widest = 16);
 // Packet radius search.  Either one request (`single`, host copy, `packets`
 // packets of `width` queries) or the group of a batch (`d_grp`, sizes read on the device); with
 // both, every request of the group is on the cloud `single->cv` (kernel

@@ -588,6 +588,15 @@ __global__ void __launch_bounds__(kPkThreads) k_radius_packet(PacketArgs a) {
             }
             // first: the leaves' points as one run; leaf l holds [first, first + length) of it
             const uint32_t len = rg.y - rg.x;
+            if (MODE == 0 && !kRanges && __any_sync(0xffffffffu, li != 0)) {
+                // counted: a leaf's points for all the queries that hold it at once (one query at a time: FP32 counts
+                // of 100k cubes of 6 m on a dense tile 2524 us, so 2345; FP64 1424, 1259)
+                for (int l = 0; l < g; ++l) {
+                    const uint32_t mask = __shfl_sync(0xffffffffu, li, l), n = __shfl_sync(0xffffffffu, len, l);
+                    if (mask & lbit) cnt += n;
+                }
+                li = 0;
+            }
             uint32_t end = len;
 #pragma unroll
             for (int off = 1; off < kGroup; off <<= 1) {
@@ -1046,9 +1055,11 @@ CloudView cloud_view(const Cloud& c) {
 //   2k   105 / 125 / 159 / 262 / 435 / 849           100k 968 / 688 / 588 / 588 / 664 / 772
 //   8k   176 / 198 / 265 / 385 / 626 / 1063          500k 4476 / 2618 / 1959 / 1735 / 1638 / 1720
 // (with circles of 560 points on a dense tile 100k: 2256 / 1560 / 1238 / 1159 / 1333 / 1937).
-uint32_t packet_width(uint64_t nq, int device) {
+// FP32 counts take 32 as well (widest): a leaf's contexts are made by all lanes at once, and there are no results
+// to append: 500k squares of 3 m 5029 us at 16, 4795 at 32, spheres of 0.5 m 531, 507; FP32 lists are faster at 16.
+uint32_t packet_width(uint64_t nq, int device, uint32_t widest) {
     const uint64_t packets = (uint64_t)sm_count_p(device) * kPkWarps * 8 * 2;
-    uint32_t w = 16;
+    uint32_t w = widest;
     while (w > 1 && (nq + w - 1) / w < packets) w >>= 1;
     return w;
 }
@@ -1144,7 +1155,7 @@ cudaError_t launch_radius_packet(Cloud& c, int kernel, int algo, int mode, bool 
     r.approx_cut = c.approx_cut;
     r.approx_upper = (uint32_t)c.approx_upper;
     KernelClock clk(c, 0);
-    const uint32_t w = packet_width(nq, c.device);
+    const uint32_t w = packet_width(nq, c.device, fp32 && mode == 0 ? 32 : 16);
     e = launch_radius_table(c.device, c.stream, kernel, algo, mode, fp32, nullptr, &r, (nq + w - 1) / w, w, d_order,
                             d_counts, d_counts2, d_offsets, d_out, out_capacity, c.packet_ctr.as<uint32_t>(),
                             c.stats.as<unsigned long long>(), c.d_err.as<uint32_t>(), 0, chunks);
