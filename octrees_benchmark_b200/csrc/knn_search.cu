@@ -1063,20 +1063,22 @@ struct KnnNear {
 __device__ __noinline__ KnnNear knn_near_ranges(const uint32_t* offsets, const uint2* ranges, const double* centers,
                                                 const double (*radii)[3], double x, double y, double z, uint32_t K,
                                                 uint32_t bucket, KnnNear st, uint32_t* fcs, uint8_t* depths,
-                                                uint16_t* keys, uint2* list) {
+                                                float* keys, uint2* list) {
     const int lane = threadIdx.x & 31;
     const double p[3] = {x, y, z};
     st.m = 0;
 #pragma unroll 1
     while (st.open > 0 && st.taken < knn_near_points(K) && st.m < kGrpRanges) {
-        uint32_t key = 0xffffffffu;
+        uint32_t key = 0xffffffffu;  // (bounds are not negative: their bits ascend as they do)
         int at = 0;
 #pragma unroll 1
-        for (int t = lane; t < st.open; t += 32)
-            if (keys[t] < key) {
-                key = keys[t];
+        for (int t = lane; t < st.open; t += 32) {
+            const uint32_t kt = __float_as_uint(keys[t]);
+            if (kt < key) {
+                key = kt;
                 at = t;
             }
+        }
         const uint32_t least = __reduce_min_sync(0xffffffffu, key);
         at = __shfl_sync(0xffffffffu, at, __ffs(__ballot_sync(0xffffffffu, key == least)) - 1);
         const uint32_t fc = fcs[at], depth = depths[at];
@@ -1106,31 +1108,38 @@ __device__ __noinline__ KnnNear knn_near_ranges(const uint32_t* offsets, const u
             const int to = st.open + __popc(sm & lanemask_lt());
             fcs[to] = whole ? child : cfc;
             depths[to] = whole ? (uint8_t)255 : (uint8_t)(depth + 1);
-            keys[to] = (uint16_t)(__float_as_uint(lb) >> 16);
+            keys[to] = lb;
         }
         st.open += __popc(sm);
         __syncwarp();
         if (st.open + 7 > kGrpStack) {
-            // no room for the next node's children: the far entries go (any K points bound the K-th distance)
-            uint32_t most = 0;
+            // no room for the next node's children: the far half of the bounds' span goes, and again until half the
+            // entries are left (any K points bound the K-th distance; halves of the span and not of the largest
+            // bound, as the bounds of a query far from the cloud differ by little)
+            uint32_t least_left = 0xffffffffu, most = 0;
 #pragma unroll 1
-            for (int t = lane; t < st.open; t += 32) most = max(most, (uint32_t)keys[t]);
-            float limit = __uint_as_float(__reduce_max_sync(0xffffffffu, most) << 16);
+            for (int t = lane; t < st.open; t += 32) {
+                least_left = min(least_left, __float_as_uint(keys[t]));
+                most = max(most, __float_as_uint(keys[t]));
+            }
+            const float low = __uint_as_float(__reduce_min_sync(0xffffffffu, least_left));
+            float span = __uint_as_float(__reduce_max_sync(0xffffffffu, most)) - low;
 #pragma unroll 1
-            for (int tries = 0; st.open > kGrpStack / 2 && tries < 64; ++tries) {
-                limit *= 0.5f;
+            for (int tries = 0; st.open > kGrpStack / 2 && span > 0.0f && tries < 24; ++tries) {
+                span *= 0.5f;
                 int left = 0;
 #pragma unroll 1
                 for (int t = 0; t < st.open; t += 32) {
                     uint32_t f = 0;
-                    uint16_t k = 0xffff;
+                    float k = 0.0f;
                     uint8_t d = 0;
-                    if (t + lane < st.open) {
+                    const bool in = t + lane < st.open;
+                    if (in) {
                         f = fcs[t + lane];
                         d = depths[t + lane];
                         k = keys[t + lane];
                     }
-                    const bool stay = __uint_as_float((uint32_t)k << 16) <= limit;  // (0xffff is no number)
+                    const bool stay = in && k - low <= span;
                     const uint32_t sb = __ballot_sync(0xffffffffu, stay);
                     if (stay) {  // at or below the lanes' own positions
                         const int to = left + __popc(sb & lanemask_lt());
@@ -1143,7 +1152,7 @@ __device__ __noinline__ KnnNear knn_near_ranges(const uint32_t* offsets, const u
                 }
                 st.open = left;
             }
-            if (st.open + 7 > kGrpStack) st.open = kGrpStack - 8;
+            if (st.open > kGrpStack / 2) st.open = kGrpStack / 2;  // (equal bounds)
         }
     }
     return st;
@@ -1155,7 +1164,7 @@ __global__ void __launch_bounds__(kGrpThreads, 7) k_knn_group(KnnGroupArgs a) {
     __shared__ uint32_t s_n[kGrpWarps];               // pairs in the buffer
     __shared__ uint32_t st_fc[kGrpWarps][kGrpStack];  // first child of a node
     __shared__ uint8_t st_d[kGrpWarps][kGrpStack];    // its children's depth
-    __shared__ uint16_t st_key[kGrpWarps][kGrpStack];  // its bound (upper half of the FP32 bits), for cold queries
+    __shared__ float st_key[kGrpWarps][kGrpStack];    // its bound in FP32, for cold queries
     __shared__ uint2 s_rg[kGrpWarps][kGrpRanges];
     // the nodes that the warp's last walks passed one by one from the root (centre, first child), by
     // depth: a walk starts at the deepest that holds its whole ball
@@ -1181,7 +1190,7 @@ __global__ void __launch_bounds__(kGrpThreads, 7) k_knn_group(KnnGroupArgs a) {
     uint16_t* ord = reinterpret_cast<uint16_t*>(hist + bins);
     uint32_t* sf = st_fc[warp];
     uint8_t* sdp = st_d[warp];
-    uint16_t* sk = st_key[warp];
+    float* sk = st_key[warp];
     uint2* list = s_rg[warp];
     uint32_t* np = &s_n[warp];
     unsigned long long f_tests = 0, f_64 = 0, f_band = 0;
@@ -1338,7 +1347,7 @@ __global__ void __launch_bounds__(kGrpThreads, 7) k_knn_group(KnnGroupArgs a) {
                         if (lane == 0) {
                             sf[0] = fc0;
                             sdp[0] = 1;
-                            sk[0] = 0;
+                            sk[0] = 0.0f;
                         }
                         sp = 1;
                     }
