@@ -766,6 +766,8 @@ constexpr uint32_t kGrpRanges = 64;   // ranges gathered before they are tested
 constexpr int kScanBlocks = 2;        // 32-point blocks in flight (k = 50, 500k: 1 3.02 ms, 2 2.85, 4 3.22)
 constexpr double kGrpSeed = 1.5;      // provisional threshold / largest recent k-th distance of the run
 constexpr double kSeedFade = 0.95;    // what an earlier k-th distance counts for a query later (0.7: +8 % at k = 10)
+// In the place of the slot a query seeds from: a head seeds no slot of the run, a centre outside the box none at all.
+constexpr uint32_t kHeadSeed = 0xfffffffeu, kNoSeed = 0xfffffffdu;
 constexpr uint32_t kBinMany = 48;
 // Heads, as a power of two: every 16th query, of k = 1 every 64th.  A head starts cold, which for k = 1 costs several
 // times what the others do, and the head's distance is as good a start from further away (0 for centres at cloud
@@ -1182,6 +1184,8 @@ __global__ void __launch_bounds__(kGrpThreads, 7) k_knn_group(KnnGroupArgs a) {
         for (int t = threadIdx.x; t < (kMaxDepth + 1) * 3; t += kGrpThreads) (&s_rad[0][0][0])[t] = gr[t];
         __syncthreads();
     }
+    if (MULTI != 1 && lane < 3) s_pc[warp][0][lane] = a.single.cv.centers[lane];
+    __syncwarp();
     const uint32_t cap = a.cap, bins = a.bins;
     unsigned char* mine = smem + (size_t)warp * knn_group_bytes(cap, bins);
     double* bd = reinterpret_cast<double*>(mine);
@@ -1280,6 +1284,7 @@ __global__ void __launch_bounds__(kGrpThreads, 7) k_knn_group(KnnGroupArgs a) {
 #pragma unroll 1
             for (int t = lane; t < (kMaxDepth + 1) * 3; t += 32) (&s_radii[0][0])[t] = gr[t];
             if (lane == 0) s_view[warp] = reqs[ri].cv;
+            if (lane < 3) pc[0][lane] = reqs[ri].cv.centers[lane];
             cur_cloud = reqs[ri].cloud_id;
             path_len = 0;
             __syncwarp();
@@ -1311,6 +1316,13 @@ __global__ void __launch_bounds__(kGrpThreads, 7) k_knn_group(KnnGroupArgs a) {
                              __shfl_sync(0xffffffffu, ahead_c, 2)};
         ahead_pos = next < chunk_end && pos + 1 < (uint32_t)KRQ(q_end) && (!heads || ((packet + 1) & (S - 1))) ? pos + 1 : 0xffffffffu;
         if (ahead_pos != 0xffffffffu) ahead_q = a.order ? a.order[ahead_pos] : ahead_pos;
+        // A centre outside the cloud's box (by more than rounding) starts cold and seeds no other: its k-th distance is
+        // decided by how far it is from the cloud, and a ball a little larger holds much of the cloud.  20k centres
+        // around a cube of 500k points, k = 10: 570 -> 220 us, beside a plane 1056 -> 274; centres inside keep their time
+        const bool outside = __any_sync(
+            0xffffffffu, lane < 3 && fabs(ahead_c - pc[0][lane % 3]) > 1.000001 * s_radii[0][lane % 3]);
+        cold = cold || outside;
+        seed_slot = outside ? kNoSeed : head ? kHeadSeed : slot;
         double thr = cold ? (double)INFINITY : kGrpSeed * seed;
         // FP32 filter: query - box centre in FP32, the FP32 threshold, and A + B (box radius +
         // |query - centre|_inf) for new thresholds
@@ -1625,9 +1637,8 @@ __global__ void __launch_bounds__(kGrpThreads, 7) k_knn_group(KnnGroupArgs a) {
         }
         if (!ok) ahead_pos = 0xffffffffu;  // not read
         run_kth = fmax(kth, kSeedFade * run_kth);
-        seed_slot = head ? 0xfffffffeu : slot;  // a head seeds no slot of the run
         seed_ri = ri;
-        if (head && lane == 0) __stcg(&a.head_kth[slot], kth);
+        if (seed_slot == kHeadSeed && lane == 0) __stcg(&a.head_kth[slot], kth);
         __syncwarp();
     }
     if constexpr (F32) {

@@ -62,3 +62,51 @@ def test_time_of_long_lists_far_away(cube):
     beside = knn_ms(oc, at + [150.0, 0.0, 0.0], 1000)
     around = knn_ms(oc, at + 200.0 * rng.uniform(-1.0, 1.0, at.shape), 1000)
     assert max(beside, around) < 2.5 * inside, (inside, beside, around)
+
+
+@pytest.mark.parametrize("k", [1, 10, 70])
+@pytest.mark.parametrize("share", [0.02, 0.5, 1.0])
+def test_centres_outside_the_box(cube, k, share):
+    """Batches that seed, with centres outside the box among them, alone and in a batch of two clouds."""
+    import torch
+
+    from octrees_benchmark_b200 import LinearOctree
+    from octrees_benchmark_b200.engine import BatchEngine, Request
+
+    rng = np.random.default_rng(k)
+    clouds = [cube[:40_000], cube[:30_000] * [1.0, 1.0, 0.0]]
+    ocs = [LinearOctree(xyz, encoder=enc, max_points_leaf=16) for xyz, enc in zip(clouds, (1, 5))]
+    reqs, want = [], []
+    for xyz, oc in zip(clouds, ocs):
+        q = xyz[rng.integers(0, len(xyz), 30_000)]
+        out = rng.random(len(q)) < share
+        q[out] += rng.uniform(-150.0, 150.0, (int(out.sum()), 3))
+        got = oc.knn(q, k)
+        oc.set_search_config(packet=False)
+        want.append(oc.knn(q, k))
+        oc.set_search_config(packet=True)
+        assert all(np.array_equal(a, b) for a, b in zip(want[-1], got))
+        reqs.append(Request(oc, "knn", torch.from_numpy(q).cuda(), k=k))
+    engine = BatchEngine()
+    places = engine.run(reqs)
+    for p, w in zip(places, want):
+        got = engine.knn_result(p, k)
+        assert all(np.array_equal(a, b) for a, b in zip(w, got))
+
+
+@pytest.mark.parametrize("flat", [False, True])
+def test_time_of_large_batches_outside_the_box(cube, flat):
+    """A batch that seeds takes about the time of one whose centres all start cold (knn_estimate -1); outside the box
+    2.7 and 3.7 times that while those centres were seeded too."""
+    import torch
+
+    from octrees_benchmark_b200 import LinearOctree
+
+    rng = np.random.default_rng(5)
+    xyz = cube * [1.0, 1.0, 0.0] if flat else cube
+    q = xyz[rng.integers(0, len(xyz), 20_000)] + ([150.0, 0.0, 0.0] if flat else rng.uniform(-200.0, 200.0, (20_000, 3)))
+    oc = LinearOctree(xyz, encoder=5, max_points_leaf=64, stream=torch.cuda.current_stream().cuda_stream)
+    seeded = knn_ms(oc, q, 10)
+    oc.set_search_config(knn_estimate=-1)
+    cold = knn_ms(oc, q, 10)
+    assert seeded < 1.6 * cold, (seeded, cold)
