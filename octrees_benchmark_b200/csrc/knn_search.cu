@@ -1047,9 +1047,15 @@ __device__ __noinline__ KnnCut knn_cut(double* d, uint32_t* ix, uint32_t n, doub
     return c;
 }
 
-// Bytes of dynamic shared memory of one warp.
+// Open nodes of a cold query that are kept, by the buffer (k <= 64: up to 128 points are looked for).
+__host__ __device__ constexpr int knn_open_nodes(uint32_t cap) { return cap <= 192 ? kGrpStack / 2 : kGrpStack; }
+
+// Bytes of dynamic shared memory of one warp: pairs, bins, and the bounds of a cold query's open nodes, whose place
+// the ranking's order of the pairs takes when no node is open any more.  (Shared memory is L1 cache that the walks
+// lack: at k = 44 and 13, 1.6 KB a block more for the bounds cost 2 to 3 % of the time.)
 __host__ __device__ constexpr size_t knn_group_bytes(uint32_t cap, uint32_t bins) {
-    return (size_t)cap * 12 + (size_t)bins * 4 + (size_t)cap * 2;
+    const size_t open = 4 * (size_t)knn_open_nodes(cap), ord = 2 * (size_t)cap;
+    return (size_t)cap * 12 + (size_t)bins * 4 + (open > ord ? open : ord);
 }
 
 // A cold query's first points: nodes and ranges taken best first (the smallest bound of all that are open, as
@@ -1065,7 +1071,7 @@ struct KnnNear {
 __device__ __noinline__ KnnNear knn_near_ranges(const uint32_t* offsets, const uint2* ranges, const double* centers,
                                                 const double (*radii)[3], double x, double y, double z, uint32_t K,
                                                 uint32_t bucket, KnnNear st, uint32_t* fcs, uint8_t* depths,
-                                                float* keys, uint2* list) {
+                                                float* keys, int room, uint2* list) {
     const int lane = threadIdx.x & 31;
     const double p[3] = {x, y, z};
     st.m = 0;
@@ -1114,7 +1120,7 @@ __device__ __noinline__ KnnNear knn_near_ranges(const uint32_t* offsets, const u
         }
         st.open += __popc(sm);
         __syncwarp();
-        if (st.open + 7 > kGrpStack) {
+        if (st.open + 7 > room) {
             // no room for the next node's children: the far half of the bounds' span goes, and again until half the
             // entries are left (any K points bound the K-th distance; halves of the span and not of the largest
             // bound, as the bounds of a query far from the cloud differ by little)
@@ -1127,7 +1133,7 @@ __device__ __noinline__ KnnNear knn_near_ranges(const uint32_t* offsets, const u
             const float low = __uint_as_float(__reduce_min_sync(0xffffffffu, least_left));
             float span = __uint_as_float(__reduce_max_sync(0xffffffffu, most)) - low;
 #pragma unroll 1
-            for (int tries = 0; st.open > kGrpStack / 2 && span > 0.0f && tries < 24; ++tries) {
+            for (int tries = 0; st.open > room / 2 && span > 0.0f && tries < 24; ++tries) {
                 span *= 0.5f;
                 int left = 0;
 #pragma unroll 1
@@ -1154,7 +1160,7 @@ __device__ __noinline__ KnnNear knn_near_ranges(const uint32_t* offsets, const u
                 }
                 st.open = left;
             }
-            if (st.open > kGrpStack / 2) st.open = kGrpStack / 2;  // (equal bounds)
+            if (st.open > room / 2) st.open = room / 2;  // (equal bounds)
         }
     }
     return st;
@@ -1166,7 +1172,6 @@ __global__ void __launch_bounds__(kGrpThreads, 7) k_knn_group(KnnGroupArgs a) {
     __shared__ uint32_t s_n[kGrpWarps];               // pairs in the buffer
     __shared__ uint32_t st_fc[kGrpWarps][kGrpStack];  // first child of a node
     __shared__ uint8_t st_d[kGrpWarps][kGrpStack];    // its children's depth
-    __shared__ float st_key[kGrpWarps][kGrpStack];    // its bound in FP32, for cold queries
     __shared__ uint2 s_rg[kGrpWarps][kGrpRanges];
     // the nodes that the warp's last walks passed one by one from the root (centre, first child), by
     // depth: a walk starts at the deepest that holds its whole ball
@@ -1194,7 +1199,7 @@ __global__ void __launch_bounds__(kGrpThreads, 7) k_knn_group(KnnGroupArgs a) {
     uint16_t* ord = reinterpret_cast<uint16_t*>(hist + bins);
     uint32_t* sf = st_fc[warp];
     uint8_t* sdp = st_d[warp];
-    float* sk = st_key[warp];
+    float* sk = reinterpret_cast<float*>(ord);  // bounds of a cold query's open nodes
     uint2* list = s_rg[warp];
     uint32_t* np = &s_n[warp];
     unsigned long long f_tests = 0, f_64 = 0, f_band = 0;
@@ -1319,8 +1324,9 @@ __global__ void __launch_bounds__(kGrpThreads, 7) k_knn_group(KnnGroupArgs a) {
         // A centre outside the cloud's box (by more than rounding) starts cold and seeds no other: its k-th distance is
         // decided by how far it is from the cloud, and a ball a little larger holds much of the cloud.  20k centres
         // around a cube of 500k points, k = 10: 570 -> 220 us, beside a plane 1056 -> 274; centres inside keep their time
-        const bool outside = __any_sync(
-            0xffffffffu, lane < 3 && fabs(ahead_c - pc[0][lane % 3]) > 1.000001 * s_radii[0][lane % 3]);
+        bool outside = false;
+        if (lane < 3) outside = fabs(ahead_c - pc[0][lane]) > 1.000001 * s_radii[0][lane];
+        outside = __any_sync(0xffffffffu, outside);
         cold = cold || outside;
         seed_slot = outside ? kNoSeed : head ? kHeadSeed : slot;
         double thr = cold ? (double)INFINITY : kGrpSeed * seed;
@@ -1408,7 +1414,8 @@ __global__ void __launch_bounds__(kGrpThreads, 7) k_knn_group(KnnGroupArgs a) {
                 for (;;) {
                     if (phase == 0) {
                         const KnnNear st = knn_near_ranges(KRQV(offsets), KRQV(ranges), KRQV(centers), s_radii, p[0], p[1],
-                                                           p[2], K, a.bucket, KnnNear{sp, taken, 0}, sf, sdp, sk, list);
+                                                           p[2], K, a.bucket, KnnNear{sp, taken, 0}, sf, sdp, sk,
+                                                           knn_open_nodes(cap), list);
                         sp = st.taken < knn_near_points(K) ? st.open : 0;
                         taken = st.taken;
                         m = st.m;
