@@ -57,7 +57,7 @@ L2_FLUSH_BYTES = 512 << 20
 # device launches of this library per timed step (counted from an ncu launch list of this bench):
 # plain: radius count, 3 scan kernels, fill; kNN.  The packet paths order the queries of each call first
 # (keys, histogram scan, 3 sort passes) and search the radius set in one pass (+ 3 scan kernels and the
-# chunk compaction), or count and fill with the FP32 filter; kNN in groups adds the fallback launch.
+# chunk compaction), with the FP32 filter too; the collecting kNN adds the fallback launch.
 LAUNCHES_PER_STEP = {"plain": 6, "packet": 10 + 7, "packet_fp32": 10 + 7, "knn_per_query": 10 + 6,
                      # engine: epoch, keys, histogram scan, 4 sort passes, one-pass radius, 3 scan kernels,
                      # chunk compaction, request totals, group kNN, fallback kNN
@@ -65,10 +65,10 @@ LAUNCHES_PER_STEP = {"plain": 6, "packet": 10 + 7, "packet_fp32": 10 + 7, "knn_p
 BUILD_BYTES_PER_POINT = 112  # encode 32 + sort 20 + reorder 52 + leaf counting 8
 BUILD_BYTES_PER_NODE = 36    # offsets 4 + ranges 8 + centers 24
 # DRAM bytes (read + write) per query of the search kernels, from ncu captures of this script's
-# tile at 6M points (the same density, 200k queries each): k_knn_group k=50 355.6 + 125.2 MB, one-pass
-# k_radius_packet r=2.5 207.5 + 50.3 MB
-KNN_DRAM_BYTES_PER_QUERY = (355.6e6 + 125.2e6) / 200_000
-RADIUS_DRAM_BYTES_PER_QUERY = (207.5e6 + 50.3e6) / 200_000
+# tile at 6M points (the same density, 200k queries each): k_knn_group k=50 366.7 + 129.3 MB, one-pass
+# k_radius_packet r=2.5 211.5 + 52.1 MB
+KNN_DRAM_BYTES_PER_QUERY = (366.7e6 + 129.3e6) / 200_000
+RADIUS_DRAM_BYTES_PER_QUERY = (211.5e6 + 52.1e6) / 200_000
 
 
 def measured_peak():

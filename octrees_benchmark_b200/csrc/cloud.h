@@ -59,7 +59,7 @@ struct DevBuf {
 };
 
 // The memory pool of every cloud's arrays on a device (created on first use,
-// kept for the process; it holds up to 8 GB of freed storage for reuse).
+// kept for the process; it holds all freed storage for reuse, until oct_trim_cloud_memory gives it back).
 cudaMemPool_t cloud_pool(int device);
 // The stream of a destroyed cloud, kept for the next one (at most kIdleStreams a device: creating and destroying a
 // stream costs a small cloud as much as its sort); stream_get creates one when none is idle, idle_streams_drop
@@ -204,7 +204,7 @@ struct Cloud {
     uint32_t qs_epoch = 0;
     DevBuf packet_ctr;  // dynamic packet counters
     DevBuf knn_fb;      // collecting kNN: fallback count (u64) at 0, fallback query list (u32) from byte 16
-    DevBuf knn_heads;   // group kNN: the heads' largest k-th distances (f64 per head)
+    DevBuf knn_heads;   // collecting kNN: the heads' k-th distances (f64 per head)
     DevBuf stats;       // device counters: points tested, FP64 band re-tests, ...
     // FP32 leaf-relative coordinates (x, y, z, 0) per sorted point, built on demand
     DevBuf rel;
@@ -214,7 +214,7 @@ struct Cloud {
     // search configuration (oct_set_search_config)
     int packet = 1;
     int fp32_filter = 0;  // 0, OCT_FP32_ALL, OCT_FP32_RADIUS or OCT_FP32_KNN
-    int knn_packet = 1;  // kNN (k <= 64, packet path): groups of queries per warp
+    int knn_packet = 1;  // kNN (packet path): the collecting search, else sorted lists (k <= 64)
     uint32_t knn_bucket = 256;
     int two_pass = 0;   // 1: packet radius searches count, then fill (no result chunks)
     // neighborsStruct searches of the current call: 0, or neighborsApprox's precisionLevel + 1
@@ -226,8 +226,8 @@ struct Cloud {
     const double* axes = nullptr;
     uint32_t axes_stride = 0;
     DevBuf q_axes;
-    double knn_est = kKnnEstimate;  // register kNN: provisional-threshold factor (0: off)
-    uint32_t knn_chunk = kKnnGroupChunk;  // group kNN: consecutive groups per warp fetch
+    double knn_est = kKnnEstimate;  // kNN provisional threshold: the sorted lists' factor; the collecting search seeds its queries unless 0
+    uint32_t knn_chunk = kKnnGroupChunk;  // collecting kNN: pairs of consecutive queries per warp fetch
     // one-pass radius search: result chunk pool, each chunk's query and place in its chain, counter
     DevBuf ck_pool, ck_rec, ck_ctr;
 

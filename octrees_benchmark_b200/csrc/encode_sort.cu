@@ -1129,7 +1129,7 @@ cudaError_t launch_gather(Cloud& c, const double* d_xyz, const uint32_t* d_perm,
 // ---------------------------------------------------------------------------
 // Query ordering for the packet searches: the query centres are keyed with the
 // cloud's box and curve and stably sorted by the top 24 key bits (3 onesweep
-// passes), so that the 32 queries of a warp are spatial neighbours.
+// passes), so that the queries of a warp are spatial neighbours.
 // ---------------------------------------------------------------------------
 // Device-sized sort of a batch's query keys (the batched engine): the key
 // count and the epoch base are read on the device, and every pass runs a fixed

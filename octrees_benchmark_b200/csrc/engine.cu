@@ -11,15 +11,16 @@
 //      its curve key in its cloud's frame) and the digit histograms; a 3-5
 //      pass onesweep sort of these keys orders every request's centres along
 //      its cloud's curve while each request keeps its own position range;
-//   3. per radius variant one persistent packet launch counts, a scan turns
-//      the counts into CSR offsets and a second launch fills; the kNN groups
-//      run at the same time on a forked stream;
+//   3. per radius variant one persistent packet launch searches: every centre's
+//      results go to its own chain of chunks and are counted.  A scan turns the
+//      counts into CSR offsets and the chunks are compacted there; the kNN
+//      variants run at the same time on a forked stream;
 //   4. a 16-byte summary (radius total, error word) and the per-request result
 //      sizes come back.
 // Every size of steps 2-4 is read on the device, so a batch shape (the set of
 // variants and the pass count) is captured once as a CUDA graph and replayed
 // for every later batch of that shape.  When the radius results outgrow the
-// result array the host grows it and runs the batch again.
+// result array or the chunks, the host grows them and runs the batch again.
 #include <algorithm>
 #include <cstdio>
 #include <cstring>

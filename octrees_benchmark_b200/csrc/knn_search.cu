@@ -735,7 +735,7 @@ __global__ void __launch_bounds__(kKnnThreads, 8) k_knn_reg(KnnTableArgs a) {
 // which costs L2 hits).  Every kKnnHeadStride-th query (of k = 1 every 64th) is a head: heads are handed
 // out first; the first query of a run (and each query handed out alone at the
 // end) starts from the nearest head of its request that has finished.  A query
-// without a seed, and a query that found fewer than k pairs within its seeded
+// without a seed (one whose centre lies outside the cloud's box among them), and a query that found fewer than k pairs within its seeded
 // threshold, takes the k-th distance among the first 2 k points (3/2 k of k > 256) that a
 // best-first walk comes to (knn_near_ranges): an upper bound of its k-th
 // distance, so the walk that follows always suffices.  What is left (a stack or a buffer that cannot hold a
@@ -755,7 +755,7 @@ __global__ void __launch_bounds__(kKnnThreads, 8) k_knn_reg(KnnTableArgs a) {
 // (2 KB more a block: 2.87 -> 2.97 ms).  Whole calls before (groups of four with
 // sorted lists for k <= 64, bitonic merges in shared memory above) and now:
 //   10M-point tile: 500k, k = 50 3700 -> 2787 us; 50k, k = 50 1069 -> 430; 5k, k = 50
-//   497 -> 195; 200, k = 50 345 -> 105; 5M: 30k, k = 250 2300 -> 710; 3k, k = 900
+//   497 -> 195; 200, k = 50 345 -> 105; 5M: 30k, k = 250 2300 -> 636; 3k, k = 900
 //   2400 -> 610.  k = 1: see kHeadBitsOne.
 // ---------------------------------------------------------------------------
 
@@ -789,9 +789,9 @@ struct KnnGroupArgs {
     double* d2;
     uint32_t* counts;
     uint32_t* err;
-    double est;                       // > 0: groups are seeded; 0: every query starts from its own node
-    uint32_t* packet_ctr;             // [0] runs of `chunk` groups, [1] single groups at the end, [2] heads
-    uint32_t chunk;                   // consecutive groups per fetch (>= 1)
+    double est;                       // > 0: queries are seeded; else every one starts from the points next to it
+    uint32_t* packet_ctr;             // [0] runs of `chunk` queries, [1] single queries at the end, [2] heads
+    uint32_t chunk;                   // pairs of consecutive queries per fetch (>= 1)
     uint32_t heads;                   // 1: every kKnnHeadStride-th query is a head, taken first
     double* head_kth;                 // per head: the largest k-th distance it found (NaN: not yet, < 0: none)
     unsigned long long* stats;        // FP32 filter: point tests, FP64 tests, band hits (may be null)

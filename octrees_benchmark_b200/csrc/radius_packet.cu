@@ -1,5 +1,5 @@
 // Batched ("packet") radius search: neighbors / neighborsPrune / neighborsStruct
-// for up to 32 spatially ordered queries per warp (packet_width).
+// for 1 to 16 spatially ordered queries per warp (FP32 counts: to 32; packet_width).
 //
 // Reference path replaced: the same as radius_search.cu - singleTraversal
 // (inc/structures/linear_octree.hpp:653-686) with the criteria and leaf actions of
@@ -20,7 +20,7 @@
 // are written by the whole warp.  Packets are handed out by an atomic counter so
 // that long and short packets balance.
 //
-// Bound: instruction issue (2.45k warp instructions per query at r = 2.5 on the
+// Bound: instruction issue (2.5k warp instructions per query at r = 2.5 on the
 // 10M-point tile, DRAM below 5 % of peak): the pair loop takes about 1k of them,
 // the child tests 0.6k.  500k queries there: 2122 us with one leaf at a time and
 // one pass per four active queries, 1904 us with the leaf groups, 1638 us with
@@ -70,7 +70,7 @@ struct PacketArgs {
                                 // one_cloud, single.cv is the cloud of every request of grp
     const DynGroup* grp;        // sizes and request table of a batch group (device)
     uint64_t packets;           // packets of a single-request launch
-    uint32_t width;             // queries per packet of a single-request launch (1 to 32)
+    uint32_t width;             // queries per packet of a single-request launch (1 to 16; FP32 counts: to 32)
     bool one_cloud;             // host dispatch: grp's requests all search single.cv
     const uint32_t* order;      // query visiting order (global positions), or null
     unsigned long long* counts;

@@ -167,7 +167,7 @@ class LinearOctree:
     def set_search_config(self, packet: bool = True, fp32_filter: bool = False, radius_lanes: int = 8,
                           knn_packet: bool = True, knn_bucket: int = 256, two_pass: bool = False,
                           knn_estimate: int = 0, knn_group_run: int = 0):
-        """Search path: packet (32 curve-ordered queries per warp) or one query per
+        """Search path: packet (curve-ordered queries, 1 to 16 per warp by their number) or one query per
         ``radius_lanes`` lanes; FP32 filter with FP64 re-tests (radius: leaf-relative points;
         group kNN: points relative to the box centre, FP64 only near the k-th distance; ``fp32_filter``
         True / OCT_FP32_ALL both, OCT_FP32_RADIUS or OCT_FP32_KNN one of them); the collecting kNN
