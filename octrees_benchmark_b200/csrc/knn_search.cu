@@ -754,8 +754,8 @@ __global__ void __launch_bounds__(kKnnThreads, 8) k_knn_reg(KnnTableArgs a) {
 // shared memory, which is taken from the L1 that serves neighbouring queries
 // (2 KB more a block: 2.87 -> 2.97 ms).  Whole calls before (groups of four with
 // sorted lists for k <= 64, bitonic merges in shared memory above) and now:
-//   10M-point tile: 500k, k = 50 3700 -> 2787 us; 50k, k = 50 1069 -> 430; 5k, k = 50
-//   497 -> 195; 200, k = 50 345 -> 105; 5M: 30k, k = 250 2300 -> 636; 3k, k = 900
+//   10M-point tile: 500k, k = 50 3700 -> 2754 us; 50k, k = 50 1069 -> 430; 5k, k = 50
+//   497 -> 195; 200, k = 50 345 -> 105; 5M: 30k, k = 250 2300 -> 627; 3k, k = 900
 //   2400 -> 610.  k = 1: see kHeadBitsOne.
 // ---------------------------------------------------------------------------
 
